@@ -1,0 +1,465 @@
+// clmd_cycle.cuh -- what the persistent step kernels share (clmd_cycle.cu: any
+// size, the whole GPU, grid barriers; clmd_small.cu: small systems, one
+// thread-block cluster): the replicated scalar logic (skin, rebuild
+// decision), the list search of one atom, and the warp-cooperative pair
+// forces.
+#pragma once
+
+#include "clmd_mixed.cuh"
+#include "clmd_system.hpp"
+
+namespace clmd {
+
+constexpr int kSmallThreads = 512; // threads per CTA of the small-system kernel at most
+constexpr int kRowBufC = 32;      // candidate buffer of the list search
+
+struct Geo {
+  double rs2, cfx, cfy, cfz;
+  int ncx, ncy, ncz, ncell;
+  int nox, noy, noz, pad;
+  int offx[3], offy[3], offz[3];
+};
+
+struct Blk {
+  clmd_scalars q;
+  Geo g;
+  double kf[CLMD_MXSORTS];
+  double bcast[4];
+  int scale[CLMD_MXSORTS];
+  int rebuild;
+  int stop;
+};
+
+// ---------------------------------------------------------------------------
+// scalar logic (thread 0 of each block on its replica)
+// ---------------------------------------------------------------------------
+
+// neighbor-pbc-mav.f:48-60, 101-105 and the cell grid
+static __device__ void prologue(const Params& P, Blk& B, int step) {
+  clmd_scalars& q = B.q;
+  if (q.dmms > (q.atrskin - P.atrcut)) {  // :48-51
+    if (q.status == 0) {
+      q.status = CLMD_ERR_SKIN;
+      q.fail_step = step;
+    }
+    B.stop = 1;
+    B.rebuild = 0;
+    return;
+  }
+  q.dmmav = (double)(float)q.dmmst * q.dmmsu / 256.0;  // :53
+  if (step != P.btim && step > 0) {                      // :55-60
+    q.atrskin = P.atrcut + (q.atrskin - P.atrcut) * (double)P.nbtim / (double)q.dmmst;
+    q.atrskin = fmin(P.boxx / 2.0, q.atrskin);
+    q.atrskin = fmin(P.boxy / 2.0, q.atrskin);
+    q.atrskin = fmin(P.boxz / 2.0, q.atrskin);
+  }
+  Geo& g = B.g;
+  g.rs2 = q.atrskin * q.atrskin;
+  double side = q.atrskin * (1.0 + 1e-9);
+  int n3[3] = {(int)floor(P.boxx / side), (int)floor(P.boxy / side), (int)floor(P.boxz / side)};
+  int mx[3] = {P.ncx_max, P.ncy_max, P.ncz_max};
+  int* offs[3] = {g.offx, g.offy, g.offz};
+  int* nos[3] = {&g.nox, &g.noy, &g.noz};
+  for (int d = 0; d < 3; d++) {
+    n3[d] = max(1, min(n3[d], mx[d]));
+    if (n3[d] >= 3) {
+      offs[d][0] = -1; offs[d][1] = 0; offs[d][2] = 1; *nos[d] = 3;
+    } else if (n3[d] == 2) {
+      offs[d][0] = 0; offs[d][1] = 1; *nos[d] = 2;
+    } else {
+      offs[d][0] = 0; *nos[d] = 1;
+    }
+  }
+  g.ncx = n3[0];
+  g.ncy = n3[1];
+  g.ncz = n3[2];
+  g.ncell = n3[0] * n3[1] * n3[2];
+  g.cfx = (double)g.ncx / P.boxx;
+  g.cfy = (double)g.ncy / P.boxy;
+  g.cfz = (double)g.ncz / P.boxz;
+  q.dmmax = fmax(q.dmms, q.dmmax);  // :101-105
+  q.dmms = 0.0;
+  q.dmmst = 0;
+  q.nrebuild = q.nrebuild + 1;
+  q.last_rebuild_step = step;
+}
+
+// int-verlet-mav.f:64-74 / int-verlet-nh-mav.f:70-78
+static __device__ void skin(const Params& P, Blk& B, double dmmr, int step) {
+  clmd_scalars& q = B.q;
+  dmmr = 2.2 * sqrt(dmmr);
+  q.dmms = q.dmms + dmmr;
+  q.dmmsu = q.dmmsu + dmmr - q.dmmh[q.dmmi];
+  q.dmmh[q.dmmi] = dmmr;
+  q.dmmi = (q.dmmi + 1) & 255;
+  q.dmmst = q.dmmst + 1;
+  B.rebuild = q.dmms > (q.atrskin - P.atrcut - 2.0 * q.dmms / (double)(float)q.dmmst);
+  if (B.rebuild) prologue(P, B, step);
+}
+
+// ---------------------------------------------------------------------------
+// the list rebuild (neighbor-pbc-mav.f:67-99) as barrier-separated phases
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool nbt(const Params& P, double rs2, const double4& a,
+                                    const double4& b) {
+  double dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+  dx = mimage_nb(dx, P.boxx, P.ibx);
+  dy = mimage_nb(dy, P.boxy, P.iby);
+  dz = mimage_nb(dz, P.boxz, P.ibz);
+  double r2 = dx * dx + dy * dy + dz * dz;
+  return r2 <= rs2;
+}
+
+// the candidate slots of a cell row: [a0, b0) and, where the x-neighbours
+// wrap, [a1, b1) (scalars, not arrays indexed by the range: those would live
+// in local memory)
+__device__ __forceinline__ int xr(const Geo& g, const int* cs, int row, int cx, int& a0,
+                                  int& b0, int& a1, int& b1) {
+  int n = g.ncx;
+  if (n >= 3) {
+    if (cx >= 1 && cx <= n - 2) {
+      a0 = cs[row + cx - 1]; b0 = cs[row + cx + 2];
+      return 1;
+    }
+    if (cx == 0) {
+      a0 = cs[row]; b0 = cs[row + 2];
+      a1 = cs[row + n - 1]; b1 = cs[row + n];
+      return 2;
+    }
+    a0 = cs[row + n - 2]; b0 = cs[row + n];
+    a1 = cs[row]; b1 = cs[row + 1];
+    return 2;
+  }
+  a0 = cs[row];
+  b0 = cs[row + n];
+  return 1;
+}
+
+template <bool FILL>
+__device__ __forceinline__ int scan_cells(const Params& P, const Geo& g, int p, int refi,
+                                          const double4& pi, const double4* pos,
+                                          const int* perm, const int* cs, int* bq, int* bref,
+                                          int* out) {
+  int cx = min((int)(pi.x * g.cfx), g.ncx - 1);
+  int cy = min((int)(pi.y * g.cfy), g.ncy - 1);
+  int cz = min((int)(pi.z * g.cfz), g.ncz - 1);
+  int n = 0;
+  for (int a = 0; a < g.noz; a++) {
+    int zz = cz + g.offz[a];
+    zz += (zz < 0) ? g.ncz : 0;
+    zz -= (zz >= g.ncz) ? g.ncz : 0;
+    for (int b = 0; b < g.noy; b++) {
+      int yy = cy + g.offy[b];
+      yy += (yy < 0) ? g.ncy : 0;
+      yy -= (yy >= g.ncy) ? g.ncy : 0;
+      int row = (zz * g.ncy + yy) * g.ncx;
+      int a0, b0, a1 = 0, b1 = 0;
+      const int nr = xr(g, cs, row, cx, a0, b0, a1, b1);
+      for (int r = 0; r < nr; r++) {
+        const int qb = r ? b1 : b0;
+        for (int q = r ? a1 : a0; q < qb; q++) {
+          if (q == p) continue;
+          double4 pq = pos[q];
+          int refq = perm[q];
+          bool hit = (refi < refq) ? nbt(P, g.rs2, pi, pq) : nbt(P, g.rs2, pq, pi);
+          if (hit) {
+            if (FILL) {
+              out[n] = q;
+            } else if (n < kRowBufC) {
+              bq[n] = q;
+              bref[n] = refq;
+            }
+            n++;
+          }
+        }
+      }
+    }
+  }
+  return n;
+}
+
+// Rows longer than the search's buffer, one after the other by the whole
+// warp: lanes with n > 0 name a row of n entries (slots, in any order) that
+// starts at list[start]; each is put in ascending reference order, *lo gets
+// the number of entries below the owner's reference index.  Up to 256
+// entries sit in registers, 8 per lane, and every entry's place is the count
+// of smaller keys (distinct, so the places are a permutation); a longer row
+// is left to its lane's insertion sort.  A liquid droplet's rows run to ~130
+// entries, where one lane's insertion sort in memory took ~130 us.
+static __device__ void sort_long_rows(int* list, const int* perm, unsigned long long start, int n,
+                                      int refi, int& lo) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int kT = 8;
+  const int lane = threadIdx.x & 31;
+  unsigned todo = __ballot_sync(FULL, n > 0);
+  __syncwarp();  // the owners' entries are visible to every lane
+  while (todo) {
+    const int ow = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int m = __shfl_sync(FULL, n, ow), ref = __shfl_sync(FULL, refi, ow);
+    int* row = list + __shfl_sync(FULL, start, ow);
+    if (m > 32 * kT) {
+      if (lane == ow) {
+        for (int a = 1; a < m; a++) {
+          int kq = row[a], kr = perm[kq];
+          int b = a - 1;
+          while (b >= 0 && perm[row[b]] > kr) {
+            row[b + 1] = row[b];
+            b--;
+          }
+          row[b + 1] = kq;
+        }
+        lo = 0;
+        for (int a = 0; a < m; a++) lo += perm[row[a]] < refi;
+      }
+      __syncwarp();
+      continue;
+    }
+    int q[kT], key[kT], rank[kT], below = 0;
+#pragma unroll
+    for (int t = 0; t < kT; t++) {
+      const int k = lane + 32 * t;
+      q[t] = k < m ? row[k] : 0;
+      key[t] = k < m ? perm[q[t]] : 0x7fffffff;
+      rank[t] = 0;
+      below += __popc(__ballot_sync(FULL, k < m && key[t] < ref));
+    }
+#pragma unroll
+    for (int u = 0; u < kT; u++) {
+      if (32 * u >= m) break;
+      for (int l = 0; l < 32; l++) {
+        const int other = __shfl_sync(FULL, key[u], l);
+#pragma unroll
+        for (int t = 0; t < kT; t++) rank[t] += other < key[t];
+      }
+    }
+    __syncwarp();  // every lane has read the row
+#pragma unroll
+    for (int t = 0; t < kT; t++)
+      if (lane + 32 * t < m) row[rank[t]] = q[t];
+    if (lane == ow) lo = below;
+    __syncwarp();
+  }
+}
+
+struct CycleArgs {
+  double4* pos0;
+  double4* pos1;
+  double *vx, *vy, *vz, *ax, *ay, *az;
+  double *vxn, *vyn, *vzn;
+  // mixed Nose-Hoover: the accelerations between a step's force pass and its
+  // velocity pass, FP32 (the storage of the FP64 sweeps' iterate vxn..vzn,
+  // which that path does not use)
+  float *afx, *afy, *afz;
+  int *perm, *iperm;
+  double4* pos_s;
+  double *vx_s, *vy_s, *vz_s, *ax_s, *ay_s, *az_s;
+  int* perm_s;
+  int *cell_count, *cell_start, *cell_fill, *cell_atoms, *atom_cell, *scan_aux;
+  int *list, *row_start, *row_len, *row_lo;
+  double* red;  // 2 x kRedSlots x gridDim partials
+};
+
+// neighbor-pbc-mav.f:67-71
+__device__ __forceinline__ double4 wrap_box(const Params& P, double4 v) {
+  v.x = fmod(fmod(v.x, P.boxx) + P.boxx, P.boxx);
+  v.y = fmod(fmod(v.y, P.boxy) + P.boxy, P.boxy);
+  v.z = fmod(fmod(v.z, P.boxz) + P.boxz, P.boxz);
+  return v;
+}
+
+// for-a-lj-n-pbc-m.f:92-142 for one atom: fsum in the reference's order
+// (accumulated by warp_forces below)
+struct Pair {
+  double fx, fy, fz, esum, vir;
+};
+
+// Pair forces, warp-cooperative, for the 32 consecutive slots of a warp, whose
+// rows are contiguous in the list (the search allocates them with one
+// warp-wide cursor step).  Lanes evaluate the pair terms of 32 consecutive
+// list entries at a time (balanced work whatever the row lengths), stage them
+// in shared memory, and each owner lane then adds its own terms in list
+// order, i.e. in the reference's order, with the same +/- as the serial code.
+// FP64: the terms of kGroup chunks are staged before the owner lanes add
+// theirs, so that more owners work at once (a row's terms still go in
+// list order)
+#ifndef CLMD_FORCE_GROUP
+#define CLMD_FORCE_GROUP 4
+#endif
+constexpr int kGroup = CLMD_FORCE_GROUP;
+struct WarpStage {
+  double tx[32 * kGroup], ty[32 * kGroup], tz[32 * kGroup];
+  int flag[32 * kGroup];  // 0 nothing, 1 add, 2 subtract
+};
+
+template <bool MIXED>
+__device__ __forceinline__ void warp_forces(const Params& P, DevState* st, const double4* pos,
+                                            const int* list, int st0, int len, int lo,
+                                            const double4& pa, double bf1, double bf2,
+                                            double& fx, double& fy, double& fz, double& esum,
+                                            double& vir, WarpStage& W, bool& bad) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int e = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    int t = __shfl_up_sync(FULL, e, o);
+    if (lane >= o) e += t;
+  }
+  const int tot = __shfl_sync(FULL, e, 31);
+  e -= len;  // exclusive prefix: this lane's row starts at wbase + e
+  const int wbase = __shfl_sync(FULL, st0, 0);
+  const int sa = (int)pa.w;
+  constexpr bool mixed = MIXED;
+  float sx = 0.f, sy = 0.f, sz = 0.f, kx = 0.f, ky = 0.f, kz = 0.f;  // mixed: Kahan sums
+  fx = 0.0;
+  fy = 0.0;
+  fz = 0.0;
+  // this chunk's entry and neighbour position are fetched first, and the
+  // next chunk's entry with them, so that the loads overlap the owner search
+  int jnext = lane < tot ? list[wbase + lane] : 0;
+  for (int c = 0; c < tot; c += 32) {
+    const int k = c + lane;
+    const int kk = k < tot ? k : tot - 1;
+    const int jc = jnext;
+    double4 pb = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (k < tot) pb = pos[jc];
+    if (k + 32 < tot) jnext = list[wbase + k + 32];
+    int ow = 0;
+#pragma unroll
+    for (int sft = 16; sft >= 1; sft >>= 1) {
+      int cand = ow + sft;
+      int ec = __shfl_sync(FULL, e, cand & 31);
+      if (cand <= 31 && ec <= kk) ow = cand;
+    }
+    const double ox = __shfl_sync(FULL, pa.x, ow);
+    const double oy = __shfl_sync(FULL, pa.y, ow);
+    const double oz = __shfl_sync(FULL, pa.z, ow);
+    const int osp = __shfl_sync(FULL, sa, ow);
+    const int oe = __shfl_sync(FULL, e, ow);
+    const int olo = __shfl_sync(FULL, lo, ow);
+    int flag = 0;
+    double tx = 0.0, ty = 0.0, tz = 0.0;
+    if (k < tot) {
+      bool own = (k - oe) >= olo;  // neighbour has the larger reference index
+      double dx, dy, dz;
+      if (own) {
+        dx = ox - pb.x; dy = oy - pb.y; dz = oz - pb.z;
+      } else {
+        dx = pb.x - ox; dy = pb.y - oy; dz = pb.z - oz;
+      }
+      dx = mimage_bf(dx, P.boxx, P.ibx, bf1, bf2);
+      dy = mimage_bf(dy, P.boxy, P.iby, bf1, bf2);
+      dz = mimage_bf(dz, P.boxz, P.ibz, bf1, bf2);
+      double rij2 = dx * dx + dy * dy + dz * dz;
+      if (rij2 <= P.atr2) {
+        double r2 = rij2;
+        double rij6 = 0.0;
+        if (!mixed) {
+          rij2 = 1.0 / rij2;
+          rij6 = rij2 * rij2 * rij2;
+        }
+        int ij = osp + (int)pb.w;
+        if (ij < 2 || ij > 4) {
+          raise_err(st, CLMD_ERR_BAD_SPECIES);
+          bad = true;
+        } else if (mixed) {
+          double e, w;
+          pair_term_f32(P, ij, r2, dx, dy, dz, tx, ty, tz, e, w);
+          if (own) {
+            esum = esum + e;
+            vir = vir + w;
+            flag = 1;
+          } else {
+            flag = 2;
+          }
+        } else {
+          double fij = pair_fij(P, ij, rij2, rij6);
+          tx = fij * dx;
+          ty = fij * dy;
+          tz = fij * dz;
+          if (own) {
+            esum = esum + pair_e(P, ij, rij6);
+            vir = vir + fij * r2;
+            flag = 1;
+          } else {
+            flag = 2;
+          }
+        }
+      }
+    }
+    const int a0 = e > c ? e : c;
+    const int a1 = (e + len) < (c + 32) ? (e + len) : (c + 32);
+    if (mixed) {
+      // each row's terms in this chunk summed by a segmented scan across the
+      // lanes (a fixed tree: deterministic), then added to the owner's
+      // Kahan sums chunk by chunk: every lane works, where the ordered
+      // FP64 sum below has only the owners working
+      const float sg = flag == 1 ? 1.0f : (flag == 2 ? -1.0f : 0.0f);
+      float v0 = sg * (float)tx, v1 = sg * (float)ty, v2 = sg * (float)tz;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int ou = __shfl_up_sync(FULL, ow, off);
+        const float u0 = __shfl_up_sync(FULL, v0, off);
+        const float u1 = __shfl_up_sync(FULL, v1, off);
+        const float u2 = __shfl_up_sync(FULL, v2, off);
+        if (lane >= off && ou == ow) {
+          v0 = __fadd_rn(v0, u0);
+          v1 = __fadd_rn(v1, u1);
+          v2 = __fadd_rn(v2, u2);
+        }
+      }
+      const int last = a1 > a0 ? a1 - 1 - c : 0;  // my row's last entry in the chunk
+      const float p0 = __shfl_sync(FULL, v0, last);
+      const float p1 = __shfl_sync(FULL, v1, last);
+      const float p2 = __shfl_sync(FULL, v2, last);
+      if (a1 > a0) {
+        kahan_add(sx, kx, p0);
+        kahan_add(sy, ky, p1);
+        kahan_add(sz, kz, p2);
+      }
+      continue;
+    }
+    const int g = (c >> 5) % kGroup;
+    W.tx[32 * g + lane] = tx;
+    W.ty[32 * g + lane] = ty;
+    W.tz[32 * g + lane] = tz;
+    W.flag[32 * g + lane] = flag;
+    if (g != kGroup - 1 && c + 32 < tot) continue;  // the group is not full yet
+    __syncwarp();
+    const int cg = c - 32 * g;  // the group's first entry
+    const int b0 = e > cg ? e : cg;
+    const int b1 = (e + len) < (c + 32) ? (e + len) : (c + 32);
+    for (int a = b0; a < b1; a++) {
+      int q = a - cg;
+      int f = W.flag[q];
+      if (f == 1) {
+        fx = fx + W.tx[q];
+        fy = fy + W.ty[q];
+        fz = fz + W.tz[q];
+      } else if (f == 2) {
+        fx = fx - W.tx[q];
+        fy = fy - W.ty[q];
+        fz = fz - W.tz[q];
+      }
+    }
+    __syncwarp();
+  }
+  if (mixed) {
+    fx = (double)sx;
+    fy = (double)sy;
+    fz = (double)sz;
+  }
+}
+
+__device__ __forceinline__ int sp_block(const Params& P, int ref) {
+  for (int s = 0; s < P.atsorts; s++)
+    if (ref >= P.sp_start[s] && ref < P.sp_start[s + 1]) return s;
+  return -1;
+}
+
+// clmd_small.cu: systems of up to 16 * kSmallThreads atoms
+void small_setup(clmd_system* S);
+void small_launch(clmd_system* S, const CycleArgs& A, int nsteps, int mode);
+
+}  // namespace clmd

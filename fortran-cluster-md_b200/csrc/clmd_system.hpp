@@ -60,6 +60,9 @@ struct clmd_system {
   // launch geometry
   int nblk = 1;          // ceil(N / kBlock)
   int cyc_blocks = 1;    // co-resident blocks of the persistent kernel
+  int small_ctas = 0;    // CTAs of the small-system kernel's cluster (0: the grid kernel)
+  int small_threads = 0;
+  bool debug_barrier = false;  // clmd_debug_barrier in force
   long long launches = 0;
   // captured main-loop graph: analysis + ftcsi steps
   cudaGraphExec_t cyc_exec = nullptr;

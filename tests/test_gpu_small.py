@@ -1,0 +1,94 @@
+"""The step kernel of small systems (one thread-block cluster, one atom per
+thread) at the edges of its range: one and several CTAs, partial warps, the
+largest size and the first beyond it, rows longer than the search's buffer.
+FP64 velocity Verlet is bit-identical to the oracle; Nose-Hoover and the
+energy sums agree within the rounding of the sums, mixed precision within
+the FP32 rounding of the pair terms over a few steps."""
+import numpy as np
+import pytest
+
+import clmd
+import orc
+from conftest import droplet_state, random_state, start_pair
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [3, 32, 33, 128, 129, 1000, 2048, 2049, 4097, 8192, 8193]
+
+
+def rel(a, b):
+    return abs(a - b) / max(abs(b), 1e-300)
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_small_verlet_bit_exact(gpu, n):
+    cfg = clmd.lj_config(n, 0.01 if n < 10 else 0.04, 0.8)
+    g, o = clmd.System(cfg), orc.Oracle(cfg, neighbor_mode=1 if n > 64 else 0)
+    start_pair(g, o, cfg, random_state(cfg, 5 + n))
+    g.steps(1, 25)
+    for i in range(1, 26):
+        o.integrator(i)
+    a, b = g.get_state(), o.get_state()
+    for k in ("x", "y", "z", "vx", "vy", "vz", "ax", "ay", "az"):
+        assert np.array_equal(getattr(a, k), getattr(b, k)), k
+    for u, v in zip(g.halflist(), o.halflist()):
+        assert np.array_equal(u, v)
+    sg, so = g.scalars(), o.scalars()
+    assert (sg.nrebuild, sg.dmmst, sg.atrskin) == (so.nrebuild, so.dmmst, so.atrskin)
+    # sums of n terms in another order: n ulps at most of the terms' scale
+    assert abs(sg.ekin - so.ekin) <= 1e-12 * so.ekin
+    assert abs(sg.epot - so.epot) <= 1e-12 * max(abs(so.epot), 1.0)
+
+
+@pytest.mark.parametrize("n", [33, 129, 2049, 8192])
+@pytest.mark.parametrize("ethst", ["N", "X"])
+def test_small_thermostats(gpu, n, ethst):
+    cfg = clmd.lj_config(n, 0.04, 0.8, ethst=ethst,
+                         integrator=clmd.INT_NOSE if ethst == "N" else clmd.INT_VERLET)
+    if ethst == "X":
+        cfg.apth = b"X" + b"-" * (clmd.MXSORTS - 1)
+    g, o = clmd.System(cfg), orc.Oracle(cfg, neighbor_mode=1 if n > 64 else 0)
+    start_pair(g, o, cfg, random_state(cfg, 9 + n))
+    g.run(1, 20)
+    o.run(1, 20)
+    a, b = g.get_state(), o.get_state()
+    # 20 steps amplify the sums' rounding (1e-15) by far less than 1e4
+    for k in ("x", "y", "z", "vx", "vy", "vz"):
+        np.testing.assert_allclose(getattr(a, k), getattr(b, k), rtol=1e-9, atol=1e-10)
+    sg, so = g.scalars(), o.scalars()
+    assert rel(sg.ekin, so.ekin) < 1e-11
+    if ethst == "N":
+        assert abs(sg.psi - so.psi) < 1e-11
+        assert abs(sg.nh_iters - so.nh_iters) <= 1
+
+
+@pytest.mark.parametrize("drops,radius", [(2, 3.4), (1, 7.0)])
+def test_small_long_rows_bit_exact(gpu, drops, radius):
+    """Rows of ~100 entries (liquid droplets) and, at the largest list radius
+    in the denser blob, of more."""
+    cfg = clmd.lj_config(4000, 0.03, 0.7, rskin=3.4)
+    g, o = clmd.System(cfg), orc.Oracle(cfg, neighbor_mode=1)
+    start_pair(g, o, cfg, droplet_state(cfg, 3, drops, radius))
+    for u, v in zip(g.halflist(), o.halflist()):
+        assert np.array_equal(u, v)
+    g.steps(1, 12)
+    for i in range(1, 13):
+        o.integrator(i)
+    a, b = g.get_state(), o.get_state()
+    for k in ("x", "y", "z", "vx", "vy", "vz", "ax", "ay", "az"):
+        assert np.array_equal(getattr(a, k), getattr(b, k)), k
+
+
+@pytest.mark.parametrize("n", [129, 4097])
+def test_small_mixed_forces(gpu, n):
+    cfg = clmd.lj_config(n, 0.05, 0.75, precision=clmd.PREC_MIXED, integrator=clmd.INT_NOSE,
+                         ethst="N")
+    g, o = clmd.System(cfg), orc.Oracle(cfg, neighbor_mode=1)
+    start_pair(g, o, cfg, random_state(cfg, 77))
+    g.integrator(1)
+    o.integrator(1)
+    a, b = g.get_state(), o.get_state()
+    ga = np.stack([a.ax, a.ay, a.az])
+    oa = np.stack([b.ax, b.ay, b.az])
+    assert np.linalg.norm(ga - oa) <= 1e-5 * np.linalg.norm(oa)
+    assert g.scalars().status == 0
