@@ -58,6 +58,7 @@ static void fill_params(const clmd_config* c, Params* P) {
   P->ibx = 1.0 / c->boxx;
   P->iby = 1.0 / c->boxy;
   P->ibz = 1.0 / c->boxz;
+  P->img = 0.49 * std::min(c->boxx, std::min(c->boxy, c->boxz));
   P->dt = c->dt;
   P->atrcut = c->atrcut;
   P->atr2 = c->atrcut * c->atrcut;
@@ -184,6 +185,7 @@ extern "C" int clmd_create(const clmd_config* cfg, clmd_system** out) {
   CK(dalloc(&S->api, N));
   CK(dalloc(&S->perm, N)); CK(dalloc(&S->iperm, N)); CK(dalloc(&S->perm_s, N));
   CK(dalloc(&S->pos_s, N));
+  CK(dalloc(&S->posf, N));
   CK(dalloc(&S->vx_s, N)); CK(dalloc(&S->vy_s, N)); CK(dalloc(&S->vz_s, N));
   CK(dalloc(&S->ax_s, N)); CK(dalloc(&S->ay_s, N)); CK(dalloc(&S->az_s, N));
   CK(dalloc(&S->sx, N)); CK(dalloc(&S->sy, N)); CK(dalloc(&S->sz, N));
@@ -262,7 +264,7 @@ extern "C" int clmd_destroy(clmd_system* S) {
   cudaStreamSynchronize(S->stream);
   free_graphs(S);
   void* ps[] = {S->pos, S->pos_alt, S->red, S->vx, S->vy, S->vz, S->ax, S->ay, S->az, S->api, S->perm, S->iperm,
-                S->perm_s, S->pos_s, S->vx_s, S->vy_s, S->vz_s, S->ax_s, S->ay_s, S->az_s,
+                S->perm_s, S->pos_s, S->posf, S->vx_s, S->vy_s, S->vz_s, S->ax_s, S->ay_s, S->az_s,
                 S->liqref, S->sx, S->sy,
                 S->sz, S->vxn, S->vyn, S->vzn, S->list, S->row_start, S->row_len, S->row_lo,
                 S->cell_count, S->cell_start, S->cell_fill, S->cell_atoms, S->atom_cell,

@@ -122,9 +122,8 @@ __global__ void k_clu_bonds(Params P, DevState* st, const double4* pos, const in
     double4 pj = pos[j];
     int sj = (int)pj.w;
     if (!fre && sj != 1) break;
-    double dx = mimage_bf(pi.x - pj.x, P.boxx, P.ibx, bf1, bf2);
-    double dy = mimage_bf(pi.y - pj.y, P.boxy, P.iby, bf1, bf2);
-    double dz = mimage_bf(pi.z - pj.z, P.boxz, P.ibz, bf1, bf2);
+    double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+    mimage_bf3(P, dx, dy, dz, bf1, bf2);
     double rij2 = dx * dx + dy * dy + dz * dz;
     if (rij2 <= P.atskin2) {
       uf_union(parent, perm, i, j);

@@ -29,9 +29,12 @@
 
 namespace clmd {
 
-constexpr int kPB = 256;          // threads per block
+#ifndef CLMD_PB
+#define CLMD_PB 512
+#endif
+constexpr int kPB = CLMD_PB;      // threads per block
 #ifndef CLMD_CYCLE_MINB
-#define CLMD_CYCLE_MINB 4         // resident blocks per SM the registers must allow
+#define CLMD_CYCLE_MINB (1024 / CLMD_PB)         // resident blocks per SM the registers must allow
 #endif
 constexpr int kRedSlots = 16;     // partial-sum slots per buffer
 
@@ -107,6 +110,31 @@ __device__ __forceinline__ double get_max(const double* buf, int slot, double* s
   return r;
 }
 
+constexpr int kTileLog = 11, kMaxTiles = 2048;
+
+// exclusive scan over the block (sh: a warp's sum each); total: the block's
+__device__ __forceinline__ int block_scan(int v, int* sh, int& total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  __syncthreads();
+  if (lane == 31) sh[w] = incl;
+  __syncthreads();
+  int before = 0;
+  total = 0;
+#pragma unroll
+  for (int k = 0; k < kPB / 32; k++) {
+    const int t = sh[k];
+    before += k < w ? t : 0;
+    total += t;
+  }
+  return before + incl - v;
+}
+
 // The list rebuild, in place: positions wrapped and, with the velocities and
 // perm, put in cell order (gathered into pos_s, vx_s.., perm_s; the search
 // reads the new order there and copies each slot back as it takes it).
@@ -115,13 +143,17 @@ __device__ __forceinline__ double get_max(const double* buf, int slot, double* s
 // drift (the last reader of a step's accelerations) and the force pass that
 // overwrites them, so there they are not moved
 static __device__ bool rebuild(const Params& P, DevState* st, Blk& B, const CycleArgs& A,
-                               double4* pos, double* sh, bool acc) {
+                               double4* pos, WarpStage* stage, bool acc) {
   const int N = P.N;
   const int G = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
   const Geo& g = B.g;
-  // R1: histogram of the wrapped positions (neighbor-pbc-mav.f:67-71; the
-  // gather below stores them wrapped)
+  __shared__ int ssh[kPB / 32];
+  int* toff = (int*)stage;  // [kMaxTiles], until the search
+  static_assert(sizeof(WarpStage) * (kPB / 32) >= sizeof(int) * kMaxTiles, "tile offsets");
+  // R1: histogram of the wrapped positions (neighbor-pbc-mav.f:67-71; R4
+  // stores them wrapped); the count before an atom's own is its arrival
+  // number in the cell (kept in row_lo, dead until the search writes it)
   if (t0 == 0) st->list_used = 0ull;
   for (int p = t0; p < N; p += G) {
     const double4 v = wrap_box(P, pos[p]);
@@ -130,120 +162,102 @@ static __device__ bool rebuild(const Params& P, DevState* st, Blk& B, const Cycl
     int cz = min((int)(v.z * g.cfz), g.ncz - 1);
     int c = (cz * g.ncy + cy) * g.ncx + cx;
     A.atom_cell[p] = c;
-    atomicAdd(&A.cell_count[c], 1);
+    A.row_lo[p] = atomicAdd(&A.cell_count[c], 1);
   }
   if (!gbar(st)) return false;
-  // R2: tile sums
+  // R2: per tile of cells an exclusive scan (into cell_fill) and its sum;
+  // the counts go back to zero.  At most kMaxTiles tiles, so that every
+  // block can hold the tiles' offsets in shared memory
   const int ncell = g.ncell;
-  const int ntiles = (ncell + kScanTile - 1) / kScanTile;
-  constexpr int per = kScanTile / kPB;
+  int tlog = kTileLog;
+  while (((ncell - 1) >> tlog) >= kMaxTiles) tlog++;
+  const int ntiles = ((ncell - 1) >> tlog) + 1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int b = blockIdx.x; b < ntiles; b += gridDim.x) {
-    int base = b * kScanTile, s = 0;
-    for (int k = 0; k < per; k++) {
-      int c = base + threadIdx.x * per + k;
-      if (c < ncell) s += A.cell_count[c];
+    constexpr int per = (1 << kTileLog) / kPB;
+    int carry = 0;
+    for (int sub = 0; sub < 1 << (tlog - kTileLog); sub++) {
+      const int c0 = (b << tlog) + (sub << kTileLog) + threadIdx.x * per;
+      int n[per], s = 0;
+#pragma unroll
+      for (int k = 0; k < per; k++) {
+        n[k] = c0 + k < ncell ? __ldcg(A.cell_count + c0 + k) : 0;
+        s += n[k];
+      }
+      int total;
+      int ex = carry + block_scan(s, ssh, total);
+#pragma unroll
+      for (int k = 0; k < per; k++) {
+        if (c0 + k < ncell) {
+          A.cell_fill[c0 + k] = ex;
+          A.cell_count[c0 + k] = 0;
+        }
+        ex += n[k];
+      }
+      carry += total;
     }
-    double t = block_sum((double)s, sh);
-    if (threadIdx.x == 0) A.scan_aux[b] = (int)t;
+    if (threadIdx.x == 0) A.scan_aux[b] = carry;
   }
   if (!gbar(st)) return false;
-  // R3: offsets of each tile, exclusive scan inside it, counts cleared
-  __shared__ int ssh[33];
-  for (int b = blockIdx.x; b < ntiles; b += gridDim.x) {
-    double pre = 0.0;
-    for (int k = threadIdx.x; k < b; k += blockDim.x) pre += (double)__ldcg(A.scan_aux + k);
-    double pt = block_sum(pre, sh);
-    __shared__ int tile_off;
-    if (threadIdx.x == 0) tile_off = (int)pt;
-    __syncthreads();
-    int base = b * kScanTile;
-    int loc[per];
-    int s = 0;
-    for (int k = 0; k < per; k++) {
-      int c = base + threadIdx.x * per + k;
-      loc[k] = c < ncell ? A.cell_count[c] : 0;
+  // R3: every block scans the tiles' sums; the atoms' reference numbers go
+  // to their cells in arrival order, and the cells get their final starts
+  {
+    constexpr int kT = kMaxTiles / kPB;
+    int s = 0, loc[kT];
+#pragma unroll
+    for (int k = 0; k < kT; k++) {
+      const int t = threadIdx.x * kT + k;
+      loc[k] = t < ntiles ? __ldcg(A.scan_aux + t) : 0;
       s += loc[k];
     }
-    // block exclusive scan of s
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int incl = s;
+    int total;
+    int ex = block_scan(s, ssh, total);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (lane == 31) ssh[w] = incl;
-    __syncthreads();
-    if (w == 0) {
-      int v = lane < nw ? ssh[lane] : 0;
-      int vi = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, vi, o);
-        if (lane >= o) vi += t;
-      }
-      if (lane < nw) ssh[lane] = vi - v;
-    }
-    __syncthreads();
-    int ex = tile_off + ssh[w] + incl - s;
-    for (int k = 0; k < per; k++) {
-      int c = base + threadIdx.x * per + k;
-      if (c < ncell) {
-        A.cell_start[c] = ex;
-        A.cell_fill[c] = ex;
-        A.cell_count[c] = 0;
-      }
+    for (int k = 0; k < kT; k++) {
+      toff[threadIdx.x * kT + k] = ex;
       ex += loc[k];
     }
     __syncthreads();
   }
+  for (int p = t0; p < N; p += G) {
+    const int c = A.atom_cell[p];
+    A.cell_atoms[__ldcg(A.cell_fill + c) + toff[c >> tlog] + A.row_lo[p]] = A.perm[p];
+  }
+  for (int c = t0; c < ncell; c += G) A.cell_start[c] = __ldcg(A.cell_fill + c) + toff[c >> tlog];
   if (t0 == 0) A.cell_start[ncell] = N;
   if (!gbar(st)) return false;
-  // R4: counting-sort scatter
+  // R4: each atom's place is its cell's start plus the number of smaller
+  // reference indices in the cell; its state goes there in the scratch arrays
   for (int p = t0; p < N; p += G) {
-    int slot = atomicAdd(&A.cell_fill[A.atom_cell[p]], 1);
-    A.cell_atoms[slot] = p;
+    const int c = A.atom_cell[p], ref = A.perm[p];
+    const int c0 = __ldcg(A.cell_start + c), c1 = __ldcg(A.cell_start + c + 1);
+    const double4 v = wrap_box(P, pos[p]);
+    int q = c0;
+    for (int k = c0; k < c1; k++) q += __ldcg(A.cell_atoms + k) < ref;
+    A.pos_s[q] = v;
+    A.posf[q] = make_float4((float)v.x, (float)v.y, (float)v.z, __int_as_float(ref));
+    A.vx_s[q] = A.vx[p];
+    A.vy_s[q] = A.vy[p];
+    A.vz_s[q] = A.vz[p];
+    if (acc) {
+      A.ax_s[q] = A.ax[p];
+      A.ay_s[q] = A.ay[p];
+      A.az_s[q] = A.az[p];
+    }
+    A.perm_s[q] = ref;
   }
   if (!gbar(st)) return false;
-  // R5: per cell: order by reference index, gather into scratch
-  for (int c = t0; c < ncell; c += G) {
-    int c0 = A.cell_start[c], c1 = A.cell_start[c + 1];
-    for (int a = c0 + 1; a < c1; a++) {
-      int key = A.cell_atoms[a], kr = A.perm[key];
-      int b = a - 1;
-      while (b >= c0 && A.perm[A.cell_atoms[b]] > kr) {
-        A.cell_atoms[b + 1] = A.cell_atoms[b];
-        b--;
-      }
-      A.cell_atoms[b + 1] = key;
-    }
-    for (int q = c0; q < c1; q++) {
-      int o = A.cell_atoms[q];
-      A.pos_s[q] = wrap_box(P, pos[o]);
-      A.vx_s[q] = A.vx[o];
-      A.vy_s[q] = A.vy[o];
-      A.vz_s[q] = A.vz[o];
-      if (acc) {
-        A.ax_s[q] = A.ax[o];
-        A.ay_s[q] = A.ay[o];
-        A.az_s[q] = A.az[o];
-      }
-      A.perm_s[q] = A.perm[o];
-    }
-  }
-  if (!gbar(st)) return false;
-  // R6: rows (neighbor-pbc-mav.f:73-99), warp-aligned grid-stride, over the
+  // R5: rows (neighbor-pbc-mav.f:73-99), warp-aligned grid-stride, over the
   // new order in the scratch arrays; each slot is committed (copied back)
   // by the thread that takes it
   const double4* npos = A.pos_s;
   const int* perm = A.perm_s;
-  const int lane = threadIdx.x & 31;
   for (int base0 = t0 - lane; base0 < N; base0 += G) {
     int p = base0 + lane;
     bool active = p < N;
     int cnt = 0, refi = 0;
     double4 pi = make_double4(0, 0, 0, 0);
-    int bq[kRowBufC], bref[kRowBufC];
+    int2* buf = (int2*)&stage[w] + lane;
     if (active) {
       pi = npos[p];
       refi = perm[p];
@@ -258,7 +272,7 @@ static __device__ bool rebuild(const Params& P, DevState* st, Blk& B, const Cycl
       }
       A.perm[p] = refi;
       A.iperm[refi] = p;
-      cnt = scan_cells<false>(P, g, p, refi, pi, npos, perm, A.cell_start, bq, bref, nullptr);
+      cnt = row_search(P, g, p, refi, pi, npos, A.posf, A.cell_start, buf, nullptr);
     }
     int incl = cnt;
 #pragma unroll
@@ -266,49 +280,22 @@ static __device__ bool rebuild(const Params& P, DevState* st, Blk& B, const Cycl
       int t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
-    unsigned long long wbase = 0;
-    if (lane == 31) wbase = atomicAdd(&st->list_used, (unsigned long long)incl);
-    wbase = __shfl_sync(0xffffffffu, wbase, 31);
-    if (!active) continue;
-    unsigned long long start = wbase + (unsigned long long)(incl - cnt);
+    unsigned long long start = 0;
+    if (lane == 31) start = atomicAdd(&st->list_used, (unsigned long long)incl);
+    start = __shfl_sync(0xffffffffu, start, 31) + (unsigned long long)(incl - cnt);
+    int lo = 0, longer = 0;
     if (start + (unsigned long long)cnt > (unsigned long long)P.list_cap) {
       raise_err(st, CLMD_ERR_LIST_OVERFLOW);
-      A.row_start[p] = 0;
-      A.row_len[p] = 0;
-      A.row_lo[p] = 0;
-      continue;
-    }
-    int* row = A.list + start;
-    int lo = 0;
-    if (cnt <= kRowBufC) {
-      for (int a = 1; a < cnt; a++) {
-        int kr = bref[a], kq = bq[a];
-        int b = a - 1;
-        while (b >= 0 && bref[b] > kr) {
-          bref[b + 1] = bref[b];
-          bq[b + 1] = bq[b];
-          b--;
-        }
-        bref[b + 1] = kr;
-        bq[b + 1] = kq;
-      }
-      for (int a = 0; a < cnt; a++) {
-        row[a] = bq[a];
-        lo += bref[a] < refi;
-      }
+      start = 0;
+      cnt = 0;
+    } else if (cnt > kRowCap) {
+      longer = cnt;
+      row_search(P, g, p, refi, pi, npos, A.posf, A.cell_start, nullptr, A.list + start);
     } else {
-      scan_cells<true>(P, g, p, refi, pi, npos, perm, A.cell_start, nullptr, nullptr, row);
-      for (int a = 1; a < cnt; a++) {
-        int kq = row[a], kr = perm[kq];
-        int b = a - 1;
-        while (b >= 0 && perm[row[b]] > kr) {
-          row[b + 1] = row[b];
-          b--;
-        }
-        row[b + 1] = kq;
-      }
-      for (int a = 0; a < cnt; a++) lo += perm[row[a]] < refi;
+      lo = row_store(buf, cnt, refi, A.list + start);
     }
+    sort_long_rows(A.list, perm, start, longer, refi, lo);
+    if (!active) continue;
     A.row_start[p] = (int)start;
     A.row_len[p] = cnt;
     A.row_lo[p] = lo;
@@ -338,6 +325,7 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
   if (gated(st)) return;
   __shared__ Blk B;
   __shared__ double sh[kPB / 32];
+  extern __shared__ __align__(16) WarpStage stage[];  // [kPB / 32]
   const int N = P.N;
   const int G = gridDim.x * blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -370,7 +358,7 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
       prologue(P, B, step);
     }
     __syncthreads();
-    if (!B.stop) rebuild(P, st, B, A, posb(0), sh, true);
+    if (!B.stop) rebuild(P, st, B, A, posb(0), stage, true);
     goto done;
   }
 
@@ -473,7 +461,7 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
         rb ^= 1;
         if (B.stop) goto done;
         if (B.rebuild) {
-          if (!rebuild(P, st, B, A, posb(cur), sh, false)) goto stop_or_timeout;
+          if (!rebuild(P, st, B, A, posb(cur), stage, false)) goto stop_or_timeout;
         }
       }
       // ---- forces (+ kick, + next drift)
@@ -490,7 +478,6 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
         double esum = 0.0, vir = 0.0, ek = 0.0, d2 = 0.0, dp = 0.0, sv = 0.0;
         const double psi = B.q.psi;
         const double dth = dt / 2, m = P.apmas[0], Q = P.Q;
-        __shared__ WarpStage stage[kPB / 32];
         WarpStage& W = stage[threadIdx.x >> 5];
         const int lane = threadIdx.x & 31;
         bool bad = false;  // (raised in st->err_new too)
@@ -504,7 +491,8 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
           // lane 0 is active whenever the warp is; only its row start is used
           warp_forces<MIXED>(P, st, pos, A.list, lane == 0 ? A.row_start[p] : 0,
                       act ? A.row_len[p] : 0,
-                      act ? A.row_lo[p] : 0, pa, bf1, bf2, f.fx, f.fy, f.fz, f.esum, f.vir, W, bad);
+                      act ? A.row_lo[p] : 0, pa, bf1, bf2, f.fx, f.fy, f.fz, f.esum, f.vir,
+                      last, W, bad);
           // lanes past N still evaluated pair terms of their warp's atoms
           esum = esum + f.esum;
           vir = vir + f.vir;
@@ -829,6 +817,7 @@ static CycleArgs cycle_args(clmd_system* S) {
   A.vx_s = S->vx_s; A.vy_s = S->vy_s; A.vz_s = S->vz_s;
   A.ax_s = S->ax_s; A.ay_s = S->ay_s; A.az_s = S->az_s;
   A.perm_s = S->perm_s;
+  A.posf = S->posf;
   A.cell_count = S->cell_count; A.cell_start = S->cell_start; A.cell_fill = S->cell_fill;
   A.cell_atoms = S->cell_atoms; A.atom_cell = S->atom_cell; A.scan_aux = S->scan_aux;
   A.list = S->list; A.row_start = S->row_start; A.row_len = S->row_len; A.row_lo = S->row_lo;
@@ -843,10 +832,13 @@ static CycleKernel cycle_kernel(const clmd_system* S) {
   return th ? k_cycle<false, true, false> : k_cycle<false, false, false>;
 }
 
+constexpr int kStageBytes = (kPB / 32) * (int)sizeof(WarpStage);
+
 int cycle_blocks_for(clmd_system* S) {
   small_setup(S);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cycle_kernel(S), kPB, 0);
+  cudaFuncSetAttribute(cycle_kernel(S), cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cycle_kernel(S), kPB, kStageBytes);
   if (per_sm < 1) per_sm = 1;
   int nb = S->num_sms * per_sm;
   int need = (S->P.N + kPB - 1) / kPB;
@@ -864,6 +856,7 @@ void cycle_launch(clmd_system* S, int nsteps, int mode) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S->cyc_blocks);
   cfg.blockDim = dim3(kPB);
+  cfg.dynamicSmemBytes = kStageBytes;
   cfg.stream = S->stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;

@@ -11,13 +11,15 @@
 namespace clmd {
 
 constexpr int kSmallThreads = 512; // threads per CTA of the small-system kernel at most
-constexpr int kRowBufC = 32;      // candidate buffer of the list search
-
 struct Geo {
   double rs2, cfx, cfy, cfz;
   int ncx, ncy, ncz, ncell;
   int nox, noy, noz, pad;
   int offx[3], offy[3], offz[3];
+  // the FP32 list test: r^2 below flo is a neighbour, above fhi is none; in
+  // between the FP64 test decides
+  float flo, fhi;
+  int sel;  // a dimension has fewer than three cells: images per pair
 };
 
 struct Blk {
@@ -77,6 +79,16 @@ static __device__ void prologue(const Params& P, Blk& B, int step) {
   g.cfx = (double)g.ncx / P.boxx;
   g.cfy = (double)g.ncy / P.boxy;
   g.cfz = (double)g.ncz / P.boxz;
+  g.sel = g.ncx < 3 || g.ncy < 3 || g.ncz < 3;
+  {
+    // FP32 coordinates in [0, L] and shifted by L are off by at most
+    // e = 4 L 2^-24 together; r^2 by 2 e (|dx| + |dy| + |dz|) + 3 e^2 and its
+    // own few roundings
+    const double e = fmax(fmax(P.boxx, P.boxy), P.boxz) * 2.4e-7;
+    const double band = 4.0 * e * q.atrskin + 3.0 * e * e + 1e-6 * g.rs2;
+    g.flo = (float)(g.rs2 - band);
+    g.fhi = (float)(g.rs2 + band);
+  }
   q.dmmax = fmax(q.dmms, q.dmmax);  // :101-105
   q.dmms = 0.0;
   q.dmmst = 0;
@@ -110,74 +122,6 @@ __device__ __forceinline__ bool nbt(const Params& P, double rs2, const double4& 
   return r2 <= rs2;
 }
 
-// the candidate slots of a cell row: [a0, b0) and, where the x-neighbours
-// wrap, [a1, b1) (scalars, not arrays indexed by the range: those would live
-// in local memory)
-__device__ __forceinline__ int xr(const Geo& g, const int* cs, int row, int cx, int& a0,
-                                  int& b0, int& a1, int& b1) {
-  int n = g.ncx;
-  if (n >= 3) {
-    if (cx >= 1 && cx <= n - 2) {
-      a0 = cs[row + cx - 1]; b0 = cs[row + cx + 2];
-      return 1;
-    }
-    if (cx == 0) {
-      a0 = cs[row]; b0 = cs[row + 2];
-      a1 = cs[row + n - 1]; b1 = cs[row + n];
-      return 2;
-    }
-    a0 = cs[row + n - 2]; b0 = cs[row + n];
-    a1 = cs[row]; b1 = cs[row + 1];
-    return 2;
-  }
-  a0 = cs[row];
-  b0 = cs[row + n];
-  return 1;
-}
-
-template <bool FILL>
-__device__ __forceinline__ int scan_cells(const Params& P, const Geo& g, int p, int refi,
-                                          const double4& pi, const double4* pos,
-                                          const int* perm, const int* cs, int* bq, int* bref,
-                                          int* out) {
-  int cx = min((int)(pi.x * g.cfx), g.ncx - 1);
-  int cy = min((int)(pi.y * g.cfy), g.ncy - 1);
-  int cz = min((int)(pi.z * g.cfz), g.ncz - 1);
-  int n = 0;
-  for (int a = 0; a < g.noz; a++) {
-    int zz = cz + g.offz[a];
-    zz += (zz < 0) ? g.ncz : 0;
-    zz -= (zz >= g.ncz) ? g.ncz : 0;
-    for (int b = 0; b < g.noy; b++) {
-      int yy = cy + g.offy[b];
-      yy += (yy < 0) ? g.ncy : 0;
-      yy -= (yy >= g.ncy) ? g.ncy : 0;
-      int row = (zz * g.ncy + yy) * g.ncx;
-      int a0, b0, a1 = 0, b1 = 0;
-      const int nr = xr(g, cs, row, cx, a0, b0, a1, b1);
-      for (int r = 0; r < nr; r++) {
-        const int qb = r ? b1 : b0;
-        for (int q = r ? a1 : a0; q < qb; q++) {
-          if (q == p) continue;
-          double4 pq = pos[q];
-          int refq = perm[q];
-          bool hit = (refi < refq) ? nbt(P, g.rs2, pi, pq) : nbt(P, g.rs2, pq, pi);
-          if (hit) {
-            if (FILL) {
-              out[n] = q;
-            } else if (n < kRowBufC) {
-              bq[n] = q;
-              bref[n] = refq;
-            }
-            n++;
-          }
-        }
-      }
-    }
-  }
-  return n;
-}
-
 // Rows longer than the search's buffer, one after the other by the whole
 // warp: lanes with n > 0 name a row of n entries (slots, in any order) that
 // starts at list[start]; each is put in ascending reference order, *lo gets
@@ -186,7 +130,7 @@ __device__ __forceinline__ int scan_cells(const Params& P, const Geo& g, int p, 
 // of smaller keys (distinct, so the places are a permutation); a longer row
 // is left to its lane's insertion sort.  A liquid droplet's rows run to ~130
 // entries, where one lane's insertion sort in memory took ~130 us.
-static __device__ void sort_long_rows(int* list, const int* perm, unsigned long long start, int n,
+static __device__ __noinline__ void sort_long_rows(int* list, const int* perm, unsigned long long start, int n,
                                       int refi, int& lo) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int kT = 8;
@@ -255,16 +199,27 @@ struct CycleArgs {
   double4* pos_s;
   double *vx_s, *vy_s, *vz_s, *ax_s, *ay_s, *az_s;
   int* perm_s;
+  float4* posf;  // positions in FP32, reference index in .w, in cell order
   int *cell_count, *cell_start, *cell_fill, *cell_atoms, *atom_cell, *scan_aux;
   int *list, *row_start, *row_len, *row_lo;
   double* red;  // 2 x kRedSlots x gridDim partials
 };
 
-// neighbor-pbc-mav.f:67-71
+// neighbor-pbc-mav.f:67-71, dmod(dmod(x, L) + L, L).  Within one box length
+// of the box both dmods are a subtraction or nothing, exact either way (of
+// neighbouring binades at most), so the result is the same bits without the
+// two library calls
+__device__ __forceinline__ double wrap_1(double x, double L) {
+  if (x > -L && x < L + L) {
+    const double u = (x >= L ? x - L : x) + L;
+    return u >= L + L ? u - (L + L) : u >= L ? u - L : u;
+  }
+  return fmod(fmod(x, L) + L, L);
+}
 __device__ __forceinline__ double4 wrap_box(const Params& P, double4 v) {
-  v.x = fmod(fmod(v.x, P.boxx) + P.boxx, P.boxx);
-  v.y = fmod(fmod(v.y, P.boxy) + P.boxy, P.boxy);
-  v.z = fmod(fmod(v.z, P.boxz) + P.boxz, P.boxz);
+  v.x = wrap_1(v.x, P.boxx);
+  v.y = wrap_1(v.y, P.boxy);
+  v.z = wrap_1(v.z, P.boxz);
   return v;
 }
 
@@ -297,7 +252,8 @@ __device__ __forceinline__ void warp_forces(const Params& P, DevState* st, const
                                             const int* list, int st0, int len, int lo,
                                             const double4& pa, double bf1, double bf2,
                                             double& fx, double& fy, double& fz, double& esum,
-                                            double& vir, WarpStage& W, bool& bad) {
+                                            double& vir, bool energies, WarpStage& W,
+                                            bool& bad) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int e = len;
@@ -348,9 +304,7 @@ __device__ __forceinline__ void warp_forces(const Params& P, DevState* st, const
       } else {
         dx = pb.x - ox; dy = pb.y - oy; dz = pb.z - oz;
       }
-      dx = mimage_bf(dx, P.boxx, P.ibx, bf1, bf2);
-      dy = mimage_bf(dy, P.boxy, P.iby, bf1, bf2);
-      dz = mimage_bf(dz, P.boxz, P.ibz, bf1, bf2);
+      mimage_bf3(P, dx, dy, dz, bf1, bf2);
       double rij2 = dx * dx + dy * dy + dz * dz;
       if (rij2 <= P.atr2) {
         double r2 = rij2;
@@ -366,25 +320,21 @@ __device__ __forceinline__ void warp_forces(const Params& P, DevState* st, const
         } else if (mixed) {
           double e, w;
           pair_term_f32(P, ij, r2, dx, dy, dz, tx, ty, tz, e, w);
-          if (own) {
+          if (own && energies) {
             esum = esum + e;
             vir = vir + w;
-            flag = 1;
-          } else {
-            flag = 2;
           }
+          flag = own ? 1 : 2;
         } else {
           double fij = pair_fij(P, ij, rij2, rij6);
           tx = fij * dx;
           ty = fij * dy;
           tz = fij * dz;
-          if (own) {
+          if (own && energies) {
             esum = esum + pair_e(P, ij, rij6);
             vir = vir + fij * r2;
-            flag = 1;
-          } else {
-            flag = 2;
           }
+          flag = own ? 1 : 2;
         }
       }
     }
@@ -456,6 +406,124 @@ __device__ __forceinline__ int sp_block(const Params& P, int ref) {
   for (int s = 0; s < P.atsorts; s++)
     if (ref >= P.sp_start[s] && ref < P.sp_start[s + 1]) return s;
   return -1;
+}
+
+// the search's hits of one thread, until its row is written: in the
+// pair-force stage's memory, not in use then (entry k of lane l at
+// [32 k + l]; arrays of a thread's own would live in local memory)
+constexpr int kRowCap = (int)(sizeof(WarpStage) / 32 / 8);
+
+// neighbor-pbc-mav.f:73-99: the neighbours of one atom (slot p, wrapped
+// position pa) among the cells around it, into buf (the first kRowCap) or all
+// of them into out; returns their number.  cf: the atoms' positions in FP32
+// with the reference index in .w, in cell order.
+// The test is FP32 (with three or more cells per dimension the image is the
+// cell range's shift) and FP64, the reference's expression, only within the
+// FP32 rounding of the list radius: the same list, a quarter of the FP64
+// instructions, and 16 bytes a candidate instead of 36.  Two candidates are
+// loaded at a time and the next cell row's range ahead of this one's tests:
+// a thread's chain of loads, not their number, bounds the search.
+__device__ __forceinline__ int row_search(const Params& P, const Geo& g, int p, int ref,
+                                          const double4& pa, const double4* pos,
+                                          const float4* cf, const int* cs, int2* buf, int* out) {
+  const int ncx = g.ncx, ncy = g.ncy, ncz = g.ncz, noy = g.noy, noz = g.noz;
+  const int cx = min((int)(pa.x * g.cfx), ncx - 1);
+  const int cy = min((int)(pa.y * g.cfy), ncy - 1);
+  const int cz = min((int)(pa.z * g.cfz), ncz - 1);
+  const float lx = (float)P.boxx, ly = (float)P.boxy, lz = (float)P.boxz;
+  const float px = (float)pa.x, py = (float)pa.y, pz = (float)pa.z;
+  const float flo = g.flo, fhi = g.fhi;
+  const bool sel = g.sel != 0;
+  // the cells of a row: [xa, xb), and the one the row wraps to (edge), at a
+  // box length's shift
+  const int xa = ncx < 3 ? 0 : max(cx - 1, 0), xb = ncx < 3 ? ncx : min(cx + 2, ncx);
+  const bool edge = ncx >= 3 && (cx == 0 || cx == ncx - 1);
+  const int xw = cx == 0 ? ncx - 1 : 0;
+  const float wx = sel ? 0.f : (cx == 0 ? lx : -lx);
+  int n = 0, ka = 0, kb = 0;
+  float ny, nz;  // the next row's image shifts
+  int a0, b0, a1 = 0, b1 = 0;
+  auto next = [&]() {  // cell ranges and shifts of row (ka, kb), then on to the next
+    int zz = cz + ka - (noz == 3), yy = cy + kb - (noy == 3);
+    nz = sel ? 0.f : (zz < 0 ? lz : (zz >= ncz ? -lz : 0.f));
+    ny = sel ? 0.f : (yy < 0 ? ly : (yy >= ncy ? -ly : 0.f));
+    zz += zz < 0 ? ncz : (zz >= ncz ? -ncz : 0);
+    yy += yy < 0 ? ncy : (yy >= ncy ? -ncy : 0);
+    const int* row = cs + (zz * ncy + yy) * ncx;
+    a0 = row[xa];
+    b0 = row[xb];
+    if (edge) {
+      a1 = row[xw];
+      b1 = row[xw + 1];
+    }
+    if (++kb == noy) {
+      kb = 0;
+      ka++;
+    }
+  };
+  auto test = [&](const float4& c, int q, float x, float y, float z) {
+    float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+    if (sel) {
+      dx -= fabsf(dx) > 0.5f * lx ? copysignf(lx, dx) : 0.f;
+      dy -= fabsf(dy) > 0.5f * ly ? copysignf(ly, dy) : 0.f;
+      dz -= fabsf(dz) > 0.5f * lz ? copysignf(lz, dz) : 0.f;
+    }
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    if (!(r2 <= fhi) || q == p) return;  // (a NaN is no neighbour)
+    const int refq = __float_as_int(c.w);
+    if (!(r2 < flo)) {
+      const double4 pq = pos[q];
+      if (!((ref < refq) ? nbt(P, g.rs2, pa, pq) : nbt(P, g.rs2, pq, pa))) return;
+    }
+    if (out)
+      out[n] = q;
+    else if (n < kRowCap)
+      buf[n * 32] = make_int2(q, refq);
+    n++;
+  };
+  next();
+  for (bool more = true; more;) {
+    int q = a0, e = b0;
+    const int q1 = a1, e1 = edge ? b1 : a1;
+    const float y = py + ny, z = pz + nz;
+    float x = px;
+    more = ka < noz;
+    if (more) next();
+    for (int part = 0;; part++) {
+#pragma unroll 1
+      for (; q < e; q += 2) {
+        const float4 c0 = cf[q], c1 = cf[min(q + 1, e - 1)];
+        test(c0, q, x, y, z);
+        if (q + 1 < e) test(c1, q + 1, x, y, z);
+      }
+      if (part || !edge) break;
+      q = q1;
+      e = e1;
+      x = px + wx;
+    }
+  }
+  return n;
+}
+
+// a row's hits in the buffer (n <= kRowCap) put in ascending reference order
+// and written out; returns how many lie below the owner's reference index
+__device__ __forceinline__ int row_store(int2* buf, int n, int ref, int* row) {
+  for (int k = 1; k < n; k++) {
+    const int2 e = buf[k * 32];
+    int b = k - 1;
+    while (b >= 0 && buf[b * 32].y > e.y) {
+      buf[(b + 1) * 32] = buf[b * 32];
+      b--;
+    }
+    buf[(b + 1) * 32] = e;
+  }
+  int lo = 0;
+  for (int k = 0; k < n; k++) {
+    const int2 e = buf[k * 32];
+    row[k] = e.x;
+    lo += e.y < ref;
+  }
+  return lo;
 }
 
 // clmd_small.cu: systems of up to 16 * kSmallThreads atoms

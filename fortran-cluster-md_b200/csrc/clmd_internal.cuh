@@ -32,6 +32,7 @@ constexpr int kScanTile = 2048;    // counts per block of the cell scan
 struct Params {
   double apmas[CLMD_MXSORTS];
   double boxx, boxy, boxz, ibx, iby, ibz;
+  double img;  // 0.49 times the shortest box length: nearer pairs need no image
   double dt, atrcut, atr2, atskin2, sig1;
   double c1[5], c2[5], c3[5], eps[5];
   double Q, att;
@@ -165,6 +166,27 @@ __device__ __forceinline__ double reduce_partials(const double* p, int n, double
 __device__ __forceinline__ double mimage_bf(double d, double L, double iL, double bf1,
                                             double bf2) {
   return d + L * (bf1 - (double)(int)(bf2 + d * iL));
+}
+
+// the three of them.  |d| < 0.49 L: the integer is bf1, the result d itself;
+// 0.51 L < |d| < 1.49 L: it is bf1 +- 1, the result d -+ L with the same
+// single rounding; only what lies nearer to a half box length (in no list
+// unless the box is tiny) needs the conversions to integer and back, which
+// cost more than the rest of the distance.
+__device__ __forceinline__ double mimage_far(double d, double L, double iL, double bf1,
+                                             double bf2) {
+  const double a = fabs(d);
+  if (a < 0.49 * L) return d;
+  if (a > 0.51 * L && a < 1.49 * L) return d - copysign(L, d);
+  return mimage_bf(d, L, iL, bf1, bf2);
+}
+__device__ __forceinline__ void mimage_bf3(const Params& P, double& dx, double& dy, double& dz,
+                                           double bf1, double bf2) {
+  if (!(fmax(fmax(fabs(dx), fabs(dy)), fabs(dz)) < P.img)) {
+    dx = mimage_far(dx, P.boxx, P.ibx, bf1, bf2);
+    dy = mimage_far(dy, P.boxy, P.iby, bf1, bf2);
+    dz = mimage_far(dz, P.boxz, P.ibz, bf1, bf2);
+  }
 }
 
 // LJ pair factor f_ij and energy term (for-a-lj-n-pbc-m.f:113-131); with

@@ -61,9 +61,7 @@ __global__ void __launch_bounds__(kBlock) k_force(Params P, DevState* st, const 
       } else {
         dx = pb.x - pa.x; dy = pb.y - pa.y; dz = pb.z - pa.z;
       }
-      dx = mimage_bf(dx, P.boxx, P.ibx, bf1, bf2);
-      dy = mimage_bf(dy, P.boxy, P.iby, bf1, bf2);
-      dz = mimage_bf(dz, P.boxz, P.ibz, bf1, bf2);
+      mimage_bf3(P, dx, dy, dz, bf1, bf2);
       double rij2 = dx * dx + dy * dy + dz * dz;
       if (rij2 <= P.atr2) {
         double r2 = rij2;

@@ -47,10 +47,6 @@ struct SmallShared {
   WarpStage stage[kSW];
 };
 
-// the search's hits of one thread, until its row is written: the pair-force
-// stage's memory (not in use then)
-constexpr int kRowCap = (int)(sizeof(WarpStage) / 32 / 8);
-
 struct Grp {
   int C, nw, rank, lane;
   int mine;  // this warp's number in the cluster
@@ -96,52 +92,6 @@ struct Atom {
   int start, len, lo;     // its list row
   bool act;
 };
-
-__device__ __forceinline__ void s_find(const Params& P, const Geo& g, const Atom& a, int p,
-                                       const double4* pos, const int* perm, const int* cs, int q,
-                                       int& n, int2* buf, int* out) {
-  if (q == p) return;
-  const double4 pq = pos[q];
-  const int refq = perm[q];
-  const bool hit = (a.ref < refq) ? nbt(P, g.rs2, a.q, pq) : nbt(P, g.rs2, pq, a.q);
-  if (!hit) return;
-  if (out)
-    out[n] = q;
-  else if (n < kRowCap)
-    buf[n * 32] = make_int2(q, refq);
-  n++;
-}
-
-// the neighbours of one atom among the 27 cells around it: into buf (the
-// first kRowCap), or all of them into out; the next cell row's range is
-// loaded while this one's candidates are tested
-__device__ __forceinline__ int s_search(const Params& P, const Geo& g, const Atom& a, int p,
-                                        const double4* pos, const int* perm, const int* cs,
-                                        int2* buf, int* out) {
-  const int cx = min((int)(a.q.x * g.cfx), g.ncx - 1);
-  const int cy = min((int)(a.q.y * g.cfy), g.ncy - 1);
-  const int cz = min((int)(a.q.z * g.cfz), g.ncz - 1);
-  const int rows = g.noz * g.noy;
-  auto row_at = [&](int k) {
-    const int kz = k / g.noy;
-    int zz = cz + g.offz[kz], yy = cy + g.offy[k - kz * g.noy];
-    zz += zz < 0 ? g.ncz : 0;
-    zz -= zz >= g.ncz ? g.ncz : 0;
-    yy += yy < 0 ? g.ncy : 0;
-    yy -= yy >= g.ncy ? g.ncy : 0;
-    return (zz * g.ncy + yy) * g.ncx;
-  };
-  int n = 0, a0, b0, a1 = 0, b1 = 0;
-  int nr = xr(g, cs, row_at(0), cx, a0, b0, a1, b1);
-  for (int k = 0; k < rows; k++) {
-    const int m = nr, c0 = a0, d0 = b0, c1 = a1, d1 = b1;
-    if (k + 1 < rows) nr = xr(g, cs, row_at(k + 1), cx, a0, b0, a1, b1);
-    for (int q = c0; q < d0; q++) s_find(P, g, a, p, pos, perm, cs, q, n, buf, out);
-    if (m > 1)
-      for (int q = c1; q < d1; q++) s_find(P, g, a, p, pos, perm, cs, q, n, buf, out);
-  }
-  return n;
-}
 
 // neighbor-pbc-mav.f:67-99: positions wrapped, atoms put in cell order (ties
 // by reference index, as k_cycle), rows searched and sorted.  acc: the
@@ -223,6 +173,7 @@ static __device__ bool s_rebuild(const Params& P, DevState* st, SmallShared& S, 
       A.az_s[dst] = a.az;
     }
     A.perm_s[dst] = a.ref;
+    A.posf[dst] = make_float4((float)a.q.x, (float)a.q.y, (float)a.q.z, __int_as_float(a.ref));
     A.iperm[a.ref] = dst;
   }
   G.barrier();
@@ -241,7 +192,7 @@ static __device__ bool s_rebuild(const Params& P, DevState* st, SmallShared& S, 
     a.ref = A.perm_s[p];
     A.perm[p] = a.ref;
     pos[p] = a.q;
-    cnt = s_search(P, g, a, p, A.pos_s, A.perm_s, A.cell_start, buf, nullptr);
+    cnt = row_search(P, g, p, a.ref, a.q, A.pos_s, A.posf, A.cell_start, buf, nullptr);
   }
   // one warp-wide cursor step: a warp's 32 rows are contiguous
   const int inc = s_pre(cnt, lane);
@@ -259,22 +210,9 @@ static __device__ bool s_rebuild(const Params& P, DevState* st, SmallShared& S, 
     a.start = a.len = 0;
   } else if (cnt > kRowCap) {
     longer = cnt;
-    s_search(P, g, a, p, A.pos_s, A.perm_s, A.cell_start, nullptr, A.list + base);
+    row_search(P, g, p, a.ref, a.q, A.pos_s, A.posf, A.cell_start, nullptr, A.list + base);
   } else {
-    for (int k = 1; k < cnt; k++) {
-      const int2 e = buf[k * 32];
-      int b = k - 1;
-      while (b >= 0 && buf[b * 32].y > e.y) {
-        buf[(b + 1) * 32] = buf[b * 32];
-        b--;
-      }
-      buf[(b + 1) * 32] = e;
-    }
-    for (int k = 0; k < cnt; k++) {
-      const int2 e = buf[k * 32];
-      A.list[base + k] = e.x;
-      a.lo += e.y < a.ref;
-    }
+    a.lo = row_store(buf, cnt, a.ref, A.list + base);
   }
   sort_long_rows(A.list, A.perm_s, base, longer, a.ref, a.lo);
   if (a.act) {
@@ -447,7 +385,7 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
         double fx, fy, fz, esum = 0.0, vir = 0.0, ek = 0.0, d2 = 0.0, sv = 0.0, dp = 0.0;
         bool bad = false;
         warp_forces<MIXED>(P, st, cur ? A.pos1 : A.pos0, A.list, a.start, a.len, a.lo, a.q, bf1,
-                           bf2, fx, fy, fz, esum, vir, W, bad);
+                           bf2, fx, fy, fz, esum, vir, last, W, bad);
         if (bad) G.put_err(CLMD_ERR_BAD_SPECIES);
         if (a.act) {
           const double mass = P.apmas[(int)a.q.w - 1], iatm = 1.0 / mass;

@@ -27,6 +27,7 @@ struct clmd_system {
   double *vx_s = nullptr, *vy_s = nullptr, *vz_s = nullptr;
   double *ax_s = nullptr, *ay_s = nullptr, *az_s = nullptr;
   int* perm_s = nullptr;
+  float4* posf = nullptr;
   double *sx = nullptr, *sy = nullptr, *sz = nullptr;     // staging / scratch
   double *vxn = nullptr, *vyn = nullptr, *vzn = nullptr;  // Nose-Hoover iterate
   // neighbour list
