@@ -189,7 +189,7 @@ extern "C" int clmd_create(const clmd_config* cfg, clmd_system** out) {
   CK(dalloc(&S->vx_s, N)); CK(dalloc(&S->vy_s, N)); CK(dalloc(&S->vz_s, N));
   CK(dalloc(&S->ax_s, N)); CK(dalloc(&S->ay_s, N)); CK(dalloc(&S->az_s, N));
   CK(dalloc(&S->sx, N)); CK(dalloc(&S->sy, N)); CK(dalloc(&S->sz, N));
-  CK(dalloc(&S->vxn, N)); CK(dalloc(&S->vyn, N)); CK(dalloc(&S->vzn, N));
+  CK(dalloc(&S->afx, N)); CK(dalloc(&S->afy, N)); CK(dalloc(&S->afz, N));
   CK(dalloc(&S->list, (size_t)cap));
   CK(dalloc(&S->row_start, N)); CK(dalloc(&S->row_len, N)); CK(dalloc(&S->row_lo, N));
   CK(dalloc(&S->cell_count, S->ncell_alloc + 1));
@@ -266,7 +266,7 @@ extern "C" int clmd_destroy(clmd_system* S) {
   void* ps[] = {S->pos, S->pos_alt, S->red, S->vx, S->vy, S->vz, S->ax, S->ay, S->az, S->api, S->perm, S->iperm,
                 S->perm_s, S->pos_s, S->posf, S->vx_s, S->vy_s, S->vz_s, S->ax_s, S->ay_s, S->az_s,
                 S->liqref, S->sx, S->sy,
-                S->sz, S->vxn, S->vyn, S->vzn, S->list, S->row_start, S->row_len, S->row_lo,
+                S->sz, S->afx, S->afy, S->afz, S->list, S->row_start, S->row_len, S->row_lo,
                 S->cell_count, S->cell_start, S->cell_fill, S->cell_atoms, S->atom_cell,
                 S->scan_aux, S->partials, S->st, S->parent, S->parent2, S->cl,
                 S->clf, S->cs, S->csf, S->csi, S->csif, S->cgs, S->cgsf, S->cgsa, S->cgsfa,

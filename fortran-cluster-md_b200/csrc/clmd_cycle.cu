@@ -7,9 +7,8 @@
 //
 //   velocity Verlet, per step:  [force_n + kick_n + drift_n+1] -> barrier
 //                               -> skin decision -> (rebuild: 7 barriers)
-//   Nose-Hoover, per step:      drift -> barrier -> (rebuild) -> force +
-//                               first sweep -> barrier -> one barrier per
-//                               further sweep of the implicit solve
+//   Nose-Hoover, per step:      [velocities_n + drift_n+1] -> barrier ->
+//                               (rebuild) -> force_n+1 -> barrier
 //
 // Forces of step n read the positions of step n while the fused drift writes
 // step n+1's, so positions are double-buffered (pos0/pos1); v and a are only
@@ -316,7 +315,7 @@ static __device__ bool rebuild(const Params& P, DevState* st, Blk& B, const Cycl
 }
 
 enum { SLOT_MAX = 0, SLOT_SUMV2 = 1, SLOT_EPOT = 2, SLOT_VIR = 3, SLOT_EKIN = 4,
-       SLOT_DELPS = 5, SLOT_NR = 6, SLOT_EK0 = 6 /* ek per species: 6..15 */ };
+       SLOT_WV = 5, SLOT_VV = 4, SLOT_EK0 = 6 /* ek per species: 6..15 */ };
 
 template <bool NH, bool THERMO, bool MIXED>
 __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevState* st,
@@ -475,9 +474,8 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
         // this is the launch's last step or velocities are rescaled first
         const bool keep64 = last || thermo;
         (void)keep64;
-        double esum = 0.0, vir = 0.0, ek = 0.0, d2 = 0.0, dp = 0.0, sv = 0.0;
-        const double psi = B.q.psi;
-        const double dth = dt / 2, m = P.apmas[0], Q = P.Q;
+        double esum = 0.0, vir = 0.0, ek = 0.0, d2 = 0.0, sv = 0.0, wv = 0.0, vv = 0.0;
+        const double dth = dt / 2;
         WarpStage& W = stage[threadIdx.x >> 5];
         const int lane = threadIdx.x & 31;
         bool bad = false;  // (raised in st->err_new too)
@@ -508,16 +506,13 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
             axi = fx32;
             ayi = fy32;
             azi = fz32;
-            if (keep64) {
-              A.ax[p] = axi;
-              A.ay[p] = ayi;
-              A.az[p] = azi;
-            } else {
+            if (!keep64) {
               A.afx[p] = fx32;
               A.afy[p] = fy32;
               A.afz[p] = fz32;
             }
-          } else {
+          }
+          if (!(MIXED && nh) || keep64) {
             A.ax[p] = axi;
             A.ay[p] = ayi;
             A.az[p] = azi;
@@ -546,24 +541,16 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
             A.vx[p] = vxi;
             A.vy[p] = vyi;
             A.vz[p] = vzi;
-          } else if (MIXED) {
+          } else {
             // closed-form solve (clmd_nh_root): sv = sum W^2, W = V + dth a
             // (the velocity pass forms W again from V and a)
-            double wx = A.vx[p] + dth * axi, wy = A.vy[p] + dth * ayi, wz = A.vz[p] + dth * azi;
+            const double vxi = A.vx[p], vyi = A.vy[p], vzi = A.vz[p];
+            const double wx = vxi + dth * axi, wy = vyi + dth * ayi, wz = vzi + dth * azi;
             sv = sv + wx * wx + wy * wy + wz * wz;
-          } else {
-            // int-verlet-nh-mav.f:94-120: vn = V, sumv2, first sweep's delps
-            double vxi = A.vx[p], vyi = A.vy[p], vzi = A.vz[p];
-            A.vxn[p] = vxi;
-            A.vyn[p] = vyi;
-            A.vzn[p] = vzi;
-            sv = sv + vxi * vxi + vyi * vyi + vzi * vzi;
-            double b = -dth * (axi - psi * vxi) - (vxi - vxi);
-            dp = dp + b * m * vxi * dt / Q;
-            b = -dth * (ayi - psi * vyi) - (vyi - vyi);
-            dp = dp + b * m * vyi * dt / Q;
-            b = -dth * (azi - psi * vzi) - (vzi - vzi);
-            dp = dp + b * m * vzi * dt / Q;
+            if (!MIXED && last) {  // for the count of the reference's sweeps
+              wv = wv + wx * vxi + wy * vyi + wz * vzi;
+              vv = vv + vxi * vxi + vyi * vyi + vzi * vzi;
+            }
           }
         }
         if (last) {
@@ -574,7 +561,10 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
         if (fuse) put_max(red(), SLOT_MAX, d2, sh);
         if (nh) {
           put_sum(red(), SLOT_SUMV2, sv, sh);
-          put_sum(red(), SLOT_DELPS, dp, sh);
+          if (!MIXED && last) {
+            put_sum(red(), SLOT_WV, wv, sh);
+            put_sum(red(), SLOT_VV, vv, sh);
+          }
         }
         if (!gbar(st)) goto timeout;
         if (__ldcg(&st->err_new) != 0) {
@@ -610,130 +600,14 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
       // ---- Nose-Hoover implicit solve (int-verlet-nh-mav.f:105-180)
       {
         const double dt2 = dt * dt / 2, dth = dt / 2, m = P.apmas[0], Q = P.Q;
-        const double err = 1.0e-10;
         const double psi = B.q.psi;
         double sumv2 = get_sum(red(), SLOT_SUMV2, sh, B.bcast);
-        double draw = get_sum(red(), SLOT_DELPS, sh, B.bcast);
+        const double swv = !MIXED && last ? get_sum(red(), SLOT_WV, sh, B.bcast) : 0.0;
+        const double svv = !MIXED && last ? get_sum(red(), SLOT_VV, sh, B.bcast) : 0.0;
         rb ^= 1;
-        if (MIXED) {
-          // every block solves the same scalar equation from the same sums
-          double pn;
-          if (!clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn)) {
-            if (threadIdx.x == 0 && B.q.status == 0) {
-              B.q.status = CLMD_ERR_NH_NOCONVERGE;
-              B.q.fail_step = step;
-            }
-            __syncthreads();
-            goto done;
-          }
-          // v = W c, fused with the next step's drift (the same expressions
-          // as the drift at the top of the step, PSI = pn) unless this is the
-          // launch's last step or velocities are rescaled before each step
-          const double c = 1.0 / (1.0 + dth * pn);
-          const bool fuse = !thermo && !last;
-          double d2 = 0.0, sv = 0.0;
-          double4* pos = posb(cur);
-          for (int p = t0; p < N; p += G) {
-            double axi, ayi, azi;
-            if (fuse) {
-              axi = A.afx[p];
-              ayi = A.afy[p];
-              azi = A.afz[p];
-            } else {
-              axi = A.ax[p];
-              ayi = A.ay[p];
-              azi = A.az[p];
-            }
-            double vxi = (A.vx[p] + dth * axi) * c, vyi = (A.vy[p] + dth * ayi) * c,
-                   vzi = (A.vz[p] + dth * azi) * c;
-            if (fuse) {
-              double dx = dt * vxi + dt2 * (axi - pn * vxi);
-              double dy = dt * vyi + dt2 * (ayi - pn * vyi);
-              double dz = dt * vzi + dt2 * (azi - pn * vzi);
-              sv = sv + vxi * vxi + vyi * vyi + vzi * vzi;
-              vxi = vxi + dth * (axi - pn * vxi);
-              vyi = vyi + dth * (ayi - pn * vyi);
-              vzi = vzi + dth * (azi - pn * vzi);
-              double4 q = pos[p];
-              q.x = q.x + dx;
-              q.y = q.y + dy;
-              q.z = q.z + dz;
-              pos[p] = q;
-              d2 = fmax(d2, dx * dx + dy * dy + dz * dz);
-            }
-            A.vx[p] = vxi;
-            A.vy[p] = vyi;
-            A.vz[p] = vzi;
-          }
-          if (threadIdx.x == 0) {
-            B.q.nh_iters = 1;
-            B.q.sumv2 = sumv2 * c * c;
-            B.q.psi = pn;
-            B.q.ekin = 0.5 * m * B.q.sumv2;
-          }
-          if (fuse) {
-            // the forces' reads of pos ended at the barrier before the root
-            put_max(red(), SLOT_MAX, d2, sh);
-            put_sum(red(), SLOT_SUMV2, sv, sh);
-            if (!gbar(st)) goto timeout;
-            drift_done = true;
-          } else {
-            __syncthreads();
-            drift_done = false;
-          }
-          continue;
-        }
-        double psn = psi;
-        int ready = 0, iter;
-        for (iter = 1; iter <= 1000; iter++) {
-          double pso = psn;
-          double di = -(pso * dth + 1);
-          double delps = draw - di * ((-m * sumv2 + P.nkt3_i) * dth / Q - (psi - pso));
-          delps = delps / (-dt2 * m * sumv2 / Q + di);
-          double pnext = pso + delps;
-          double s2 = 0.0, dp = 0.0;
-          int notready = 0;
-          for (int p = t0; p < N; p += G) {
-            double V[3] = {A.vx[p], A.vy[p], A.vz[p]};
-            double a[3] = {A.ax[p], A.ay[p], A.az[p]};
-            double* vn[3] = {A.vxn, A.vyn, A.vzn};
-            double nv[3];
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-              double vo = vn[d][p];
-              double b = -dth * (a[d] - pso * vo) - (V[d] - vo);
-              double nx = vo + (b + dth * vo * delps) / di;
-              if (fabs((nx - vo) / nx) > err) notready = 1;
-              nv[d] = nx;
-            }
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-              vn[d][p] = nv[d];
-              s2 = s2 + nv[d] * nv[d];
-            }
-            // the next sweep's delps terms (:110-120 with vo = this vn)
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-              double b = -dth * (a[d] - pnext * nv[d]) - (V[d] - nv[d]);
-              dp = dp + b * m * nv[d] * dt / Q;
-            }
-          }
-          put_sum(red(), SLOT_SUMV2, s2, sh);
-          put_sum(red(), SLOT_DELPS, dp, sh);
-          put_max(red(), SLOT_NR, (double)notready, sh);
-          if (!gbar(st)) goto timeout;
-          sumv2 = get_sum(red(), SLOT_SUMV2, sh, B.bcast);
-          draw = get_sum(red(), SLOT_DELPS, sh, B.bcast);
-          double nr = get_max(red(), SLOT_NR, sh, B.bcast);
-          rb ^= 1;
-          psn = pnext;
-          if (nr == 0.0) {
-            ready = 1;
-            break;
-          }
-        }
-        if (threadIdx.x == 0) B.q.nh_iters = ready ? iter : 1000;
-        if (!ready) {
+        // every block solves the same scalar equation from the same sums
+        double pn;
+        if (!clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn)) {
           if (threadIdx.x == 0 && B.q.status == 0) {
             B.q.status = CLMD_ERR_NH_NOCONVERGE;
             B.q.fail_step = step;
@@ -741,20 +615,72 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
           __syncthreads();
           goto done;
         }
-        // :171-180 write back (sumv2 of V = vn: same sum)
+        // v = W c, fused with the next step's drift (the same expressions
+        // as the drift at the top of the step, PSI = pn) unless this is the
+        // launch's last step or velocities are rescaled before each step
+        const double c = 1.0 / (1.0 + dth * pn);
+        const bool fuse = !thermo && !last;
+        double d2 = 0.0, sv = 0.0;
+        int sweeps = 1;
+        double4* pos = posb(cur);
         for (int p = t0; p < N; p += G) {
-          A.vx[p] = A.vxn[p];
-          A.vy[p] = A.vyn[p];
-          A.vz[p] = A.vzn[p];
+          double axi, ayi, azi;
+          if (MIXED && fuse) {
+            axi = A.afx[p];
+            ayi = A.afy[p];
+            azi = A.afz[p];
+          } else {
+            axi = A.ax[p];
+            ayi = A.ay[p];
+            azi = A.az[p];
+          }
+          const double V[3] = {A.vx[p], A.vy[p], A.vz[p]};
+          const double W[3] = {V[0] + dth * axi, V[1] + dth * ayi, V[2] + dth * azi};
+          double vxi = W[0] * c, vyi = W[1] * c, vzi = W[2] * c;
+          if (!MIXED && last)
+            sweeps = max(sweeps, clmd_nh_sweeps(W, V, sumv2, swv, svv, psi, m, P.nkt3_i, dt, Q));
+          if (fuse) {
+            double dx = dt * vxi + dt2 * (axi - pn * vxi);
+            double dy = dt * vyi + dt2 * (ayi - pn * vyi);
+            double dz = dt * vzi + dt2 * (azi - pn * vzi);
+            sv = sv + vxi * vxi + vyi * vyi + vzi * vzi;
+            vxi = vxi + dth * (axi - pn * vxi);
+            vyi = vyi + dth * (ayi - pn * vyi);
+            vzi = vzi + dth * (azi - pn * vzi);
+            double4 q = pos[p];
+            q.x = q.x + dx;
+            q.y = q.y + dy;
+            q.z = q.z + dz;
+            pos[p] = q;
+            d2 = fmax(d2, dx * dx + dy * dy + dz * dz);
+          }
+          A.vx[p] = vxi;
+          A.vy[p] = vyi;
+          A.vz[p] = vzi;
         }
         if (threadIdx.x == 0) {
-          B.q.sumv2 = sumv2;
-          B.q.psi = psn;
-          B.q.ekin = 0.5 * m * sumv2;
+          B.q.nh_iters = 1;
+          B.q.sumv2 = sumv2 * c * c;
+          B.q.psi = pn;
+          B.q.ekin = 0.5 * m * B.q.sumv2;
         }
-        __syncthreads();
-        drift_done = false;
-        // the next drift reads only this atom's v: no barrier needed
+        if (fuse) {
+          // the forces' reads of pos ended at the barrier before the root
+          put_max(red(), SLOT_MAX, d2, sh);
+          put_sum(red(), SLOT_SUMV2, sv, sh);
+          if (!gbar(st)) goto timeout;
+          drift_done = true;
+        } else {
+          __syncthreads();
+          drift_done = false;
+        }
+        if (!MIXED && last) {  // the sweeps the reference takes for this step
+          put_max(red(), SLOT_MAX, (double)sweeps, sh);
+          if (!gbar(st)) goto timeout;
+          const double n = get_max(red(), SLOT_MAX, sh, B.bcast);
+          if (threadIdx.x == 0) B.q.nh_iters = (int)n;
+          rb ^= 1;
+        }
       }
     }
   }
@@ -808,10 +734,7 @@ static CycleArgs cycle_args(clmd_system* S) {
   A.pos1 = S->pos_alt;
   A.vx = S->vx; A.vy = S->vy; A.vz = S->vz;
   A.ax = S->ax; A.ay = S->ay; A.az = S->az;
-  A.vxn = S->vxn; A.vyn = S->vyn; A.vzn = S->vzn;
-  A.afx = reinterpret_cast<float*>(S->vxn);
-  A.afy = reinterpret_cast<float*>(S->vyn);
-  A.afz = reinterpret_cast<float*>(S->vzn);
+  A.afx = S->afx; A.afy = S->afy; A.afz = S->afz;
   A.perm = S->perm; A.iperm = S->iperm;
   A.pos_s = S->pos_s;
   A.vx_s = S->vx_s; A.vy_s = S->vy_s; A.vz_s = S->vz_s;

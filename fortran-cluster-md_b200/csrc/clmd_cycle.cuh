@@ -190,10 +190,8 @@ struct CycleArgs {
   double4* pos0;
   double4* pos1;
   double *vx, *vy, *vz, *ax, *ay, *az;
-  double *vxn, *vyn, *vzn;
   // mixed Nose-Hoover: the accelerations between a step's force pass and its
-  // velocity pass, FP32 (the storage of the FP64 sweeps' iterate vxn..vzn,
-  // which that path does not use)
+  // velocity pass
   float *afx, *afy, *afz;
   int *perm, *iperm;
   double4* pos_s;

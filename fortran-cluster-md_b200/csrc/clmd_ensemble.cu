@@ -173,33 +173,8 @@ __device__ __forceinline__ void cta_sum2(double& a, double& b, int& f, double* s
 
 // the block sum of S (the tree of cta_sum2) and the closed-form Nose-Hoover
 // root (clmd_nh_root) on warp 0 alone, published by the second barrier:
-// the other warps skip the scalar Newton steps and their divisions
-template <int NT>
-__device__ __forceinline__ bool cta_nh_root(double S, double psi1, double nkt3, double dth,
-                                            double Q, double* sh, double& Stot, double& p) {
-  constexpr int W = NT / 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  S = wsum(S);
-  if (lane == 0) sh[w] = S;
-  __syncthreads();
-  if (w == 0) {
-    const double t = wsum(lane < W ? sh[lane] : 0.0);
-    double pr;
-    const bool ok = clmd_nh_root(t, psi1, nkt3, dth, Q, pr);
-    if (lane == 0) {
-      sh[32] = t;
-      sh[33] = pr;
-      sh[34] = ok ? 1.0 : 0.0;
-    }
-  }
-  __syncthreads();
-  Stot = sh[32];
-  p = sh[33];
-  return sh[34] != 0.0;
-}
-
-// cta_nh_root with the step's end folded in (one CTA per replica): lane 0
-// of warp 0 also records the replica's new PSI, sum v^2, ekin, step and pair
+// the other warps skip the scalar Newton steps and their divisions.  The
+// step's end is folded in (one CTA per replica): lane 0 of warp 0 also records the replica's new PSI, sum v^2, ekin, step and pair
 // terms (or the solve's failure) before the barrier that publishes the root,
 // so the step needs no barrier of its own to publish them
 template <int NT>
@@ -412,31 +387,26 @@ __device__ __forceinline__ int grp_or(int f, Cta& C) {
     return v[0] != 0.0;
   }
 }
-// the closed-form Nose-Hoover root of the group total of S (cta_nh_root for
-// one CTA; for a cluster the total first, then warp 0 of every CTA takes the
-// same root from the same total)
+// the closed-form Nose-Hoover root of a cluster's total of S: warp 0 of
+// every CTA takes the same root from the same total
 template <int NT, int CS>
-__device__ __forceinline__ bool grp_nh_root(double S, double psi1, double nkt3, double dth,
-                                            double Q, Cta& C, double& Stot, double& p) {
-  if constexpr (CS == 1) {
-    return cta_nh_root<NT>(S, psi1, nkt3, dth, Q, C.red, Stot, p);
-  } else {
-    double t = grp_sum<NT, CS>(S, C);
-    if (threadIdx.x < 32) {
-      double pr;
-      const bool ok = clmd_nh_root(t, psi1, nkt3, dth, Q, pr);
-      if (threadIdx.x == 0) {
-        C.red[33] = pr;
-        C.red[34] = ok ? 1.0 : 0.0;
-      }
+__device__ __forceinline__ bool cl_nh_root(double S, double psi1, double nkt3, double dth,
+                                           double Q, Cta& C, double& Stot, double& p) {
+  const double t = grp_sum<NT, CS>(S, C);
+  if (threadIdx.x < 32) {
+    double pr;
+    const bool ok = clmd_nh_root(t, psi1, nkt3, dth, Q, pr);
+    if (threadIdx.x == 0) {
+      C.red[33] = pr;
+      C.red[34] = ok ? 1.0 : 0.0;
     }
-    __syncthreads();
-    Stot = t;
-    p = C.red[33];
-    const bool ok = C.red[34] != 0.0;
-    __syncthreads();
-    return ok;
   }
+  __syncthreads();
+  Stot = t;
+  p = C.red[33];
+  const bool ok = C.red[34] != 0.0;
+  __syncthreads();
+  return ok;
 }
 
 template <bool SM>
@@ -851,8 +821,7 @@ __device__ int skin(Rep& R, const Args& A, double dmmr) {
 // (vo = v: vxn = v, s0 += v.v, dp += b vo dt/Q with b = -dth (a - psi1 vo))
 template <int NT, bool SM, bool MIXED, int CS, bool NHF = false>
 __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kick,
-                       bool energies, double psi1 = 0.0, double dtQ = 0.0, double* s0 = nullptr,
-                       double* dp = nullptr) {
+                       bool energies, double* s0 = nullptr) {
   const int N = R.natom, off = R.off, tid = threadIdx.x;
   const int gt = gtid<NT, CS>();
   constexpr int GT = NT * CS;
@@ -1006,7 +975,7 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
       ay = fy;
       az = fz;
     }
-    if (NHF && MIXED) {
+    if (NHF) {
       // closed-form solve (clmd_nh_root): W = V + dth a into vn, s0 += W.W
       const double dth = 0.5 * dt;
       const double wx = A.vx[off + i] + dth * ax;
@@ -1016,18 +985,6 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
       A.vyn[off + i] = wy;
       A.vzn[off + i] = wz;
       *s0 += wx * wx + wy * wy + wz * wz;
-    } else if (NHF) {
-      const double dth = 0.5 * dt;
-      const double V[3] = {A.vx[off + i], A.vy[off + i], A.vz[off + i]};
-      const double a3[3] = {ax, ay, az};
-      A.vxn[off + i] = V[0];
-      A.vyn[off + i] = V[1];
-      A.vzn[off + i] = V[2];
-#pragma unroll
-      for (int d = 0; d < 3; d++) {
-        *s0 += V[d] * V[d];
-        *dp += (-dth * (a3[d] - psi1 * V[d])) * V[d] * dtQ;
-      }
     }
     if (kick) {
       double vxi = A.vx[off + i] + 0.5 * ax * dt;
@@ -1052,7 +1009,7 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
   // one CTA, mixed Nose-Hoover: the closed-form root that follows opens with
   // barriers of its own (cta_nh_root_commit), which order this pass's
   // per-atom writes before anyone reads them
-  if constexpr (!(NHF && MIXED && CS == 1)) gsync<CS>();
+  if constexpr (!(NHF && CS == 1)) gsync<CS>();
 }
 
 template <bool MIXED>
@@ -1253,7 +1210,7 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
   const double dt = A.dt;
   Pos<SM> P{A, C, off};
   bool vin_n = false;  // uniform: the current velocities are in vxn, not vx
-  double vsc = 1.0;    // mixed: the velocities are vn * vsc (clmd_nh_root)
+  double vsc = 1.0;    // then the velocities are vn * vsc (clmd_nh_root)
   if (A.hx) host_io<NT, CS>(R, C, A, true);
   if (SM) {
     for (int i = gt; i < N; i += GT) {
@@ -1301,9 +1258,9 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
     if (A.ftcsi > 0 && R.step % A.ftcsi == 0 && R.cstep != R.step) {
       if (vin_n) {  // velocities back in vx for the analysis
         for (int i = gt; i < N; i += GT) {
-          A.vx[off + i] = MIXED ? A.vxn[off + i] * vsc : A.vxn[off + i];
-          A.vy[off + i] = MIXED ? A.vyn[off + i] * vsc : A.vyn[off + i];
-          A.vz[off + i] = MIXED ? A.vzn[off + i] * vsc : A.vzn[off + i];
+          A.vx[off + i] = A.vxn[off + i] * vsc;
+          A.vy[off + i] = A.vyn[off + i] * vsc;
+          A.vz[off + i] = A.vzn[off + i] * vsc;
         }
         vin_n = false;
         gsync<CS>();
@@ -1332,11 +1289,9 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
       vin_n = false;
       for (int i = gt; i < N; i += GT) {
         double vxi = svx[off + i], vyi = svy[off + i], vzi = svz[off + i];
-        if (MIXED) {
-          vxi = vxi * sc;
-          vyi = vyi * sc;
-          vzi = vzi * sc;
-        }
+        vxi = vxi * sc;
+        vyi = vyi * sc;
+        vzi = vzi * sc;
         double axi, ayi, azi;
         get_a<MIXED>(A, off + i, axi, ayi, azi);
         double dx, dy, dz;
@@ -1404,92 +1359,29 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
       if (!nh) {
         forces<NT, SM, MIXED, CS>(R, C, A, P, true, last);
       } else {
-        // int-verlet-nh-mav.f:91-180 with block reductions.  Each sweep is one
-        // pass: it updates vn from this sweep's delps and accumulates the
-        // next sweep's sums (sum vn^2, sum b vo dt/Q at pso + delps) in the
-        // same loop; the first pass rides on the force pass.
-        const double Q = R.Q, err = 1.0e-10, psi1 = R.psi, dtQ = dt / Q;
-        if (MIXED) {
-          double S = 0.0, unused = 0.0, p;
-          forces<NT, SM, MIXED, CS, true>(R, C, A, P, false, last, psi1, dtQ, &S, &unused);
-          if constexpr (CS == 1) {
-            if (!cta_nh_root_commit<NT>(S, psi1, R.nkt3_i, dth, Q, C.red, R, step, p)) goto out;
-            committed = true;
-          } else {
-            if (!grp_nh_root<NT, CS>(S, psi1, R.nkt3_i, dth, Q, C, S, p)) {
-              if (tid == 0 && R.status == 0) R.status = CLMD_ERR_NH_NOCONVERGE;
-              gsync<CS>();
-              goto out;
-            }
-            if (tid == 0) {
-              const double c = 1.0 / (1.0 + dth * p);
-              R.sumv2 = S * c * c;
-              R.psi = p;
-              R.ekin = 0.5 * R.sumv2;
-            }
-          }
-          vsc = 1.0 / (1.0 + dth * p);
-          vin_n = true;
+        // int-verlet-nh-mav.f:91-180: the implicit solve in closed form
+        // (clmd_nh_root); the force pass leaves W = V + dth a in vn
+        const double Q = R.Q, psi1 = R.psi;
+        double S = 0.0, p;
+        forces<NT, SM, MIXED, CS, true>(R, C, A, P, false, last, &S);
+        if constexpr (CS == 1) {
+          if (!cta_nh_root_commit<NT>(S, psi1, R.nkt3_i, dth, Q, C.red, R, step, p)) goto out;
+          committed = true;
         } else {
-          double sumv2n = 0.0, dpsum = 0.0;
-          forces<NT, SM, MIXED, CS, true>(R, C, A, P, false, last, psi1, dtQ, &sumv2n, &dpsum);
-          int nr0 = 0;
-          grp_sum2<NT, CS>(sumv2n, dpsum, nr0, C);
-          double psn = psi1;
-          int ready = 0;
-          for (int iter = 1; iter <= 1000; iter++) {
-            const double pso = psn;
-            const double di = -(pso * dth + 1);
-            double delps = dpsum - di * ((-sumv2n + R.nkt3_i) * dth / Q - (psi1 - pso));
-            delps = delps / (-dt2 * sumv2n / Q + di);
-            psn = pso + delps;
-            const double rdi = 1.0 / di;
-            double s2 = 0.0, dpn = 0.0;
-            int nr = 0;
-            for (int i = gt; i < N; i += GT) {
-              double ax, ay, az;
-              get_a<MIXED>(A, off + i, ax, ay, az);
-              const double V[3] = {A.vx[off + i], A.vy[off + i], A.vz[off + i]};
-              const double a3[3] = {ax, ay, az};
-              double* vn[3] = {A.vxn, A.vyn, A.vzn};
-              // the update rounded term by term: with fused multiply-adds the
-              // residual b never reaches exactly zero, the sweep keeps moving a
-              // near-zero component by ~1e-18 and the relative test then fails
-              // where the reference's sweep (int-verlet-nh-mav.f:117-147)
-              // settles on an exact fixed point
-  #pragma unroll
-              for (int d = 0; d < 3; d++) {
-                const double vo = vn[d][off + i];
-                const double b = __dsub_rn(__dmul_rn(-dth, __dsub_rn(a3[d], __dmul_rn(pso, vo))),
-                                           __dsub_rn(V[d], vo));
-                const double nx =
-                    __dadd_rn(vo, __dmul_rn(__dadd_rn(b, __dmul_rn(__dmul_rn(dth, vo), delps)), rdi));
-                if (fabs(__dsub_rn(nx, vo)) > err * fabs(nx)) nr = 1;
-                vn[d][off + i] = nx;
-                s2 += nx * nx;
-                dpn += (-dth * (a3[d] - psn * nx) - (V[d] - nx)) * nx * dtQ;
-              }
-            }
-            sumv2n = s2;
-            dpsum = dpn;
-            grp_sum2<NT, CS>(sumv2n, dpsum, nr, C);
-            if (!nr) {
-              ready = 1;
-              break;
-            }
-          }
-          if (!ready) {
+          if (!cl_nh_root<NT, CS>(S, psi1, R.nkt3_i, dth, Q, C, S, p)) {
             if (tid == 0 && R.status == 0) R.status = CLMD_ERR_NH_NOCONVERGE;
             gsync<CS>();
             goto out;
           }
-          vin_n = true;  // the step's velocities are in vxn until the next drift
           if (tid == 0) {
-            R.sumv2 = sumv2n;
-            R.psi = psn;
-            R.ekin = 0.5 * sumv2n;
+            const double c = 1.0 / (1.0 + dth * p);
+            R.sumv2 = S * c * c;
+            R.psi = p;
+            R.ekin = 0.5 * R.sumv2;
           }
         }
+        vsc = 1.0 / (1.0 + dth * p);
+        vin_n = true;
       }
       if (!committed) {
         if (tid == 0) {
@@ -1504,9 +1396,9 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
     if (R.step >= R.budget) {
       if (vin_n) {
         for (int i = gt; i < N; i += GT) {
-          A.vx[off + i] = MIXED ? A.vxn[off + i] * vsc : A.vxn[off + i];
-          A.vy[off + i] = MIXED ? A.vyn[off + i] * vsc : A.vyn[off + i];
-          A.vz[off + i] = MIXED ? A.vzn[off + i] * vsc : A.vzn[off + i];
+          A.vx[off + i] = A.vxn[off + i] * vsc;
+          A.vy[off + i] = A.vyn[off + i] * vsc;
+          A.vz[off + i] = A.vzn[off + i] * vsc;
         }
         vin_n = false;
         gsync<CS>();
@@ -1523,9 +1415,9 @@ out:
   gsync<CS>();
   if (vin_n) {
     for (int i = gt; i < N; i += GT) {
-      A.vx[off + i] = MIXED ? A.vxn[off + i] * vsc : A.vxn[off + i];
-      A.vy[off + i] = MIXED ? A.vyn[off + i] * vsc : A.vyn[off + i];
-      A.vz[off + i] = MIXED ? A.vzn[off + i] * vsc : A.vzn[off + i];
+      A.vx[off + i] = A.vxn[off + i] * vsc;
+      A.vy[off + i] = A.vyn[off + i] * vsc;
+      A.vz[off + i] = A.vzn[off + i] * vsc;
     }
   }
   if (SM) {

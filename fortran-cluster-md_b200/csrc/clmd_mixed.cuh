@@ -42,3 +42,35 @@ __device__ __forceinline__ bool clmd_nh_root(double S, double psi1, double nkt3,
   }
   return false;
 }
+
+// How many of the reference's sweeps (int-verlet-nh-mav.f:105-147) one atom
+// needs until the relative change of each of its velocity components stays
+// within 1e-10.  The sweeps' iterates are vn_k = al W + be V with factors
+// common to all atoms, so the scalars of every sweep follow from three sums
+// (sum W.W, W.V, V.V) without a pass over the atoms.
+__device__ __forceinline__ int clmd_nh_sweeps(const double* W, const double* V, double sww,
+                                              double swv, double svv, double psi1, double m,
+                                              double nkt3, double dt, double Q) {
+  const double dth = dt / 2, dt2 = dt * dt / 2;
+  double al = 0.0, be = 1.0, p = psi1;
+  int need = 1;
+  for (int k = 1; k <= 16; k++) {
+    const double sumv2 = al * al * sww + 2.0 * al * be * swv + be * be * svv;
+    const double up = 1.0 + dth * p;
+    const double draw = (up * sumv2 - (al * sww + be * swv)) * m * dt / Q;
+    double delps = draw + up * ((-m * sumv2 + nkt3) * dth / Q - (psi1 - p));
+    delps = delps / (-dt2 * m * sumv2 / Q - up);
+    const double a1 = (1.0 - dth * delps * al) / up, b1 = -dth * delps * be / up;
+    bool moved = false;
+    for (int d = 0; d < 3; d++) {
+      const double nx = a1 * W[d] + b1 * V[d], vo = al * W[d] + be * V[d];
+      moved |= fabs(nx - vo) > 1e-10 * fabs(nx);
+    }
+    if (moved) need = k + 1;
+    al = a1;
+    be = b1;
+    p += delps;
+    if (!moved && k > 1) break;
+  }
+  return need;
+}

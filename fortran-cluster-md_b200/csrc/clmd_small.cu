@@ -237,7 +237,7 @@ static __device__ bool s_rebuild(const Params& P, DevState* st, SmallShared& S, 
   return true;
 }
 
-enum { SS_MAX = 0, SS_SUMV2, SS_EPOT, SS_VIR, SS_EKIN, SS_DELPS, SS_NR };
+enum { SS_MAX = 0, SS_SUMV2, SS_EPOT, SS_VIR, SS_EKIN, SS_WV, SS_VV };
 
 template <bool NH, bool THERMO, bool MIXED>
 __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, CycleArgs A, int nsteps,
@@ -379,10 +379,10 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
       // forces, kick, next drift
       const double psi = B.q.psi, m = P.apmas[0], Q = P.Q;
       const bool fuse = !NH && !THERMO && !last;
-      double vox = 0.0, voy = 0.0, voz = 0.0;  // the Nose-Hoover iterate
+      double wx = 0.0, wy = 0.0, wz = 0.0;
       {
         const double bf1 = 2.0 + (double)(int)(B.q.atrskin / P.sig1), bf2 = bf1 + 0.5;
-        double fx, fy, fz, esum = 0.0, vir = 0.0, ek = 0.0, d2 = 0.0, sv = 0.0, dp = 0.0;
+        double fx, fy, fz, esum = 0.0, vir = 0.0, ek = 0.0, d2 = 0.0, sv = 0.0;
         bool bad = false;
         warp_forces<MIXED>(P, st, cur ? A.pos1 : A.pos0, A.list, a.start, a.len, a.lo, a.q, bf1,
                            bf2, fx, fy, fz, esum, vir, last, W, bad);
@@ -415,24 +415,12 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
               a.vz = a.vz + hz;
               d2 = dx * dx + dy * dy + dz * dz;
             }
-          } else if (MIXED) {
-            // closed-form solve (clmd_nh_root): W = V + dth a
-            vox = a.vx + dth * a.ax;
-            voy = a.vy + dth * a.ay;
-            voz = a.vz + dth * a.az;
-            sv = vox * vox + voy * voy + voz * voz;
           } else {
-            // int-verlet-nh-mav.f:94-120: vn = V, sumv2, first sweep's delps
-            vox = a.vx;
-            voy = a.vy;
-            voz = a.vz;
-            sv = vox * vox + voy * voy + voz * voz;
-            double b = -dth * (a.ax - psi * vox) - (vox - vox);
-            dp = dp + b * m * vox * dt / Q;
-            b = -dth * (a.ay - psi * voy) - (voy - voy);
-            dp = dp + b * m * voy * dt / Q;
-            b = -dth * (a.az - psi * voz) - (voz - voz);
-            dp = dp + b * m * voz * dt / Q;
+            // closed-form solve (clmd_nh_root): W = V + dth a
+            wx = a.vx + dth * a.ax;
+            wy = a.vy + dth * a.ay;
+            wz = a.vz + dth * a.az;
+            sv = wx * wx + wy * wy + wz * wz;
           }
         }
         if (last) {
@@ -443,7 +431,10 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
         if (fuse) G.put_max(SS_MAX, d2);
         if (NH) {
           G.put_sum(SS_SUMV2, sv);
-          if (!MIXED) G.put_sum(SS_DELPS, dp);
+          if (!MIXED && last) {  // for the count of the reference's sweeps
+            G.put_sum(SS_WV, wx * a.vx + wy * a.vy + wz * a.vz);
+            G.put_sum(SS_VV, a.vx * a.vx + a.vy * a.vy + a.vz * a.vz);
+          }
         }
         G.barrier();
         if (const int err = S.err[G.rb]) {
@@ -471,95 +462,39 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
         }
       }
       // Nose-Hoover implicit solve (int-verlet-nh-mav.f:105-180)
-      double sumv2 = G.get_sum(SS_SUMV2);
-      if (MIXED) {
-        G.rb ^= 1;
-        double pn;  // every thread takes the same root of the same sum
-        if (!clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn)) {
-          if (tid == 0 && B.q.status == 0) {
-            B.q.status = CLMD_ERR_NH_NOCONVERGE;
-            B.q.fail_step = step;
-          }
-          goto done;
-        }
-        const double c = 1.0 / (1.0 + dth * pn);
-        a.vx = vox * c;
-        a.vy = voy * c;
-        a.vz = voz * c;
-        __syncthreads();  // every thread has read this step's PSI
-        if (tid == 0) {
-          B.q.nh_iters = 1;
-          B.q.sumv2 = sumv2 * c * c;
-          B.q.psi = pn;
-          B.q.ekin = 0.5 * m * B.q.sumv2;
-        }
-        __syncthreads();
-        continue;
-      }
-      double draw = G.get_sum(SS_DELPS), psn = psi;
+      const double sumv2 = G.get_sum(SS_SUMV2);
+      const double swv = !MIXED && last ? G.get_sum(SS_WV) : 0.0;
+      const double svv = !MIXED && last ? G.get_sum(SS_VV) : 0.0;
       G.rb ^= 1;
-      int ready = 0, iter;
-      for (iter = 1; iter <= 1000; iter++) {
-        const double err = 1.0e-10, pso = psn, di = -(pso * dth + 1);
-        double delps = draw - di * ((-m * sumv2 + P.nkt3_i) * dth / Q - (psi - pso));
-        delps = delps / (-dt2 * m * sumv2 / Q + di);
-        const double pnext = pso + delps;
-        double s2 = 0.0, dp = 0.0;
-        bool more = false;
-        if (a.act) {
-          const double V[3] = {a.vx, a.vy, a.vz}, acc[3] = {a.ax, a.ay, a.az};
-          double vn[3] = {vox, voy, voz};
-#pragma unroll
-          for (int d = 0; d < 3; d++) {
-            const double vo = vn[d];
-            const double b = -dth * (acc[d] - pso * vo) - (V[d] - vo);
-            const double nx = vo + (b + dth * vo * delps) / di;
-            if (fabs((nx - vo) / nx) > err) more = true;
-            vn[d] = nx;
-          }
-#pragma unroll
-          for (int d = 0; d < 3; d++) s2 = s2 + vn[d] * vn[d];
-          // the next sweep's delps terms (:110-120 with vo = this vn)
-#pragma unroll
-          for (int d = 0; d < 3; d++) {
-            const double b = -dth * (acc[d] - pnext * vn[d]) - (V[d] - vn[d]);
-            dp = dp + b * m * vn[d] * dt / Q;
-          }
-          vox = vn[0];
-          voy = vn[1];
-          voz = vn[2];
-        }
-        G.put_sum(SS_SUMV2, s2);
-        G.put_sum(SS_DELPS, dp);
-        G.put(SS_NR, __any_sync(0xffffffffu, more) ? 1.0 : 0.0);
-        G.barrier();
-        sumv2 = G.get_sum(SS_SUMV2);
-        draw = G.get_sum(SS_DELPS);
-        const double nr = G.get_max(SS_NR);
-        G.rb ^= 1;
-        psn = pnext;
-        if (nr == 0.0) {
-          ready = 1;
-          break;
-        }
-      }
-      if (tid == 0) B.q.nh_iters = ready ? iter : 1000;
-      if (!ready) {
+      double pn;  // every thread takes the same root of the same sum
+      if (!clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn)) {
         if (tid == 0 && B.q.status == 0) {
           B.q.status = CLMD_ERR_NH_NOCONVERGE;
           B.q.fail_step = step;
         }
         goto done;
       }
-      // :171-180 (sumv2 of V = vn: same sum)
-      a.vx = vox;
-      a.vy = voy;
-      a.vz = voz;
+      int sweeps = 1;
+      if (!MIXED && last) {
+        if (a.act) {
+          const double W3[3] = {wx, wy, wz}, V3[3] = {a.vx, a.vy, a.vz};
+          sweeps = clmd_nh_sweeps(W3, V3, sumv2, swv, svv, psi, m, P.nkt3_i, dt, Q);
+        }
+        G.put_max(SS_MAX, (double)sweeps);
+        G.barrier();
+        sweeps = (int)G.get_max(SS_MAX);
+        G.rb ^= 1;
+      }
+      const double c = 1.0 / (1.0 + dth * pn);
+      a.vx = wx * c;
+      a.vy = wy * c;
+      a.vz = wz * c;
       __syncthreads();  // every thread has read this step's PSI
       if (tid == 0) {
-        B.q.sumv2 = sumv2;
-        B.q.psi = psn;
-        B.q.ekin = 0.5 * m * sumv2;
+        B.q.nh_iters = sweeps;
+        B.q.sumv2 = sumv2 * c * c;
+        B.q.psi = pn;
+        B.q.ekin = 0.5 * m * B.q.sumv2;
       }
       __syncthreads();
     }

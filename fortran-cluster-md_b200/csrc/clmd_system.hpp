@@ -29,7 +29,7 @@ struct clmd_system {
   int* perm_s = nullptr;
   float4* posf = nullptr;
   double *sx = nullptr, *sy = nullptr, *sz = nullptr;     // staging / scratch
-  double *vxn = nullptr, *vyn = nullptr, *vzn = nullptr;  // Nose-Hoover iterate
+  float *afx = nullptr, *afy = nullptr, *afz = nullptr;  // mixed Nose-Hoover: a step's accelerations
   // neighbour list
   int* list = nullptr;
   int *row_start = nullptr, *row_len = nullptr, *row_lo = nullptr;

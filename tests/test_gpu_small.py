@@ -40,7 +40,7 @@ def test_small_verlet_bit_exact(gpu, n):
     assert abs(sg.epot - so.epot) <= 1e-12 * max(abs(so.epot), 1.0)
 
 
-@pytest.mark.parametrize("n", [33, 129, 2049, 8192])
+@pytest.mark.parametrize("n", [33, 129, 2049, 8192, 8193])
 @pytest.mark.parametrize("ethst", ["N", "X"])
 def test_small_thermostats(gpu, n, ethst):
     cfg = clmd.lj_config(n, 0.04, 0.8, ethst=ethst,
