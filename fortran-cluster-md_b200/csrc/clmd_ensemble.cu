@@ -40,16 +40,12 @@ namespace clmd_ens {
 namespace cg = cooperative_groups;
 
 constexpr int kFptCap = 128;  // first-passage sizes tracked per replica
-#ifndef CLMD_SEARCH_PRUNE
-#define CLMD_SEARCH_PRUNE 0
-#endif
-#ifndef CLMD_SEARCH_CHUNK
-#define CLMD_SEARCH_CHUNK 2
-#endif
-// list search: candidate indices loaded ahead of their tests (2: measured
-// best of 1, 2, 4 and 8 on the batched workload, all bit-identical)
-constexpr int kSearchChunk = CLMD_SEARCH_CHUNK;
 constexpr int kNcMax = 28;    // cells per dimension at most (cells never narrower than the list radius)
+
+// 16-bit cell starts [ncell + 1] in whole 8-byte words
+__host__ __device__ constexpr size_t cells16_bytes(int ncell) {
+  return ((size_t)ncell + 2 + 3) / 4 * 8;
+}
 
 struct Rep {
   // parameters (reduced units: sigma = eps = m = 1)
@@ -76,6 +72,7 @@ struct Args {
   void* a;  // float[3][pool] (mixed) or double[3][pool] (FP64)
   long long pool;
   int *list, *rlen, *sorted, *cellid, *parent, *cs, *cl, *fpt;
+  uint2* cand;  // the search's candidates where shared memory does not hold them
   int* orig;  // per slot: the pool index (offset + atom number) of the atom it holds
   Rep* reps;
   const int* items;
@@ -84,6 +81,7 @@ struct Args {
   int* ctr;
   double rc, atskin, dt;
   int nbtim, ftcsi, lstride, integrator, nwin;
+  int smem;  // dynamic shared memory of this launch (bytes)
   int lg;  // mixed force pass: 1 << lg lanes per atom (0: one thread per atom)
   int reorder_every;  // the atoms' order renewed at every k-th rebuild
   int ncmax;  // cells per dimension this launch's shared memory holds
@@ -271,7 +269,12 @@ struct Cta {
   double* sx;  // positions in shared memory (nullptr: global)
   double* sy;
   double* sz;
-  int* cstart;  // [ncell + 1]: cell c holds sorted[cstart[c] .. cstart[c + 1])
+  // cell c holds the sorted slots cstart[c] .. cstart[c + 1]: 32-bit, or
+  // 16-bit (cs16) for a replica with its positions in shared memory
+  int* cstart;
+  unsigned short* cs16;
+  uint2* cand;        // the search's candidates in cell order (search_row)
+  unsigned ulo, uhi;  // its test: below ulo a neighbour, above uhi none
   double red[3 * 32 + 8];
   int ncx, ncell, nox, offx[3];
   double cf, rs2;
@@ -439,6 +442,13 @@ __device__ bool prologue(Rep& R, Cta& C, const Args& A, int step) {
     R.atrskin = fmin(R.box / 2.0, R.atrskin);
   }
   C.rs2 = R.atrskin * R.atrskin;
+  {
+    // coordinates in 2^-16 of the box, truncated: a difference is off by less
+    // than 1, its square sum by less than 2 (|dx| + |dy| + |dz|) + 3
+    const double r = R.atrskin * 65536.0 / R.box, band = 4.0 * r + 8.0;
+    C.ulo = (unsigned)fmax(r * r - band, 0.0);
+    C.uhi = (unsigned)(r * r + band);
+  }
   int n = (int)floor(R.box / (R.atrskin * (1.0 + 1e-9)));
   n = max(1, min(n, kNcMax));
   C.ncx = n;
@@ -564,6 +574,121 @@ __device__ void cta_scan(int* cnt, int n) {
   __syncthreads();
 }
 
+// cta_scan of 16-bit counts, two to a word
+template <int NT>
+__device__ void cta_scan16(unsigned* word, int nw) {
+  __shared__ int wsums[NT / 32 + 1];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int per = (nw + NT - 1) / NT, b0 = min(tid * per, nw), b1 = min(b0 + per, nw);
+  int s = 0;
+  for (int k = b0; k < b1; k++) s += (word[k] & 0xffffu) + (word[k] >> 16);
+  int incl = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) wsums[w] = incl;
+  __syncthreads();
+  unsigned ex = incl - s;
+  for (int k = 0; k < w; k++) ex += wsums[k];
+  for (int k = b0; k < b1; k++) {
+    const unsigned v = word[k];
+    word[k] = ex | (ex + (v & 0xffffu)) << 16;
+    ex += (v & 0xffffu) + (v >> 16);
+  }
+  __syncthreads();
+}
+
+// The list row of the atom in slot i, at place q0 of the cell order
+// (neighbour k at list[lbase + k N + i], at most the stride of them); returns
+// the neighbours found.
+// A candidate is 8 bytes in cell order: its coordinates in 2^-16 of the box
+// and its slot's low 16 bits.  The 16-bit differences wrap like the periodic
+// box, so the nearest image needs no test, and three integer products decide
+// all candidates but those within the truncation of the list radius (~0.3% of
+// r^2), which FP64 positions decide (mi_sel and r^2 rounded term by term; r^2
+// does not depend on the pair's orientation): the pair set is the FP64
+// test's.  That test alone, three FP64 positions a candidate gathered by
+// slot, ran a chain of ~150 cycles per candidate in every lane.  Two
+// candidates are loaded at a time, and the next cell row's range ahead of
+// this one's tests.
+template <bool SM>
+__device__ __forceinline__ int search_row(const Cta& C, const Args& A, const Pos<SM>& P, int q0,
+                                          int i, int N, double L, long long lbase) {
+  const int ncx = C.ncx, nox = C.nox;
+  const unsigned ulo = C.ulo, uhi = C.uhi;
+  const uint2* cand = C.cand;
+  const uint2 me = cand[q0];
+  int cx, cy, cz;
+  {
+    const double cf = C.cf;
+    cx = min((int)(P.x(i) * cf), ncx - 1);
+    cy = min((int)(P.y(i) * cf), ncx - 1);
+    cz = min((int)(P.z(i) * cf), ncx - 1);
+  }
+  // the cells of a row: [xa, xb), and the one the row wraps to (edge)
+  const int xa = nox < 3 ? 0 : max(cx - 1, 0), xb = nox < 3 ? ncx : min(cx + 2, ncx);
+  const bool edge = nox == 3 && (cx == 0 || cx == ncx - 1);
+  const int xw = cx == 0 ? ncx - 1 : 0;
+  int n = 0, ka = 0, kb = 0, a0, b0, a1 = 0, b1 = 0;
+  int* out = A.list + lbase + i;
+  auto start = [&](int c) { return SM ? (int)C.cs16[c] : C.cstart[c]; };
+  auto next = [&]() {
+    int zz = cz + ka - (nox == 3), yy = cy + kb - (nox == 3);
+    zz += zz < 0 ? ncx : (zz >= ncx ? -ncx : 0);
+    yy += yy < 0 ? ncx : (yy >= ncx ? -ncx : 0);
+    const int row = (zz * ncx + yy) * ncx;
+    a0 = start(row + xa);
+    b0 = start(row + xb);
+    if (edge) {
+      a1 = start(row + xw);
+      b1 = start(row + xw + 1);
+    }
+    if (++kb == nox) {
+      kb = 0;
+      ka++;
+    }
+  };
+  auto test = [&](uint2 c, int q) {
+    const int dx = (short)(me.x - c.x), dy = (short)((me.x >> 16) - (c.x >> 16)),
+              dz = (short)(me.y - c.y);
+    const unsigned u = (unsigned)(dx * dx) + (unsigned)(dy * dy) + (unsigned)(dz * dz);
+    if (u > uhi || q == q0) return;
+    const int j = SM ? (int)(c.y >> 16) : (C.ident ? q : A.sorted[P.off + q]);
+    if (u >= ulo) {
+      const double hL = 0.5 * L;
+      const double x = mi_sel(__dsub_rn(P.x(i), P.x(j)), L, hL),
+                   y = mi_sel(__dsub_rn(P.y(i), P.y(j)), L, hL),
+                   z = mi_sel(__dsub_rn(P.z(i), P.z(j)), L, hL);
+      const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+      if (!(r2 <= C.rs2)) return;
+    }
+    if (n < A.lstride) *out = j;
+    out += N;
+    n++;
+  };
+  next();
+  for (bool more = true; more;) {
+    int q = a0, e = b0;
+    const int q1 = a1, e1 = b1;
+    more = ka < nox;
+    if (more) next();
+    for (int part = 0;; part++) {
+#pragma unroll 1
+      for (; q < e; q += 2) {
+        const uint2 c0 = cand[q], c1 = cand[min(q + 1, e - 1)];
+        test(c0, q);
+        if (q + 1 < e) test(c1, q + 1);
+      }
+      if (part || !edge) break;
+      q = q1;
+      e = e1;
+    }
+  }
+  return n;
+}
+
 // cell list + rows (ELL, transposed per replica: entry k of atom i at
 // list[off*stride + k*N + i]); cells are index-sorted so row order is fixed
 template <int NT, bool SM, int CS>
@@ -572,48 +697,82 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
   const int gt = gtid<NT, CS>();
   constexpr int GT = NT * CS;
   const double L = R.box;
-  // one array does the counting sort: counts at cnt[c + 1], an in-place
-  // exclusive scan turns them into starts, and the scatter's atomics advance
-  // each to its cell's end = the next cell's start.  One CTA keeps it in
-  // shared memory; a cluster keeps it in global memory (its scratch) and
-  // then copies the result into every CTA's shared memory for the search.
-  int* cnt = C.cstart;
-  if constexpr (CS > 1) cnt = A.cscr + (long long)(blockIdx.x / CS) * A.cscr_stride;
-  for (int c = gt; c <= C.ncell; c += GT) cnt[c] = 0;
   if (tid == 0) C.ident = 0;  // until a reorder into cell order below
-  gsync<CS>();
-  for (int i = gt; i < N; i += GT) {
-    const double x = wrap_box(P.x(i), L), y = wrap_box(P.y(i), L), z = wrap_box(P.z(i), L);
-    P.set(i, x, y, z);
-    int cx = min((int)(x * C.cf), C.ncx - 1), cy = min((int)(y * C.cf), C.ncx - 1),
-        cz = min((int)(z * C.cf), C.ncx - 1);
-    int c = (cz * C.ncx + cy) * C.ncx + cx;
-    A.cellid[off + i] = c;
-    atomicAdd(&cnt[c + 1], 1);
-  }
-  gsync<CS>();
-  if (grank<CS>() == 0) cta_scan<NT>(cnt + 1, C.ncell);
-  gsync<CS>();
-  // scatter in arrival order (parent[] is free outside the analysis), then
-  // each atom takes the place of its rank by index inside its cell: the
-  // cell order is fixed whatever the order of the atomics
-  int* tmp = A.parent + off;
-  for (int i = gt; i < N; i += GT) {
-    int slot = atomicAdd(&cnt[A.cellid[off + i] + 1], 1);
-    tmp[slot] = i;
-  }
-  gsync<CS>();
-  if constexpr (CS > 1) {
-    for (int c = tid; c <= C.ncell; c += NT) C.cstart[c] = __ldcg(cnt + c);
+  if constexpr (SM) {
+    // 16-bit counts, two to a word: the count before an atom's own is its
+    // arrival number; both travel in cellid[] (cells < 2^15).  The slots go
+    // to their cells in arrival order, then each takes the place of its rank
+    // by index inside its cell: the cell order is fixed whatever the order
+    // of the atomics
+    unsigned* word = (unsigned*)C.cs16;
+    const int nw = (C.ncell + 2) / 2;
+    for (int k = tid; k < nw; k += NT) word[k] = 0u;
     __syncthreads();
+    for (int i = tid; i < N; i += NT) {
+      const double x = wrap_box(P.x(i), L), y = wrap_box(P.y(i), L), z = wrap_box(P.z(i), L);
+      P.set(i, x, y, z);
+      const int cx = min((int)(x * C.cf), C.ncx - 1), cy = min((int)(y * C.cf), C.ncx - 1),
+                cz = min((int)(z * C.cf), C.ncx - 1);
+      const int c = (cz * C.ncx + cy) * C.ncx + cx, sh = 16 * (c & 1);
+      const unsigned before = (atomicAdd(word + (c >> 1), 1u << sh) >> sh) & 0xffffu;
+      A.cellid[off + i] = (int)(before << 15) | c;
+    }
+    __syncthreads();
+    cta_scan16<NT>(word, nw);
+    int* tmp = A.parent + off;
+    for (int i = tid; i < N; i += NT) {
+      const int v = A.cellid[off + i], q = C.cs16[v & 0x7fff] + (v >> 15);
+      tmp[q] = i;
+    }
+    __syncthreads();
+    for (int i = tid; i < N; i += NT) {
+      const int c = A.cellid[off + i] & 0x7fff, c0 = C.cs16[c], c1 = C.cs16[c + 1];
+      int r = c0;
+      for (int q = c0; q < c1; q++) r += tmp[q] < i;
+      A.sorted[off + r] = i;
+    }
+    __syncthreads();
+  } else {
+    // one array does the counting sort: counts at cnt[c + 1], an in-place
+    // exclusive scan turns them into starts, and the scatter's atomics
+    // advance each to its cell's end = the next cell's start.  One CTA keeps
+    // it in shared memory; a cluster keeps it in global memory (its scratch)
+    // and then copies the result into every CTA's shared memory.
+    int* cnt = C.cstart;
+    if constexpr (CS > 1) cnt = A.cscr + (long long)(blockIdx.x / CS) * A.cscr_stride;
+    for (int c = gt; c <= C.ncell; c += GT) cnt[c] = 0;
+    gsync<CS>();
+    for (int i = gt; i < N; i += GT) {
+      const double x = wrap_box(P.x(i), L), y = wrap_box(P.y(i), L), z = wrap_box(P.z(i), L);
+      P.set(i, x, y, z);
+      int cx = min((int)(x * C.cf), C.ncx - 1), cy = min((int)(y * C.cf), C.ncx - 1),
+          cz = min((int)(z * C.cf), C.ncx - 1);
+      int c = (cz * C.ncx + cy) * C.ncx + cx;
+      A.cellid[off + i] = c;
+      atomicAdd(&cnt[c + 1], 1);
+    }
+    gsync<CS>();
+    if (grank<CS>() == 0) cta_scan<NT>(cnt + 1, C.ncell);
+    gsync<CS>();
+    // in arrival order (parent[] is free outside the analysis), then by rank
+    int* tmp = A.parent + off;
+    for (int i = gt; i < N; i += GT) {
+      int slot = atomicAdd(&cnt[A.cellid[off + i] + 1], 1);
+      tmp[slot] = i;
+    }
+    gsync<CS>();
+    if constexpr (CS > 1) {
+      for (int c = tid; c <= C.ncell; c += NT) C.cstart[c] = __ldcg(cnt + c);
+      __syncthreads();
+    }
+    for (int i = gt; i < N; i += GT) {
+      const int c = A.cellid[off + i], c0 = C.cstart[c], c1 = C.cstart[c + 1];
+      int r = 0;
+      for (int q = c0; q < c1; q++) r += tmp[q] < i;
+      A.sorted[off + c0 + r] = i;
+    }
+    gsync<CS>();
   }
-  for (int i = gt; i < N; i += GT) {
-    const int c = A.cellid[off + i], c0 = C.cstart[c], c1 = C.cstart[c + 1];
-    int r = 0;
-    for (int q = c0; q < c1; q++) r += tmp[q] < i;
-    A.sorted[off + c0 + r] = i;
-  }
-  gsync<CS>();
   // either order may be kept for a few rebuilds (atoms move little between
   // rebuilds: measured +1.8% for cell-ordered cluster replicas renewed every
   // third rebuild instead of every one); the search and the forces use
@@ -661,133 +820,34 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
       A.vx[off + p] = gx[p];
       A.vy[off + p] = gy[p];
       A.vz[off + p] = gz[p];
-      if (R.reorder == 2)
-        A.sorted[off + p] = A.cellid[off + A.sorted[off + p]];  // old index -> new slot
-      else
-        A.sorted[off + p] = p;  // the cells now hold consecutive slots
+      // reorder 2: old index -> new slot; reorder 1: the cells now hold
+      // consecutive slots
+      A.sorted[off + p] = R.reorder == 2 ? A.cellid[off + A.sorted[off + p]] : p;
     }
     if (tid == 0) C.ident = R.reorder == 1;
     gsync<CS>();
   }
-  const double hL = 0.5 * L, rs2 = C.rs2;
   const long long lbase = (long long)off * A.lstride;
   int over = 0, nsum = 0;
-  // the atoms in cell order (sorted[]), whatever order their slots have: the
-  // lanes of a warp then search overlapping stencils (similar candidate
-  // counts, the same candidates read by several lanes at once)
-  const bool ident = C.ident;
+  {
+    const double k = 65536.0 / L;
+    auto u16 = [&](double x) { return (unsigned)(int)(x * k) & 0xffffu; };
+    for (int q = gt; q < N; q += GT) {
+      const int i = C.ident ? q : A.sorted[off + q];
+      C.cand[q] = make_uint2(u16(P.x(i)) | u16(P.y(i)) << 16, u16(P.z(i)) | (unsigned)i << 16);
+    }
+    gsync<CS>();
+  }
+  // the atoms in cell order, whatever order their slots have: the lanes of a
+  // warp then search overlapping stencils (similar candidate counts, the same
+  // candidates read by several lanes at once)
   for (int q0 = gt; q0 < N; q0 += GT) {
-    const int i = ident ? q0 : A.sorted[off + q0];
-    const double xi = P.x(i), yi = P.y(i), zi = P.z(i);
-    int cx = min((int)(xi * C.cf), C.ncx - 1), cy = min((int)(yi * C.cf), C.ncx - 1),
-        cz = min((int)(zi * C.cf), C.ncx - 1);
-    int n = 0;
-    // with three or more cells per dimension the stencil's cells hold each
-    // neighbour once, at the periodic image nearest to atom i for every pair
-    // within the list radius (cells are at least that wide): the image
-    // shift is the cell range's, added to xi - xj with the same single
-    // rounding the minimum image (mi_sel) gives, so the pair set and r^2
-    // are those of mi_sel without its per-candidate tests; r^2 does not
-    // depend on the pair's orientation (IEEE subtraction is sign-symmetric)
-    const bool sel = C.nox < 3;
-#if CLMD_SEARCH_PRUNE
-    // the atom's distances to its cell's faces: a neighbour row (and an end
-    // cell of a row) whose nearest point is farther than the list radius
-    // holds no neighbour and is skipped (a margin of 1e-9 L covers the
-    // rounding of the cell assignment).  Off by default: bit-identical, but
-    // 3% slower on the batched workload (the per-row tests cost more than
-    // the ~20% of candidates they save)
-    const double cw = 1.0 / C.cf, mg = 1e-9 * L;
-    const double fxl = fmax(xi - cx * cw - mg, 0.0), fxr = fmax((cx + 1) * cw - xi - mg, 0.0);
-    const double fyl = fmax(yi - cy * cw - mg, 0.0), fyr = fmax((cy + 1) * cw - yi - mg, 0.0);
-    const double fzl = fmax(zi - cz * cw - mg, 0.0), fzr = fmax((cz + 1) * cw - zi - mg, 0.0);
-#endif
-    for (int a = 0; a < C.nox; a++) {
-      int zz = cz + C.offx[a];
-      const double szL = sel ? 0.0 : (zz < 0 ? L : (zz >= C.ncx ? -L : 0.0));
-      zz += zz < 0 ? C.ncx : 0;
-      zz -= zz >= C.ncx ? C.ncx : 0;
-      for (int b = 0; b < C.nox; b++) {
-        int yy = cy + C.offx[b];
-        const double syL = sel ? 0.0 : (yy < 0 ? L : (yy >= C.ncx ? -L : 0.0));
-        yy += yy < 0 ? C.ncx : 0;
-        yy -= yy >= C.ncx ? C.ncx : 0;
-        const int rowc = (zz * C.ncx + yy) * C.ncx;
-#if CLMD_SEARCH_PRUNE
-        bool lft = true, rgt = true;
-        if (!sel) {
-          const int oz = C.offx[a], oy = C.offx[b];
-          const double dz = oz < 0 ? fzl : (oz > 0 ? fzr : 0.0);
-          const double dy = oy < 0 ? fyl : (oy > 0 ? fyr : 0.0);
-          const double bx = rs2 - (dy * dy + dz * dz);
-          if (bx < 0.0) continue;
-          lft = fxl * fxl <= bx;
-          rgt = fxr * fxr <= bx;
-        }
-#else
-        const bool lft = true, rgt = true;
-#endif
-        // the x-neighbours of a cell row are contiguous in cell order: one
-        // candidate range [ca0, cb0), a second [ca1, cb1) with image shift
-        // sx1 where the row wraps (all of the row when ncx <= 2).  Scalars
-        // picked per range, not arrays indexed by it: those would live in
-        // local memory.
-        int ca0, cb0, ca1 = 0, cb1 = 0, nr = 1;
-        double sx1 = 0.0;
-        if (sel) {
-          ca0 = rowc; cb0 = rowc + C.ncx;
-        } else if (cx == 0) {
-          ca0 = rowc; cb0 = rowc + (rgt ? 2 : 1);
-          ca1 = rowc + C.ncx - 1; cb1 = rowc + C.ncx; nr = lft ? 2 : 1;
-          sx1 = L;
-        } else if (cx == C.ncx - 1) {
-          ca0 = rowc + cx - (lft ? 1 : 0); cb0 = rowc + C.ncx;
-          ca1 = rowc; cb1 = rowc + 1; nr = rgt ? 2 : 1;
-          sx1 = -L;
-        } else {
-          ca0 = rowc + cx - (lft ? 1 : 0); cb0 = rowc + cx + (rgt ? 2 : 1);
-        }
-        for (int d = 0; d < nr; d++) {
-          const int q1 = C.cstart[d ? cb1 : cb0];
-          const double sxL = d ? sx1 : 0.0;
-          // kSearchChunk candidates' indices loaded ahead of their tests
-          for (int q = C.cstart[d ? ca1 : ca0]; q < q1; q += kSearchChunk) {
-            int js[kSearchChunk];
-#pragma unroll
-            for (int u = 0; u < kSearchChunk; u++)
-              js[u] = q + u < q1 ? (ident ? q + u : A.sorted[off + q + u]) : i;
-#pragma unroll
-            for (int u = 0; u < kSearchChunk; u++) {
-              const int j = js[u];
-              if (j == i) continue;
-              double dx = __dsub_rn(xi, P.x(j)), dy = __dsub_rn(yi, P.y(j)),
-                     dz = __dsub_rn(zi, P.z(j));
-              if (sel) {
-                dx = mi_sel(dx, L, hL);
-                dy = mi_sel(dy, L, hL);
-                dz = mi_sel(dz, L, hL);
-              } else {
-                dx = __dadd_rn(dx, sxL);
-                dy = __dadd_rn(dy, syL);
-                dz = __dadd_rn(dz, szL);
-              }
-              double r2 =
-                  __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-              if (r2 <= rs2) {
-                if (n < A.lstride) A.list[lbase + (long long)n * N + i] = j;
-                n++;
-              }
-            }
-          }
-        }
-      }
-    }
-    if (n > A.lstride) {
-      over = 1;
-      n = A.lstride;
-    }
-    A.rlen[off + i] = n;
-    nsum += n;
+    const int i = C.ident ? q0 : A.sorted[off + q0];
+    const double fin = P.x(i) + P.y(i) + P.z(i);  // (an atom at a NaN has no neighbours)
+    const int n = fin == fin ? search_row<SM>(C, A, P, q0, i, N, L, lbase) : 0;
+    if (n > A.lstride) over = 1;
+    A.rlen[off + i] = min(n, A.lstride);
+    nsum += min(n, A.lstride);
   }
   {
     // the rows' total (pair terms of each force pass until the next
@@ -1457,10 +1517,16 @@ __global__ void __launch_bounds__(NT, MINB) k_ens(Args A) {
       const int ncell = R.ncmax * R.ncmax * R.ncmax;
       C.rep = r;
       C.cstart = (int*)dsm;
-      double* p = (double*)(C.cstart + ((ncell + 2) & ~1));
-      C.sx = SM ? p : nullptr;
-      C.sy = SM ? p + nmax : nullptr;
-      C.sz = SM ? p + 2 * nmax : nullptr;
+      C.cs16 = (unsigned short*)dsm;
+      C.cand = A.cand + R.off;
+      C.sx = C.sy = C.sz = nullptr;
+      if (SM) {
+        C.sx = dsm + cells16_bytes(ncell) / 8;
+        C.sy = C.sx + nmax;
+        C.sz = C.sy + nmax;
+        if (cells16_bytes(ncell) + 32 * (size_t)nmax <= (size_t)A.smem)
+          C.cand = (uint2*)(C.sz + nmax);
+      }
     }
     __syncthreads();
     unsigned long long t0 = 0;
@@ -1517,6 +1583,7 @@ __global__ void __launch_bounds__(NT, 1) k_ens_cl(Args A) {
     if (threadIdx.x == 0) {
       C.rep = r;
       C.cstart = (int*)dsm;
+      C.cand = A.cand + R.off;
       C.sx = C.sy = C.sz = nullptr;
     }
     unsigned long long t0 = 0;
@@ -1771,6 +1838,7 @@ extern "C" int clmd_ens_create(const clmd_ens_config* cfg, clmd_ensemble** out) 
   ECK(cudaMalloc(&A.cellid, 4 * P)); ECK(cudaMalloc(&A.parent, 4 * P));
   ECK(cudaMalloc(&A.cs, 4 * P)); ECK(cudaMalloc(&A.cl, 4 * P));
   ECK(cudaMalloc(&A.orig, 4 * P));
+  ECK(cudaMalloc(&A.cand, 8 * P));
   ECK(cudaMemset(A.a, 0, 3 * 8 * P));
   ECK(cudaMemset(A.rlen, 0, 4 * P));
   ECK(cudaMemset(A.cl, 0, 4 * P));
@@ -1827,7 +1895,7 @@ extern "C" int clmd_ens_destroy(clmd_ensemble* E) {
   cudaStreamSynchronize(E->stream);
   Args& A = E->A;
   void* ps[] = {A.x, A.y, A.z, A.vx, A.vy, A.vz, A.vxn, A.vyn, A.vzn, A.a, A.list, A.rlen,
-                A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.reps, A.fpt, A.summary,
+                A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.cand, A.reps, A.fpt, A.summary,
                 E->d_items, E->d_ctr, E->d_iwin, A.wtime, E->d_stage, A.cscr,
                 E->d_hoff};
   for (void* p : ps)
@@ -2058,9 +2126,16 @@ static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const i
   }
   for (int k = 0; k < nitems; k++) {
     const Rep& R = E->h_reps[slots[k]];
-    L.smem = std::max(L.smem, smem_bytes(R.natom, R.ncmax, sm));
+    size_t need = smem_bytes(R.natom, R.ncmax, sm);
+    if (sm) {  // 16-bit cells; the search's candidates too where they fit
+      const size_t base = cells16_bytes(R.ncmax * R.ncmax * R.ncmax) + 24 * (size_t)R.natom;
+      const size_t with = base + 8 * (size_t)R.natom;
+      need = with + 8192 <= E->smem_cap ? with : base;
+    }
+    L.smem = std::max(L.smem, need);
     L.ncmax = std::max(L.ncmax, R.ncmax);
   }
+  L.smem = (L.smem + 7) & ~(size_t)7;
   L.k = kernel_for(shape, sm, mixed);
   // the attribute only grows: classes that share a kernel may launch it
   // with different amounts in one sequence (occupancy follows each launch)
@@ -2090,6 +2165,7 @@ static int enqueue_class(clmd_ensemble* E, int c, const ClassLaunch& L, int nwin
   A.nwin = nwin;
   A.ncmax = L.ncmax;
   A.lg = L.lg;
+  A.smem = (int)L.smem;
   const unsigned fl = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
   ECK(cudaEventRecordWithFlags(E->ev0[c], st, fl));
   if (L.cs > 1) {

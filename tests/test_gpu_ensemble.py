@@ -651,3 +651,37 @@ def test_step_io_matches_upload_step_download(gpu):
         e2.step_io(1, [a.ctypes.data_as(C.POINTER(C.c_double)) for a in plain])
     e1.close()
     e2.close()
+
+
+@pytest.mark.parametrize("n,box,rskin", [
+    (2, 5.1, 2.55), (60, 5.4, 2.7), (150, 8.2, 2.8),  # one, two cells per dimension
+    (300, 8.5, 2.8), (1000, 40.0, 2.8),               # three and more
+    (5000, 60.0, 3.4), (8200, 55.0, 2.8),             # candidates in shared memory, outside it
+    (9300, 90.0, 2.8), (12000, 70.0, 3.1), (70000, 130.0, 2.8)])  # clusters, 16-bit slots exceeded
+def test_list_entries_match_fp64(gpu, n, box, rskin):
+    """The search's integer test with its FP64 decision near the list radius:
+    the number of list entries is that of the FP64 minimum image and square
+    sum, evaluated here term by term, with a third of the atoms placed at the
+    list radius (1 +- 1e-16 .. 1e-4) from another."""
+    from scipy.spatial import cKDTree
+
+    rng = np.random.default_rng(n)
+    a = rng.uniform(0, box, (n, 3))
+    k = n // 3
+    d = rng.normal(size=(k, 3))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    r = rskin * (1 + rng.choice([1, -1], k) * 10.0 ** rng.uniform(-16, -4, k))
+    a[n - k:] = (a[:k] + d * r[:, None]) % box
+    x = [np.ascontiguousarray(a[:, c]) for c in range(3)]
+    # (a time step in which even overlapping atoms stay where they are)
+    v = [np.full(n, 1e-9) * rng.normal(size=n) for _ in range(3)]
+    e = clmd.Ensemble(clmd.ens_config(n, 1, ftcsi=1, rskin=rskin, integrator=clmd.INT_VERLET,
+                                      precision=clmd.PREC_FP64, dt=1e-30, list_stride=512))
+    assert e.add(n, box, 0.7, *x, *v, ethst="-") is not None
+    e.step(1)
+    pairs = cKDTree(a, boxsize=box).query_pairs(rskin + 1e-3, output_type="ndarray")
+    d = a[pairs[:, 0]] - a[pairs[:, 1]]
+    d = np.where(np.abs(d) > 0.5 * box, d - np.copysign(box, d), d)
+    half = int((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1] + d[:, 2] * d[:, 2] <= rskin * rskin).sum())
+    assert e.results()[0].nrebuild == 1
+    assert e.pair_terms() == 2 * half
