@@ -72,6 +72,9 @@ struct Args {
   void* a;  // float[3][pool] (mixed) or double[3][pool] (FP64)
   long long pool;
   int *list, *rlen, *sorted, *cellid, *parent, *cs, *cl, *fpt;
+  // a window's positions of replicas that do not keep them in shared memory:
+  // a neighbour's is one 32-byte sector
+  double4* p4;
   uint2* cand;  // the search's candidates where shared memory does not hold them
   int* orig;  // per slot: the pool index (offset + atom number) of the atom it holds
   Rep* reps;
@@ -417,14 +420,22 @@ struct Pos {
   const Args& A;
   const Cta& C;
   int off;
-  __device__ __forceinline__ double x(int i) const { return SM ? C.sx[i] : A.x[off + i]; }
-  __device__ __forceinline__ double y(int i) const { return SM ? C.sy[i] : A.y[off + i]; }
-  __device__ __forceinline__ double z(int i) const { return SM ? C.sz[i] : A.z[off + i]; }
+  __device__ __forceinline__ double x(int i) const { return SM ? C.sx[i] : A.p4[off + i].x; }
+  __device__ __forceinline__ double y(int i) const { return SM ? C.sy[i] : A.p4[off + i].y; }
+  __device__ __forceinline__ double z(int i) const { return SM ? C.sz[i] : A.p4[off + i].z; }
+  __device__ __forceinline__ void get(int i, double& a, double& b, double& c) const {
+    if (SM) {
+      a = C.sx[i]; b = C.sy[i]; c = C.sz[i];
+    } else {
+      const double4 q = A.p4[off + i];
+      a = q.x; b = q.y; c = q.z;
+    }
+  }
   __device__ __forceinline__ void set(int i, double a, double b, double c) const {
     if (SM) {
       C.sx[i] = a; C.sy[i] = b; C.sz[i] = c;
     } else {
-      A.x[off + i] = a; A.y[off + i] = b; A.z[off + i] = c;
+      A.p4[off + i] = make_double4(a, b, c, 0.0);
     }
   }
 };
@@ -709,7 +720,11 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
     for (int k = tid; k < nw; k += NT) word[k] = 0u;
     __syncthreads();
     for (int i = tid; i < N; i += NT) {
-      const double x = wrap_box(P.x(i), L), y = wrap_box(P.y(i), L), z = wrap_box(P.z(i), L);
+      double x, y, z;
+      P.get(i, x, y, z);
+      x = wrap_box(x, L);
+      y = wrap_box(y, L);
+      z = wrap_box(z, L);
       P.set(i, x, y, z);
       const int cx = min((int)(x * C.cf), C.ncx - 1), cy = min((int)(y * C.cf), C.ncx - 1),
                 cz = min((int)(z * C.cf), C.ncx - 1);
@@ -743,7 +758,11 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
     for (int c = gt; c <= C.ncell; c += GT) cnt[c] = 0;
     gsync<CS>();
     for (int i = gt; i < N; i += GT) {
-      const double x = wrap_box(P.x(i), L), y = wrap_box(P.y(i), L), z = wrap_box(P.z(i), L);
+      double x, y, z;
+      P.get(i, x, y, z);
+      x = wrap_box(x, L);
+      y = wrap_box(y, L);
+      z = wrap_box(z, L);
       P.set(i, x, y, z);
       int cx = min((int)(x * C.cf), C.ncx - 1), cy = min((int)(y * C.cf), C.ncx - 1),
           cz = min((int)(z * C.cf), C.ncx - 1);
@@ -798,9 +817,7 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
     int* go = A.parent + off;
     for (int p = gt; p < N; p += GT) {
       const int q = srt[p];
-      gx[p] = P.x(q);
-      gy[p] = P.y(q);
-      gz[p] = P.z(q);
+      P.get(q, gx[p], gy[p], gz[p]);
       go[p] = A.orig[off + q];
     }
     gsync<CS>();
@@ -875,6 +892,54 @@ __device__ int skin(Rep& R, const Args& A, double dmmr) {
   return R.dmms > (R.atrskin - A.rc - 2.0 * R.dmms / (double)(float)R.dmmst);
 }
 
+// A list row walked entry by entry (stride N), with loads ahead of the pair
+// being evaluated: the next entry where positions are in shared memory; the
+// next entry's position and the entry after it where they are in global
+// memory, whose latency, entry then position, set the force pass's time.
+template <bool SM>
+struct RowWalk {
+  const int* p;
+  int len, N, j, jn;
+  double x, y, z;
+  __device__ __forceinline__ RowWalk(const Pos<SM>& P, const int* row, int len_, int N_)
+      : p(row), len(len_), N(N_), jn(0) {
+    if (SM) {
+      j = 0;
+      jn = len > 0 ? *p : 0;
+      step();
+    } else {
+      j = len > 0 ? *p : 0;
+      p += N;
+      jn = len > 1 ? *p : 0;
+      P.get(j, x, y, z);
+    }
+  }
+  __device__ __forceinline__ void step() {
+    j = jn;
+    p += N;
+  }
+  __device__ __forceinline__ void get(const Pos<SM>& P, double& a, double& b, double& c) const {
+    if (SM) {
+      P.get(j, a, b, c);
+    } else {
+      a = x;
+      b = y;
+      c = z;
+    }
+  }
+  // past entry k
+  __device__ __forceinline__ void next(const Pos<SM>& P, int k) {
+    if (SM) {
+      if (k + 1 < len) jn = *p;
+      step();
+    } else {
+      step();
+      if (k + 2 < len) jn = *p;
+      if (k + 1 < len) P.get(j, x, y, z);
+    }
+  }
+};
+
 // pair forces (for-a-lj-n-pbc-m.f, sigma = eps = m = 1) -> a; optional
 // velocity-Verlet second half kick; FP64 energy/virial sums when asked
 // NHF: also the Nose-Hoover solve's first pass on the fresh accelerations
@@ -900,16 +965,19 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
       const int i = w0 + (lane >> lg);
       const bool own = i < N;
       const int ii = own ? i : w0;
-      const double xi = P.x(ii), yi = P.y(ii), zi = P.z(ii);
+      double xi, yi, zi;
+    P.get(ii, xi, yi, zi);
       const int len = own ? A.rlen[off + i] : 0;
       float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
       const int* lp = A.list + lbase + (long long)sub * N + ii;
       const long long step = (long long)G * N;
       for (int k = sub; k < len; k += G, lp += step) {
         const int j = *lp;
-        double dx = mi_sel(xi - P.x(j), L, hL);
-        double dy = mi_sel(yi - P.y(j), L, hL);
-        double dz = mi_sel(zi - P.z(j), L, hL);
+        double dx, dy, dz;
+        P.get(j, dx, dy, dz);
+        dx = mi_sel(xi - dx, L, hL);
+        dy = mi_sel(yi - dy, L, hL);
+        dz = mi_sel(zi - dz, L, hL);
         double r2d = dx * dx + dy * dy + dz * dz;
         if (r2d <= rc2) {
           float r2 = (float)r2d;
@@ -963,22 +1031,22 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
   for (int i0 = 0; i0 < N; i0 += GT) {
     const int i = i0 + gt;
     if (i >= N) continue;
-    const double xi = P.x(i), yi = P.y(i), zi = P.z(i);
+    double xi, yi, zi;
+    P.get(i, xi, yi, zi);
     const int len = A.rlen[off + i];
     double ax, ay, az;
     if (MIXED) {
       float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-      // the next row entry is loaded while this pair is evaluated
-      const int* lp = A.list + lbase + i;
-      int jn = len > 0 ? lp[0] : 0;
+      RowWalk<SM> w(P, A.list + lbase + i, len, N);
 #pragma unroll 2
       for (int k = 0; k < len; k++) {
-        const int j = jn;
-        lp += N;
-        if (k + 1 < len) jn = *lp;
-        double dx = mi_sel(xi - P.x(j), L, hL);
-        double dy = mi_sel(yi - P.y(j), L, hL);
-        double dz = mi_sel(zi - P.z(j), L, hL);
+        const int j = w.j;
+        double dx, dy, dz;
+        w.get(P, dx, dy, dz);
+        w.next(P, k);
+        dx = mi_sel(xi - dx, L, hL);
+        dy = mi_sel(yi - dy, L, hL);
+        dz = mi_sel(zi - dz, L, hL);
         double r2d = dx * dx + dy * dy + dz * dz;
         if (r2d <= rc2) {
           float r2 = (float)r2d;
@@ -1003,16 +1071,15 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
       az = (double)fz;
     } else {
       double fx = 0.0, fy = 0.0, fz = 0.0;
-      // the next row entry is loaded while this pair is evaluated
-      const int* lp = A.list + lbase + i;
-      int jn = len > 0 ? lp[0] : 0;
+      RowWalk<SM> w(P, A.list + lbase + i, len, N);
       for (int k = 0; k < len; k++) {
-        const int j = jn;
-        lp += N;
-        if (k + 1 < len) jn = *lp;
-        double dx = mi_sel(xi - P.x(j), L, hL);
-        double dy = mi_sel(yi - P.y(j), L, hL);
-        double dz = mi_sel(zi - P.z(j), L, hL);
+        const int j = w.j;
+        double dx, dy, dz;
+        w.get(P, dx, dy, dz);
+        w.next(P, k);
+        dx = mi_sel(xi - dx, L, hL);
+        dy = mi_sel(yi - dy, L, hL);
+        dz = mi_sel(zi - dz, L, hL);
         double r2d = dx * dx + dy * dy + dz * dz;
         if (r2d <= rc2) {
           double ri2 = 1.0 / r2d;
@@ -1163,14 +1230,17 @@ __device__ void analysis(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, int st
   const double bf1 = (double)(int)(R.atrskin) + 2.0, bf2 = bf1 + 0.5;
   const long long lbase = (long long)off * A.lstride;
   for (int i = gt; i < N - 1; i += GT) {
-    const double xi = P.x(i), yi = P.y(i), zi = P.z(i);
+    double xi, yi, zi;
+    P.get(i, xi, yi, zi);
     const int len = A.rlen[off + i];
     for (int k = 0; k < len; k++) {
       int j = A.list[lbase + (long long)k * N + i];
       if (j <= i) continue;
-      double dx = mi_bf(__dsub_rn(xi, P.x(j)), L, iL, bf1, bf2);
-      double dy = mi_bf(__dsub_rn(yi, P.y(j)), L, iL, bf1, bf2);
-      double dz = mi_bf(__dsub_rn(zi, P.z(j)), L, iL, bf1, bf2);
+      double dx, dy, dz;
+      P.get(j, dx, dy, dz);
+      dx = mi_bf(__dsub_rn(xi, dx), L, iL, bf1, bf2);
+      dy = mi_bf(__dsub_rn(yi, dy), L, iL, bf1, bf2);
+      dz = mi_bf(__dsub_rn(zi, dz), L, iL, bf1, bf2);
       double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
       if (r2 <= rc2) uunion(par, i, j);
     }
@@ -1272,14 +1342,8 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
   bool vin_n = false;  // uniform: the current velocities are in vxn, not vx
   double vsc = 1.0;    // then the velocities are vn * vsc (clmd_nh_root)
   if (A.hx) host_io<NT, CS>(R, C, A, true);
-  if (SM) {
-    for (int i = gt; i < N; i += GT) {
-      C.sx[i] = A.x[off + i];
-      C.sy[i] = A.y[off + i];
-      C.sz[i] = A.z[off + i];
-    }
-    gsync<CS>();
-  }
+  for (int i = gt; i < N; i += GT) P.set(i, A.x[off + i], A.y[off + i], A.z[off + i]);
+  gsync<CS>();
   // the grid of the current list
   if (tid == 0) {
     int n = (int)floor(R.box / (R.atrskin * (1.0 + 1e-9)));
@@ -1372,7 +1436,9 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
           vyi = vyi + dth * (ayi - psi * vyi);
           vzi = vzi + dth * (azi - psi * vzi);
         }
-        P.set(i, P.x(i) + dx, P.y(i) + dy, P.z(i) + dz);
+        double px, py, pz;
+        P.get(i, px, py, pz);
+        P.set(i, px + dx, py + dy, pz + dz);
         A.vx[off + i] = vxi;
         A.vy[off + i] = vyi;
         A.vz[off + i] = vzi;
@@ -1480,13 +1546,7 @@ out:
       A.vz[off + i] = A.vzn[off + i] * vsc;
     }
   }
-  if (SM) {
-    for (int i = gt; i < N; i += GT) {
-      A.x[off + i] = C.sx[i];
-      A.y[off + i] = C.sy[i];
-      A.z[off + i] = C.sz[i];
-    }
-  }
+  for (int i = gt; i < N; i += GT) P.get(i, A.x[off + i], A.y[off + i], A.z[off + i]);
   gsync<CS>();
   if (A.hx) host_io<NT, CS>(R, C, A, false);
 }
@@ -1838,7 +1898,7 @@ extern "C" int clmd_ens_create(const clmd_ens_config* cfg, clmd_ensemble** out) 
   ECK(cudaMalloc(&A.cellid, 4 * P)); ECK(cudaMalloc(&A.parent, 4 * P));
   ECK(cudaMalloc(&A.cs, 4 * P)); ECK(cudaMalloc(&A.cl, 4 * P));
   ECK(cudaMalloc(&A.orig, 4 * P));
-  ECK(cudaMalloc(&A.cand, 8 * P));
+  ECK(cudaMalloc(&A.cand, 8 * P)); ECK(cudaMalloc(&A.p4, 32 * P));
   ECK(cudaMemset(A.a, 0, 3 * 8 * P));
   ECK(cudaMemset(A.rlen, 0, 4 * P));
   ECK(cudaMemset(A.cl, 0, 4 * P));
@@ -1895,7 +1955,7 @@ extern "C" int clmd_ens_destroy(clmd_ensemble* E) {
   cudaStreamSynchronize(E->stream);
   Args& A = E->A;
   void* ps[] = {A.x, A.y, A.z, A.vx, A.vy, A.vz, A.vxn, A.vyn, A.vzn, A.a, A.list, A.rlen,
-                A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.cand, A.reps, A.fpt, A.summary,
+                A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.cand, A.p4, A.reps, A.fpt, A.summary,
                 E->d_items, E->d_ctr, E->d_iwin, A.wtime, E->d_stage, A.cscr,
                 E->d_hoff};
   for (void* p : ps)
