@@ -2260,15 +2260,20 @@ static int enqueue_class(clmd_ensemble* E, int c, const ClassLaunch& L, int nwin
 // replica not yet timed runs a few steps)
 // only >= 0: that size class alone (the autotuner's trials)
 // the cluster class of a replica whose positions do not fit in shared
-// memory: about kClusterAtoms atoms or more per CTA, the cluster size a power
-// of two in [2, 16], the largest usable one not above it (-1: none usable).
-// 6144 rather than 3072: on 300 replicas of 9,000-50,000 atoms 6.92e9 vs
-// 6.66e9 atom-steps/s, served 9.49e9 vs 8.69e9 (1536: 5.50e9); the largest
-// served size (50,000) gets 16 CTAs either way
-constexpr int kClusterAtoms = 6144;
+// memory: about `per` atoms or more per CTA, the cluster size a power of two
+// in [2, 16], the largest usable one not above it (-1: none usable).  Large
+// pools: 6144 (300 replicas of 9,000-50,000 atoms 6.92e9 atom-steps/s, 6.66e9
+// with 3072, 5.50e9 with 1536).  A pool of at most 2304 atoms per SM cannot
+// fill the GPU at that: 3072 (9 such replicas 7.55 -> 4.74 ms per 100 steps,
+// 12: 6.82 -> 4.82, 14: 7.70 -> 7.04; beyond, 16: 8.36 -> 8.12, but 19:
+// 7.82 -> 8.75).  The pool's size, not its present load, decides: a replica's
+// sums keep their shape whatever shares the launch
+constexpr int kClusterAtoms = 6144, kClusterAtomsSmallPool = 3072, kSmallPoolPerSm = 2304;
 static int cluster_class(const clmd_ensemble* E, int n) {
+  const int per = E->A.pool <= (long long)kSmallPoolPerSm * E->nsm ? kClusterAtomsSmallPool
+                                                                     : kClusterAtoms;
   int want = 2;
-  while (want < 16 && want * kClusterAtoms < n) want *= 2;
+  while (want < 16 && want * per < n) want *= 2;
   for (int c = clmd_ensemble::kClasses - 1; c >= clmd_ensemble::kCtaClasses; c--)
     if (E->cls_cs[c] <= want && E->cl_max_clusters[c] > 0) return c;
   return -1;
