@@ -1695,6 +1695,10 @@ struct clmd_ensemble {
   int* d_iwin = nullptr;   // windows per item (balanced launches)
   int* h_iwin = nullptr;   // pinned
   float* h_wtime = nullptr;  // pinned copy of A.wtime
+  // one replica's arrays on their way in or out (9 n doubles of the largest so
+  // far): contiguous, in atom order
+  double *d_xfer = nullptr, *h_xfer = nullptr;
+  size_t xfer_cap = 0;
   double* d_stage = nullptr;  // bulk copies in atom order (pool doubles, on first use)
   long long* d_hoff = nullptr;  // clmd_ens_step_io: each slot's offset in the host arrays
   int4* h_summary = nullptr;  // pinned copy of A.summary
@@ -1957,7 +1961,7 @@ extern "C" int clmd_ens_destroy(clmd_ensemble* E) {
   void* ps[] = {A.x, A.y, A.z, A.vx, A.vy, A.vz, A.vxn, A.vyn, A.vzn, A.a, A.list, A.rlen,
                 A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.cand, A.p4, A.reps, A.fpt, A.summary,
                 E->d_items, E->d_ctr, E->d_iwin, A.wtime, E->d_stage, A.cscr,
-                E->d_hoff};
+                E->d_hoff, E->d_xfer};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (E->h_reps) cudaFreeHost(E->h_reps);
@@ -1965,6 +1969,7 @@ extern "C" int clmd_ens_destroy(clmd_ensemble* E) {
   if (E->h_iwin) cudaFreeHost(E->h_iwin);
   if (E->h_wtime) cudaFreeHost(E->h_wtime);
   if (E->h_summary) cudaFreeHost(E->h_summary);
+  if (E->h_xfer) cudaFreeHost(E->h_xfer);
   if (E->stream) cudaStreamDestroy(E->stream);
   for (int c = 0; c < clmd_ensemble::kClasses; c++) {
     if (E->cstream[c]) cudaStreamDestroy(E->cstream[c]);
@@ -2036,6 +2041,61 @@ extern "C" int clmd_ens_pair_terms(clmd_ensemble* E, int64_t* total) {
   return CLMD_OK;
 }
 
+static int ensure_xfer(clmd_ensemble* E, int n) {
+  size_t need = 9 * (size_t)n;
+  if (need <= E->xfer_cap) return CLMD_OK;
+  // (doubled: admissions in ascending sizes would allocate each time)
+  need = std::max(need, std::min(std::max(2 * E->xfer_cap, (size_t)9 * 4096),
+                                 9 * (size_t)E->A.pool));
+  ECK(cudaStreamSynchronize(E->stream));
+  cudaFree(E->d_xfer);
+  cudaFreeHost(E->h_xfer);
+  E->d_xfer = E->h_xfer = nullptr;
+  E->xfer_cap = 0;
+  ECK(cudaMalloc(&E->d_xfer, 8 * need));
+  ECK(cudaMallocHost(&E->h_xfer, 8 * need));
+  E->xfer_cap = need;
+  return CLMD_OK;
+}
+
+// an admitted replica's atoms into its pool range: x..vz, each slot holding
+// its own atom, no list rows yet (the first order does not depend on the
+// pool's history), no first passages
+__global__ void k_admit(Args A, const double* in, int n, int off, int slot) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < kFptCap) A.fpt[(size_t)slot * kFptCap + i] = -1;
+  if (i == 0) A.summary[slot] = make_int4(0, 0, 0, 0);
+  if (i >= n) return;
+  A.x[off + i] = in[i];
+  A.y[off + i] = in[n + i];
+  A.z[off + i] = in[2 * (size_t)n + i];
+  A.vx[off + i] = in[3 * (size_t)n + i];
+  A.vy[off + i] = in[4 * (size_t)n + i];
+  A.vz[off + i] = in[5 * (size_t)n + i];
+  A.orig[off + i] = off + i;
+  A.rlen[off + i] = 0;
+}
+
+// a replica's x..vz, ax..az in atom order (orig[]), nine arrays of n
+template <bool MIXED>
+__global__ void k_export(Args A, double* out, int n, int off) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const size_t s = (size_t)off + i;
+  double* o = out + (A.orig[s] - off);
+  o[0] = A.x[s];
+  o[n] = A.y[s];
+  o[2 * (size_t)n] = A.z[s];
+  o[3 * (size_t)n] = A.vx[s];
+  o[4 * (size_t)n] = A.vy[s];
+  o[5 * (size_t)n] = A.vz[s];
+  double ax, ay, az;
+  get_a<MIXED>(A, (int)s, ax, ay, az);
+  o[6 * (size_t)n] = ax;
+  o[7 * (size_t)n] = ay;
+  o[8 * (size_t)n] = az;
+}
+
 extern "C" int clmd_ens_add(clmd_ensemble* E, const clmd_replica_spec* sp, const double* x,
                             const double* y, const double* z, const double* vx,
                             const double* vy, const double* vz, int32_t* slot) {
@@ -2054,12 +2114,16 @@ extern "C" int clmd_ens_add(clmd_ensemble* E, const clmd_replica_spec* sp, const
   if (off < 0) return CLMD_ERR_NOMEM;
   Args& A = E->A;
   cudaStream_t st = E->stream;
-  ECK(cudaMemcpyAsync(A.x + off, x, 8 * N, cudaMemcpyHostToDevice, st));
-  ECK(cudaMemcpyAsync(A.y + off, y, 8 * N, cudaMemcpyHostToDevice, st));
-  ECK(cudaMemcpyAsync(A.z + off, z, 8 * N, cudaMemcpyHostToDevice, st));
-  ECK(cudaMemcpyAsync(A.vx + off, vx, 8 * N, cudaMemcpyHostToDevice, st));
-  ECK(cudaMemcpyAsync(A.vy + off, vy, 8 * N, cudaMemcpyHostToDevice, st));
-  ECK(cudaMemcpyAsync(A.vz + off, vz, 8 * N, cudaMemcpyHostToDevice, st));
+  {
+    const int rc = ensure_xfer(E, N);
+    if (rc) {
+      pool_free(E, off, N);
+      return rc;
+    }
+  }
+  const double* src[6] = {x, y, z, vx, vy, vz};
+  for (int k = 0; k < 6; k++) memcpy(E->h_xfer + (size_t)k * N, src[k], 8 * (size_t)N);
+  ECK(cudaMemcpyAsync(E->d_xfer, E->h_xfer, 48 * (size_t)N, cudaMemcpyHostToDevice, st));
   Rep& R = E->h_reps[s];
   memset(&R, 0, sizeof(Rep));
   R.box = sp->box;
@@ -2088,17 +2152,11 @@ extern "C" int clmd_ens_add(clmd_ensemble* E, const clmd_replica_spec* sp, const
   // (rows of similar length per warp; large: gathers near).
   // CLMD_ENS_ORDER=cell: cell order for every replica
   R.reorder = (fits && !E->cell_order) ? 2 : 1;
-  std::vector<int> iota(N);
-  for (int i = 0; i < N; i++) iota[i] = (int)off + i;
-  ECK(cudaMemcpyAsync(A.orig + off, iota.data(), 4 * (size_t)N, cudaMemcpyHostToDevice, st));
-  ECK(cudaMemsetAsync(A.rlen + off, 0, 4 * (size_t)N, st));  // the first order: pool history-free
-  ECK(cudaMemcpyAsync(A.reps + s, &R, sizeof(Rep), cudaMemcpyHostToDevice, st));
   E->h_summary[s] = make_int4(0, 0, 0, 0);
-  ECK(cudaMemcpyAsync(A.summary + s, &E->h_summary[s], sizeof(int4), cudaMemcpyHostToDevice,
-                      st));
-  std::vector<int> neg(kFptCap, -1);
-  ECK(cudaMemcpyAsync(A.fpt + (size_t)s * kFptCap, neg.data(), sizeof(int) * kFptCap,
-                      cudaMemcpyHostToDevice, st));
+  k_admit<<<(std::max(N, kFptCap) + 255) / 256, 256, 0, st>>>(A, E->d_xfer, N, (int)off, s);
+  ECK(cudaGetLastError());
+  E->launches++;
+  ECK(cudaMemcpyAsync(A.reps + s, &R, sizeof(Rep), cudaMemcpyHostToDevice, st));
   ECK(cudaStreamSynchronize(st));
   E->used[s] = 1;
   E->slot_off[s] = off;
@@ -2565,24 +2623,6 @@ extern "C" int clmd_ens_poll(clmd_ensemble* E, clmd_replica_result* out, int32_t
   return CLMD_OK;
 }
 
-// the atom number each slot of a reordered replica holds (orig[])
-static int slot_orig(clmd_ensemble* E, int slot, std::vector<int>& o) {
-  const int N = E->h_reps[slot].natom;
-  o.resize(N);
-  ECK(cudaMemcpyAsync(o.data(), E->A.orig + E->slot_off[slot], 4 * (size_t)N,
-                      cudaMemcpyDeviceToHost, E->stream));
-  ECK(cudaStreamSynchronize(E->stream));
-  for (int& v : o) v -= (int)E->slot_off[slot];  // pool index -> atom number
-  return CLMD_OK;
-}
-
-// a[p] (slot order) -> a[o[p]] (atom order)
-template <typename T>
-static void unpermute(T* a, const std::vector<int>& o) {
-  std::vector<T> t(a, a + o.size());
-  for (size_t p = 0; p < o.size(); p++) a[o[p]] = t[p];
-}
-
 extern "C" int clmd_ens_get_state(clmd_ensemble* E, int32_t slot, double* x, double* y,
                                   double* z, double* vx, double* vy, double* vz, double* ax,
                                   double* ay, double* az, int32_t* cl) {
@@ -2592,36 +2632,23 @@ extern "C" int clmd_ens_get_state(clmd_ensemble* E, int32_t slot, double* x, dou
   const long long off = E->slot_off[slot];
   const int N = E->h_reps[slot].natom;
   cudaStream_t st = E->stream;
-  double* dst[6] = {x, y, z, vx, vy, vz};
-  double* src[6] = {A.x, A.y, A.z, A.vx, A.vy, A.vz};
-  for (int k = 0; k < 6; k++)
-    if (dst[k]) ECK(cudaMemcpyAsync(dst[k], src[k] + off, 8 * N, cudaMemcpyDeviceToHost, st));
-  double* ad[3] = {ax, ay, az};
-  if (E->cfg.precision == CLMD_PREC_MIXED) {
-    std::vector<float> tmp(N);
-    for (int k = 0; k < 3; k++)
-      if (ad[k]) {
-        ECK(cudaMemcpyAsync(tmp.data(), (float*)A.a + k * A.pool + off, 4 * N,
-                            cudaMemcpyDeviceToHost, st));
-        ECK(cudaStreamSynchronize(st));
-        for (int i = 0; i < N; i++) ad[k][i] = tmp[i];
-      }
-  } else {
-    for (int k = 0; k < 3; k++)
-      if (ad[k])
-        ECK(cudaMemcpyAsync(ad[k], (double*)A.a + k * A.pool + off, 8 * N,
-                            cudaMemcpyDeviceToHost, st));
-  }
-  if (cl) ECK(cudaMemcpyAsync(cl, A.cl + off, 4 * N, cudaMemcpyDeviceToHost, st));
-  ECK(cudaStreamSynchronize(st));
-  if (E->h_reps[slot].reorder) {  // slots in cell order: back to atom order
-    std::vector<int> o;
-    int rc = slot_orig(E, slot, o);
+  double* dst[9] = {x, y, z, vx, vy, vz, ax, ay, az};
+  bool any = false;
+  for (double* d : dst) any = any || d;
+  if (any) {
+    const int rc = ensure_xfer(E, N);
     if (rc) return rc;
-    double* arr[9] = {x, y, z, vx, vy, vz, ax, ay, az};
-    for (double* a : arr)
-      if (a) unpermute(a, o);  // (labels are stored by atom number already)
+    auto k = E->cfg.precision == CLMD_PREC_MIXED ? k_export<true> : k_export<false>;
+    k<<<(N + 255) / 256, 256, 0, st>>>(A, E->d_xfer, N, (int)off);
+    ECK(cudaGetLastError());
+    E->launches++;
+    for (int q = 0; q < 9; q++)
+      if (dst[q])
+        ECK(cudaMemcpyAsync(dst[q], E->d_xfer + (size_t)q * N, 8 * (size_t)N,
+                            cudaMemcpyDeviceToHost, st));
   }
+  if (cl) ECK(cudaMemcpyAsync(cl, A.cl + off, 4 * (size_t)N, cudaMemcpyDeviceToHost, st));
+  ECK(cudaStreamSynchronize(st));
   return CLMD_OK;
 }
 
