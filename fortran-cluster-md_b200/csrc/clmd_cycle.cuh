@@ -122,18 +122,52 @@ __device__ __forceinline__ bool nbt(const Params& P, double rs2, const double4& 
   return r2 <= rs2;
 }
 
-// Rows longer than the search's buffer, one after the other by the whole
-// warp: lanes with n > 0 name a row of n entries (slots, in any order) that
-// starts at list[start]; each is put in ascending reference order, *lo gets
-// the number of entries below the owner's reference index.  Up to 256
-// entries sit in registers, 8 per lane, and every entry's place is the count
-// of smaller keys (distinct, so the places are a permutation); a longer row
-// is left to its lane's insertion sort.  A liquid droplet's rows run to ~130
-// entries, where one lane's insertion sort in memory took ~130 us.
-static __device__ __noinline__ void sort_long_rows(int* list, const int* perm, unsigned long long start, int n,
-                                      int refi, int& lo) {
+// One row of m <= 32 T entries (slots, in any order), by the whole warp: T
+// entries per lane in registers, and every entry's place is the count of
+// smaller reference indices (distinct, so the places are a permutation).
+// Returns the number of entries below `ref`.
+template <int T>
+__device__ __forceinline__ int sort_row(int* row, const int* perm, int m, int ref) {
   constexpr unsigned FULL = 0xffffffffu;
-  constexpr int kT = 8;
+  const int lane = threadIdx.x & 31;
+  int q[T], key[T], rank[T], below = 0;
+#pragma unroll
+  for (int t = 0; t < T; t++) {
+    const int k = lane + 32 * t;
+    q[t] = k < m ? row[k] : 0;
+    key[t] = k < m ? perm[q[t]] : 0x7fffffff;
+    rank[t] = 0;
+  }
+#pragma unroll
+  for (int t = 0; t < T; t++)
+    below += __popc(__ballot_sync(FULL, lane + 32 * t < m && key[t] < ref));
+#pragma unroll
+  for (int u = 0; u < T; u++) {
+    if (32 * u >= m) break;
+#pragma unroll 8
+    for (int l = 0; l < 32; l++) {
+      const int other = __shfl_sync(FULL, key[u], l);
+#pragma unroll
+      for (int t = 0; t < T; t++) rank[t] += other < key[t];
+    }
+  }
+  __syncwarp();  // every lane has read the row
+#pragma unroll
+  for (int t = 0; t < T; t++)
+    if (lane + 32 * t < m) row[rank[t]] = q[t];
+  __syncwarp();
+  return below;
+}
+
+// Rows longer than the search's buffer, one after the other by the whole
+// warp: lanes with n > 0 name a row of n entries that starts at list[start];
+// each is put in ascending reference order, *lo gets the number of entries
+// below the owner's reference index.  A row of more than 256 entries is left
+// to its lane's insertion sort (in memory: ~130 us for a droplet's row of 130).
+static __device__ __noinline__ void sort_long_rows(int* list, const int* perm,
+                                                   unsigned long long start, int n, int refi,
+                                                   int& lo) {
+  constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   unsigned todo = __ballot_sync(FULL, n > 0);
   __syncwarp();  // the owners' entries are visible to every lane
@@ -142,7 +176,14 @@ static __device__ __noinline__ void sort_long_rows(int* list, const int* perm, u
     todo &= todo - 1;
     const int m = __shfl_sync(FULL, n, ow), ref = __shfl_sync(FULL, refi, ow);
     int* row = list + __shfl_sync(FULL, start, ow);
-    if (m > 32 * kT) {
+    int below = 0;
+    if (m <= 64) {
+      below = sort_row<2>(row, perm, m, ref);
+    } else if (m <= 128) {
+      below = sort_row<4>(row, perm, m, ref);
+    } else if (m <= 256) {
+      below = sort_row<8>(row, perm, m, ref);
+    } else {
       if (lane == ow) {
         for (int a = 1; a < m; a++) {
           int kq = row[a], kr = perm[kq];
@@ -153,36 +194,11 @@ static __device__ __noinline__ void sort_long_rows(int* list, const int* perm, u
           }
           row[b + 1] = kq;
         }
-        lo = 0;
-        for (int a = 0; a < m; a++) lo += perm[row[a]] < refi;
+        for (int a = 0; a < m; a++) below += perm[row[a]] < refi;
       }
       __syncwarp();
-      continue;
     }
-    int q[kT], key[kT], rank[kT], below = 0;
-#pragma unroll
-    for (int t = 0; t < kT; t++) {
-      const int k = lane + 32 * t;
-      q[t] = k < m ? row[k] : 0;
-      key[t] = k < m ? perm[q[t]] : 0x7fffffff;
-      rank[t] = 0;
-      below += __popc(__ballot_sync(FULL, k < m && key[t] < ref));
-    }
-#pragma unroll
-    for (int u = 0; u < kT; u++) {
-      if (32 * u >= m) break;
-      for (int l = 0; l < 32; l++) {
-        const int other = __shfl_sync(FULL, key[u], l);
-#pragma unroll
-        for (int t = 0; t < kT; t++) rank[t] += other < key[t];
-      }
-    }
-    __syncwarp();  // every lane has read the row
-#pragma unroll
-    for (int t = 0; t < kT; t++)
-      if (lane + 32 * t < m) row[rank[t]] = q[t];
     if (lane == ow) lo = below;
-    __syncwarp();
   }
 }
 
