@@ -46,9 +46,9 @@ __device__ __forceinline__ void uf_union(int* par, const int* key, int a, int b)
 }
 
 // the main loop analyses a step once (wrt-csi.f:27 "if(cstep.ne.step)");
-// a direct stoddard() call always recomputes (clu_force)
-__device__ __forceinline__ bool clu_gate(const DevState* st) {
-  return gated(st) || (!st->clu_force && st->s.cstep == st->cur_step);
+// a direct stoddard() call always recomputes (force)
+__device__ __forceinline__ bool clu_gate(const DevState* st, int force) {
+  return gated(st) || (!force && st->s.cstep == st->cur_step);
 }
 
 __device__ __forceinline__ double kin_energy(const Params& P, int sp, double vx, double vy,
@@ -57,11 +57,11 @@ __device__ __forceinline__ double kin_energy(const Params& P, int sp, double vx,
 }
 
 // stoddard-pbc-n-m.f:60-68 / -fre.f:60-82 resets (csi(0), ceks(0) persist)
-__global__ void k_clu_init(Params P, DevState* st, int* parent, int* cs, double* cek,
+__global__ void k_clu_init(Params P, DevState* st, int force, int* parent, int* cs, double* cek,
                            int* csi, double* ceks, int* deg, int* deg1, int* cgs, int* clf,
                            int* csf, int* csif, double* cekf, double* ceksf, int* cgsf,
                            int* cgsa, int* cgsfa, unsigned long long* nbonds) {
-  if (clu_gate(st)) return;
+  if (clu_gate(st, force)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool fre = P.clustering == CLMD_CLU_FRENKEL;
   if (i < P.N) {
@@ -87,6 +87,7 @@ __global__ void k_clu_init(Params P, DevState* st, int* parent, int* cs, double*
   if (i == 0) {
     *nbonds = 0ull;
     st->nroots = 0;
+    st->s.maxcs = 0;
     if (fre) {
       csif[0] = 0;
       cgsf[0] = 0;
@@ -102,11 +103,11 @@ __global__ void k_clu_init(Params P, DevState* st, int* parent, int* cs, double*
 // ascending).  Stillinger: species-1 atoms only, and a species-2 neighbour
 // ends the row (:85).  tWF: every pair, with degree counts for the liquid
 // test and the bond kept for the second (liquid-only) union-find.
-__global__ void k_clu_bonds(Params P, DevState* st, const double4* pos, const int* perm,
+__global__ void k_clu_bonds(Params P, DevState* st, int force, const double4* pos, const int* perm,
                             const int* list, const int* row_start, const int* row_len,
                             const int* row_lo, int* parent, int* deg, int* deg1, int2* bonds,
                             unsigned long long* nbonds, int bond_cap) {
-  if (clu_gate(st)) return;
+  if (clu_gate(st, force)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.N) return;
   if (perm[i] == P.N - 1) return;  // the last atom has no row (:74)
@@ -117,6 +118,7 @@ __global__ void k_clu_bonds(Params P, DevState* st, const double4* pos, const in
   const double bf1 = (double)(int)(st->s.atrskin / P.sig1) + 2.0;
   const double bf2 = bf1 + 0.5;
   int k0 = row_start[i] + row_lo[i], k1 = row_start[i] + row_len[i];
+  int mine = 0, mine1 = 0;  // own bonds, own bonds to species 1
   for (int k = k0; k < k1; k++) {
     int j = list[k];
     double4 pj = pos[j];
@@ -128,24 +130,31 @@ __global__ void k_clu_bonds(Params P, DevState* st, const double4* pos, const in
     if (rij2 <= P.atskin2) {
       uf_union(parent, perm, i, j);
       if (fre) {
-        atomicAdd(deg + i, 1);
+        mine++;
+        mine1 += sj == 1;
         atomicAdd(deg + j, 1);
-        if (sj == 1) atomicAdd(deg1 + i, 1);
         if (si == 1) atomicAdd(deg1 + j, 1);
-        unsigned long long b = atomicAdd(nbonds, 1ull);
+        // one cursor step for the lanes that append here together
+        const unsigned m = __activemask();
+        const int lane = threadIdx.x & 31, first = __ffs(m) - 1;
+        unsigned long long b = 0;
+        if (lane == first) b = atomicAdd(nbonds, (unsigned long long)__popc(m));
+        b = __shfl_sync(m, b, first) + __popc(m & ((1u << lane) - 1u));
         if (b < (unsigned long long)bond_cap) bonds[b] = make_int2(i, j);
         else raise_err(st, CLMD_ERR_LIST_OVERFLOW);
       }
     }
   }
+  if (mine) atomicAdd(deg + i, mine);
+  if (mine1) atomicAdd(deg1 + i, mine1);
 }
 
 // labels (1-based, = smallest atom index of the component), sizes and
 // kinetic energy per label
-__global__ void k_clu_label(Params P, DevState* st, const double4* pos, const int* perm,
+__global__ void k_clu_label(Params P, DevState* st, int force, const double4* pos, const int* perm,
                             const double* vx, const double* vy, const double* vz, int* parent,
                             int* cl, int* cs, double* cek, int* cgs) {
-  if (clu_gate(st)) return;
+  if (clu_gate(st, force)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.N) return;
   int r = perm[uf_find(parent, i)];
@@ -160,14 +169,39 @@ __global__ void k_clu_label(Params P, DevState* st, const double4* pos, const in
   }
 }
 
+// first-passage cursor (stoddard-pbc-n-m-fre.f:229-241) and bookkeeping
+__device__ void clu_finish(const Params& P, DevState* st, int* cfpt) {
+  clmd_scalars& q = st->s;
+  int step = st->cur_step;
+  q.cnum = P.N;
+  if (P.clustering == CLMD_CLU_FRENKEL) {
+    const int maxcs = __ldcg(&q.maxcs);  // other blocks' maximum
+    if (maxcs > q.cbiggest) q.cbiggest = maxcs;
+    if (q.cbiggest >= q.clookfor) {
+      for (int i = q.clookfor; i <= q.cbiggest; i++) cfpt[i - 1] = step;
+      q.clookfor = q.clookfor + 1;
+    }
+  }
+}
+
+// cstep = step marks the analysis done for this step (wrt-csi.f:27)
+__device__ void clu_done(DevState* st) {
+  st->s.cstep = st->cur_step;
+  int err = atomicExch(&st->err_new, 0);
+  if (err && st->s.status == 0) {
+    st->s.status = err;
+    st->s.fail_step = st->cur_step;
+  }
+}
+
 // stoddard-pbc-n-m.f:152-155 / -fre.f:229-234: one histogram entry per label
 // value 1..natom (labels that are not a root have cs = 0 and land in csi(0),
 // which the reference never resets)
 constexpr int kSmallBins = 64;
 
-__global__ void k_clu_hist(Params P, DevState* st, const int* cs, const double* cek, int* csi,
-                           double* ceks) {
-  if (clu_gate(st)) return;
+__global__ void k_clu_hist(Params P, DevState* st, int force, const int* cs, const double* cek, int* csi,
+                           double* ceks, int* cfpt) {
+  if (clu_gate(st, force)) return;
   __shared__ int hc[kSmallBins];
   __shared__ double he[kSmallBins];
   __shared__ int bmax;
@@ -196,25 +230,10 @@ __global__ void k_clu_hist(Params P, DevState* st, const int* cs, const double* 
     if (he[b] != 0.0) atomicAdd(ceks + b, he[b]);
   }
   if (threadIdx.x == 0 && bmax > 0) atomicMax(&st->s.maxcs, bmax);
-}
-
-__global__ void k_clu_prep(DevState* st) {
-  if (clu_gate(st)) return;
-  st->s.maxcs = 0;
-}
-
-// first-passage cursor (stoddard-pbc-n-m-fre.f:229-241) and bookkeeping
-__global__ void k_clu_finish(Params P, DevState* st, int* cfpt) {
-  if (clu_gate(st)) return;
-  clmd_scalars& q = st->s;
-  int step = st->cur_step;
-  q.cnum = P.N;
-  if (P.clustering == CLMD_CLU_FRENKEL) {
-    if (q.maxcs > q.cbiggest) q.cbiggest = q.maxcs;
-    if (q.cbiggest >= q.clookfor) {
-      for (int i = q.clookfor; i <= q.cbiggest; i++) cfpt[i - 1] = step;
-      q.clookfor = q.clookfor + 1;
-    }
+  // the last block closes the analysis (Stillinger) or its first part
+  if (last_block(&st->ctr[CTR_CLU]) && threadIdx.x == 0) {
+    clu_finish(P, st, cfpt);
+    if (P.clustering != CLMD_CLU_FRENKEL) clu_done(st);
   }
 }
 
@@ -222,11 +241,11 @@ __global__ void k_clu_finish(Params P, DevState* st, int* cfpt) {
 
 // liquid atoms and cekf(0) (species-1 atoms with >= atnenum bonds of which
 // fewer than atnenum go to species 1)
-__global__ void k_liq_flag(Params P, DevState* st, const double4* pos, const int* perm,
+__global__ void k_liq_flag(Params P, DevState* st, int force, const double4* pos, const int* perm,
                            const double* vx, const double* vy, const double* vz,
                            const int* deg, const int* deg1, int* liq, int* liqref,
                            int* parent2, double* cekf) {
-  if (clu_gate(st)) return;
+  if (clu_gate(st, force)) return;
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= P.N) return;
   int sp = (int)pos[k].w;
@@ -270,34 +289,39 @@ __device__ __forceinline__ int bscan_excl(int v, int* sh, int* total) {
   return sh[w] + incl - v;
 }
 
-__global__ void k_liq_tiles(Params P, DevState* st, const int* liq, int* aux) {
-  if (clu_gate(st)) return;
+__global__ void k_liq_tiles(Params P, DevState* st, int force, const int* liq, int* aux) {
+  if (clu_gate(st, force)) return;
   __shared__ int sh[33];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int v = i < P.N ? liq[i] : 0;
   int tot;
   bscan_excl(v, sh, &tot);
   if (threadIdx.x == 0) aux[blockIdx.x] = tot;
-}
-
-__global__ void k_liq_top(DevState* st, int* aux, int ntiles) {
-  if (clu_gate(st)) return;
-  __shared__ int sh[33];
+  if (!last_block(&st->ctr[CTR_SCAN])) return;
+  // the last block scans the tiles, eight per thread and round
   int carry = 0;
-  for (int b0 = 0; b0 < ntiles; b0 += blockDim.x) {
-    int b = b0 + threadIdx.x;
-    int v = b < ntiles ? aux[b] : 0;
-    int tot;
-    int ex = bscan_excl(v, sh, &tot);
-    if (b < ntiles) aux[b] = carry + ex;
+  for (int b0 = 0; b0 < (int)gridDim.x; b0 += 8 * kBlock) {
+    int n[8], s = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int b = b0 + 8 * (int)threadIdx.x + k;
+      n[k] = b < (int)gridDim.x ? __ldcg(aux + b) : 0;
+      s += n[k];
+    }
+    int ex = carry + bscan_excl(s, sh, &tot);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int b = b0 + 8 * (int)threadIdx.x + k;
+      if (b < (int)gridDim.x) aux[b] = ex;
+      ex += n[k];
+    }
     carry += tot;
-    __syncthreads();
   }
   if (threadIdx.x == 0) st->nliq = carry;
 }
 
-__global__ void k_liq_rank(Params P, DevState* st, const int* liq, const int* aux, int* rank) {
-  if (clu_gate(st)) return;
+__global__ void k_liq_rank(Params P, DevState* st, int force, const int* liq, const int* aux, int* rank) {
+  if (clu_gate(st, force)) return;
   __shared__ int sh[33];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int v = i < P.N ? liq[i] : 0;
@@ -306,9 +330,9 @@ __global__ void k_liq_rank(Params P, DevState* st, const int* liq, const int* au
   if (i < P.N) rank[i] = aux[blockIdx.x] + ex;
 }
 
-__global__ void k_liq_union(DevState* st, const int2* bonds, const unsigned long long* nbonds,
+__global__ void k_liq_union(DevState* st, int force, const int2* bonds, const unsigned long long* nbonds,
                             int bond_cap, const int* liq, const int* perm, int* parent2) {
-  if (clu_gate(st)) return;
+  if (clu_gate(st, force)) return;
   unsigned long long nb = *nbonds;
   if (nb > (unsigned long long)bond_cap) nb = bond_cap;
   for (unsigned long long b = blockIdx.x * blockDim.x + threadIdx.x; b < nb;
@@ -321,11 +345,11 @@ __global__ void k_liq_union(DevState* st, const int2* bonds, const unsigned long
 // tWF labels are the rank (1-based) of the component's smallest liquid atom
 // in liqmon(); the reference leaves clf() of non-liquid atoms as whatever
 // the flood fill wrote (:215-218), the engine writes 0 there.
-__global__ void k_liq_label(Params P, DevState* st, const double4* pos, const int* perm,
+__global__ void k_liq_label(Params P, DevState* st, int force, const double4* pos, const int* perm,
                             const double* vx, const double* vy, const double* vz,
                             const int* liq, const int* rank, int* parent2, int* clf, int* csf,
                             double* cekf) {
-  if (clu_gate(st)) return;
+  if (clu_gate(st, force)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.N) return;
   if (!liq[i]) {
@@ -340,9 +364,24 @@ __global__ void k_liq_label(Params P, DevState* st, const double4* pos, const in
   atomicAdd(cekf + lab, kin_energy(P, sp, vx[i], vy[i], vz[i]));
 }
 
-__global__ void k_liq_hist(Params P, DevState* st, const int* csf, const double* cekf,
-                           const int* cgsf, int* csif, double* ceksf, int* cgsfa) {
-  if (clu_gate(st)) return;
+__device__ void liq_finish(const Params& P, DevState* st, int* csif, int* cfptf) {
+  clmd_scalars& q = st->s;
+  int step = st->cur_step;
+  q.cnumf = st->nliq;
+  csif[0] = P.apnum[0] - st->nliq;  // :251 (sum of csf = number of liquid atoms)
+  int bf = __ldcg(&st->nroots_f);  // other blocks' maximum
+  if (bf > q.cbiggestf) q.cbiggestf = bf;
+  if (q.cbiggestf >= q.clookforf) {
+    for (int i = q.clookforf; i <= q.cbiggestf; i++) cfptf[i - 1] = step;
+    q.clookforf = q.clookforf + 1;
+  }
+  st->nroots_f = 0;
+}
+
+__global__ void k_liq_hist(Params P, DevState* st, int force, const int* csf, const double* cekf,
+                           const int* cgsf, int* csif, double* ceksf, int* cgsfa,
+                           int* cfptf) {
+  if (clu_gate(st, force)) return;
   __shared__ int bmax;
   if (threadIdx.x == 0) bmax = 0;
   __syncthreads();
@@ -357,33 +396,10 @@ __global__ void k_liq_hist(Params P, DevState* st, const int* csf, const double*
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) atomicMax(&st->nroots_f, bmax);
-}
-
-__global__ void k_liq_finish(Params P, DevState* st, int* csif, int* cfptf) {
-  if (clu_gate(st)) return;
-  clmd_scalars& q = st->s;
-  int step = st->cur_step;
-  q.cnumf = st->nliq;
-  csif[0] = P.apnum[0] - st->nliq;  // :251 (sum of csf = number of liquid atoms)
-  int bf = st->nroots_f;
-  if (bf > q.cbiggestf) q.cbiggestf = bf;
-  if (q.cbiggestf >= q.clookforf) {
-    for (int i = q.clookforf; i <= q.cbiggestf; i++) cfptf[i - 1] = step;
-    q.clookforf = q.clookforf + 1;
-  }
-  st->nroots_f = 0;
-}
-
-// cstep = step marks the analysis done for this step (wrt-csi.f:27)
-__global__ void k_clu_done(DevState* st) {
-  if (clu_gate(st)) return;
-  st->s.cstep = st->cur_step;
-  st->clu_force = 0;
-  int err = atomicExch(&st->err_new, 0);
-  if (err && st->s.status == 0) {
-    st->s.status = err;
-    st->s.fail_step = st->cur_step;
+  if (threadIdx.x == 0 && bmax > 0) atomicMax(&st->nroots_f, bmax);
+  if (last_block(&st->ctr[CTR_CLU2]) && threadIdx.x == 0) {
+    liq_finish(P, st, csif, cfptf);
+    clu_done(st);
   }
 }
 
@@ -409,46 +425,34 @@ __global__ void k_chk_nucleation(Params P, DevState* st, const int* csi) {
   }
 }
 
-__global__ void k_clu_force(DevState* st, int f) { st->clu_force = f; }
-
 void stoddard_launch(clmd_system* S, int force) {
   const Params& P = S->P;
   cudaStream_t s = S->stream;
   int nb = S->nblk;
-  if (force) {
-    k_clu_force<<<1, 1, 0, s>>>(S->st, 1);
-    S->launches++;
-  }
-  k_clu_prep<<<1, 1, 0, s>>>(S->st);
-  k_clu_init<<<nb, kBlock, 0, s>>>(P, S->st, S->parent, S->cs, S->cek, S->csi, S->ceks,
+  k_clu_init<<<nb, kBlock, 0, s>>>(P, S->st, force, S->parent, S->cs, S->cek, S->csi, S->ceks,
                                     S->deg, S->deg1, S->cgs, S->clf, S->csf, S->csif, S->cekf,
                                     S->ceksf, S->cgsf, S->cgsa, S->cgsfa, S->nbonds);
-  k_clu_bonds<<<nb, kBlock, 0, s>>>(P, S->st, S->pos, S->perm, S->list, S->row_start,
+  k_clu_bonds<<<nb, kBlock, 0, s>>>(P, S->st, force, S->pos, S->perm, S->list, S->row_start,
                                      S->row_len, S->row_lo, S->parent, S->deg, S->deg1,
                                      S->bonds, S->nbonds, S->bond_cap);
-  k_clu_label<<<nb, kBlock, 0, s>>>(P, S->st, S->pos, S->perm, S->vx, S->vy, S->vz, S->parent,
-                                     S->cl, S->cs, S->cek, S->cgs);
-  k_clu_hist<<<nb, kBlock, 0, s>>>(P, S->st, S->cs, S->cek, S->csi, S->ceks);
-  k_clu_finish<<<1, 1, 0, s>>>(P, S->st, S->cfpt);
-  S->launches += 6;
+  k_clu_label<<<nb, kBlock, 0, s>>>(P, S->st, force, S->pos, S->perm, S->vx, S->vy, S->vz,
+                                     S->parent, S->cl, S->cs, S->cek, S->cgs);
+  k_clu_hist<<<nb, kBlock, 0, s>>>(P, S->st, force, S->cs, S->cek, S->csi, S->ceks, S->cfpt);
+  S->launches += 4;
   if (P.clustering == CLMD_CLU_FRENKEL) {
-    k_liq_flag<<<nb, kBlock, 0, s>>>(P, S->st, S->pos, S->perm, S->vx, S->vy, S->vz, S->deg,
-                                      S->deg1, S->liq, S->liqref, S->parent2, S->cekf);
-    k_liq_tiles<<<nb, kBlock, 0, s>>>(P, S->st, S->liqref, S->scan_aux);
-    k_liq_top<<<1, 1024, 0, s>>>(S->st, S->scan_aux, nb);
-    k_liq_rank<<<nb, kBlock, 0, s>>>(P, S->st, S->liqref, S->scan_aux, S->liqrank);
+    k_liq_flag<<<nb, kBlock, 0, s>>>(P, S->st, force, S->pos, S->perm, S->vx, S->vy, S->vz,
+                                      S->deg, S->deg1, S->liq, S->liqref, S->parent2, S->cekf);
+    k_liq_tiles<<<nb, kBlock, 0, s>>>(P, S->st, force, S->liqref, S->scan_aux);
+    k_liq_rank<<<nb, kBlock, 0, s>>>(P, S->st, force, S->liqref, S->scan_aux, S->liqrank);
     int ub = 4 * S->num_sms;
-    k_liq_union<<<ub, kBlock, 0, s>>>(S->st, S->bonds, S->nbonds, S->bond_cap, S->liq,
+    k_liq_union<<<ub, kBlock, 0, s>>>(S->st, force, S->bonds, S->nbonds, S->bond_cap, S->liq,
                                        S->perm, S->parent2);
-    k_liq_label<<<nb, kBlock, 0, s>>>(P, S->st, S->pos, S->perm, S->vx, S->vy, S->vz, S->liq,
-                                       S->liqrank, S->parent2, S->clf, S->csf, S->cekf);
-    k_liq_hist<<<nb, kBlock, 0, s>>>(P, S->st, S->csf, S->cekf, S->cgsf, S->csif, S->ceksf,
-                                      S->cgsfa);
-    k_liq_finish<<<1, 1, 0, s>>>(P, S->st, S->csif, S->cfptf);
-    S->launches += 8;
+    k_liq_label<<<nb, kBlock, 0, s>>>(P, S->st, force, S->pos, S->perm, S->vx, S->vy, S->vz,
+                                       S->liq, S->liqrank, S->parent2, S->clf, S->csf, S->cekf);
+    k_liq_hist<<<nb, kBlock, 0, s>>>(P, S->st, force, S->csf, S->cekf, S->cgsf, S->csif,
+                                      S->ceksf, S->cgsfa, S->cfptf);
+    S->launches += 6;
   }
-  k_clu_done<<<1, 1, 0, s>>>(S->st);
-  S->launches += 1;
 }
 
 void chk_nucleation_launch(clmd_system* S) {

@@ -71,7 +71,6 @@ struct DevState {
   double vcom[3];
   // clustering
   int nroots, nliq, nroots_f;
-  int clu_force;                // next analysis runs even if cstep == step
   unsigned int ctr[16];         // last-block counters (one per reduction site)
   unsigned int bar_count, bar_gen;  // grid barrier of cooperative kernels
   // failure-path tests only (clmd_debug_barrier): arrivals a barrier waits
