@@ -406,8 +406,7 @@ extern "C" int clmd_clear_status(clmd_system* S) {
 
 extern "C" int clmd_neighbor(clmd_system* S, int32_t* step) {
   if (!S || !step) return set_last(CLMD_ERR_ARG);
-  k_set_step_launch(S, *step);
-  cycle_launch(S, 0, 1);
+  cycle_launch(S, 0, 1, step);
   if (*step < 0) *step = -*step;  // neighbor-pbc-mav.f:63
   return fetch(S);
 }
@@ -431,15 +430,16 @@ extern "C" int clmd_zero_acc(clmd_system* S) {
 
 extern "C" int clmd_integrator(clmd_system* S, int32_t step) {
   if (!S) return set_last(CLMD_ERR_ARG);
-  k_set_step_launch(S, step);
-  cycle_launch(S, 1, 0);
+  cycle_launch(S, 1, 0, &step);
   return fetch(S);
 }
 
 extern "C" int clmd_steps(clmd_system* S, int32_t first, int32_t nsteps) {
   if (!S || nsteps < 0) return set_last(CLMD_ERR_ARG);
-  k_set_step_launch(S, first);
-  if (nsteps > 0) cycle_launch(S, nsteps, 0);
+  if (nsteps > 0)
+    cycle_launch(S, nsteps, 0, &first);
+  else
+    k_set_step_launch(S, first);
   return fetch(S);
 }
 

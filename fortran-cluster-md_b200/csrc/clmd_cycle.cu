@@ -320,7 +320,10 @@ enum { SLOT_MAX = 0, SLOT_SUMV2 = 1, SLOT_EPOT = 2, SLOT_VIR = 3, SLOT_EKIN = 4,
 template <bool NH, bool THERMO, bool MIXED>
 __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevState* st,
                                                                 CycleArgs A, int nsteps,
-                                                                int mode) {
+                                                                int mode, int first,
+                                                                int set) {
+  // set: the first step's number (main.f's loop counter) comes with the call
+  if (set && blockIdx.x == 0 && threadIdx.x == 0) st->cur_step = first;
   if (gated(st)) return;
   __shared__ Blk B;
   __shared__ double sh[kPB / 32];
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
     B.rebuild = 0;
   }
   __syncthreads();
-  int step = st->cur_step;
+  int step = set ? first : st->cur_step;
   int cur = 0;  // positions of the current step live in pos0 / pos1
   auto posb = [&](int k) { return k ? A.pos1 : A.pos0; };
   int rb = 0;  // partial-buffer toggle
@@ -718,7 +721,7 @@ done:
 // This file is compiled twice: as is (the FP64 kernels and the host side)
 // and with CLMD_CYCLE_MIXED (the mixed-precision kernels only).  In one
 // translation unit the two sets got larger local frames and ran ~4% slower.
-typedef void (*CycleKernel)(Params, DevState*, CycleArgs, int, int);
+typedef void (*CycleKernel)(Params, DevState*, CycleArgs, int, int, int, int);
 
 #ifdef CLMD_CYCLE_MIXED
 CycleKernel cycle_kernel_mixed(bool nh, bool th) {
@@ -769,11 +772,11 @@ int cycle_blocks_for(clmd_system* S) {
   return nb < need ? nb : need;
 }
 
-void cycle_launch(clmd_system* S, int nsteps, int mode) {
+void cycle_launch(clmd_system* S, int nsteps, int mode, const int* step) {
   // small systems on one cluster, unless a failure-path test has changed the
   // grid barrier, which that kernel does not use
   if (S->small_ctas && !S->debug_barrier) {
-    small_launch(S, cycle_args(S), nsteps, mode);
+    small_launch(S, cycle_args(S), nsteps, mode, step);
     return;
   }
   cudaLaunchConfig_t cfg = {};
@@ -786,7 +789,8 @@ void cycle_launch(clmd_system* S, int nsteps, int mode) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, cycle_kernel(S), S->P, S->st, cycle_args(S), nsteps, mode);
+  cudaLaunchKernelEx(&cfg, cycle_kernel(S), S->P, S->st, cycle_args(S), nsteps, mode, step ? *step : 0,
+                     step != nullptr);
   S->launches++;
 }
 #endif  // CLMD_CYCLE_MIXED

@@ -542,6 +542,6 @@ __device__ __forceinline__ int row_store(int2* buf, int n, int ref, int* row) {
 
 // clmd_small.cu: systems of up to 16 * kSmallThreads atoms
 void small_setup(clmd_system* S);
-void small_launch(clmd_system* S, const CycleArgs& A, int nsteps, int mode);
+void small_launch(clmd_system* S, const CycleArgs& A, int nsteps, int mode, const int* step);
 
 }  // namespace clmd

@@ -220,6 +220,45 @@ __global__ void k_thermo_scale(Params P, DevState* st, const int* perm, double* 
   vz[i] = vz[i] * kf;
 }
 
+// the same in one launch, one block, for systems of a few thousand atoms: two
+// launches cost more there than the block's passes over the velocities
+constexpr int kThermoOne = 8192;
+__global__ void __launch_bounds__(1024) k_thermo_one(Params P, DevState* st, const int* perm,
+                                                     double* vx, double* vy, double* vz,
+                                                     int step) {
+  if (gated(st)) return;
+  __shared__ double sh[32], eks[CLMD_MXSORTS], kfs[CLMD_MXSORTS];
+  __shared__ int scs[CLMD_MXSORTS];
+  for (int s = 0; s < P.atsorts; s++) {
+    double e = 0.0;
+    for (int i = threadIdx.x; i < P.N; i += blockDim.x)
+      if (P.atsorts == 1 || species_block(P, perm[i]) == s)
+        e += 0.5 * P.apmas[s] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
+    const double t = block_sum(e, sh);
+    if (threadIdx.x == 0) eks[s] = t;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    double ekin = 0.0;
+    for (int s = 0; s < P.atsorts; s++) {
+      const double ek = eks[s];
+      ekin = ekin + ek;
+      kfs[s] = sqrt(P.ekinT[s] / ek);
+      scs[s] = (P.apth[s] == 'X' || step == -1);
+      if (scs[s]) ekin = ekin - ek + P.ekinT[s];
+    }
+    st->s.ekin = ekin;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < P.N; i += blockDim.x) {
+    const int sp = P.atsorts == 1 ? 0 : species_block(P, perm[i]);
+    if (sp < 0 || !scs[sp]) continue;
+    vx[i] = vx[i] * kfs[sp];
+    vy[i] = vy[i] * kfs[sp];
+    vz[i] = vz[i] * kfs[sp];
+  }
+}
+
 // stopdead-m.f:30-55
 __global__ void k_mom_sum(Params P, DevState* st, const double4* pos, const double* vx,
                           const double* vy, const double* vz, double* partials) {
@@ -357,6 +396,11 @@ void force_launch(clmd_system* S, int mode, int advance) {
 }
 
 void thermostat_launch(clmd_system* S, int step) {
+  if (S->P.N <= kThermoOne) {
+    k_thermo_one<<<1, 1024, 0, S->stream>>>(S->P, S->st, S->perm, S->vx, S->vy, S->vz, step);
+    S->launches++;
+    return;
+  }
   k_thermo_sum<<<S->nblk, kBlock, 0, S->stream>>>(S->P, S->st, S->perm, S->vx, S->vy, S->vz,
                                                    S->partials, step);
   k_thermo_scale<<<S->nblk, kBlock, 0, S->stream>>>(S->P, S->st, S->perm, S->vx, S->vy,

@@ -241,7 +241,9 @@ enum { SS_MAX = 0, SS_SUMV2, SS_EPOT, SS_VIR, SS_EKIN, SS_WV, SS_VV };
 
 template <bool NH, bool THERMO, bool MIXED>
 __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, CycleArgs A, int nsteps,
-                                                   int mode) {
+                                                   int mode, int first, int set) {
+  // set: the first step's number (main.f's loop counter) comes with the call
+  if (set && blockIdx.x == 0 && threadIdx.x == 0) st->cur_step = first;
   if (gated(st)) return;  // uniform: CTA 0 writes it back after the last barrier
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmallShared& S = *reinterpret_cast<SmallShared*>(smem_raw);
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
     B.rebuild = 0;
     S.err[0] = S.err[1] = 0;
   }
-  int step = st->cur_step;
+  int step = set ? first : st->cur_step;
   const int p = G.rank * NT + tid;
   Atom a;
   a.act = p < N;
@@ -534,7 +536,7 @@ done:
 
 // compiled twice, like clmd_cycle.cu: FP64 kernels with the host side, and
 // the mixed-precision kernels alone
-typedef void (*SmallKernel)(Params, DevState*, CycleArgs, int, int);
+typedef void (*SmallKernel)(Params, DevState*, CycleArgs, int, int, int, int);
 
 #ifdef CLMD_CYCLE_MIXED
 SmallKernel small_kernel_mixed(bool nh, bool th) {
@@ -593,11 +595,12 @@ void small_setup(clmd_system* S) {
   }
 }
 
-void small_launch(clmd_system* S, const CycleArgs& A, int nsteps, int mode) {
+void small_launch(clmd_system* S, const CycleArgs& A, int nsteps, int mode, const int* step) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   small_config(S, cfg, at);
-  cudaLaunchKernelEx(&cfg, small_kernel(S), S->P, S->st, A, nsteps, mode);
+  cudaLaunchKernelEx(&cfg, small_kernel(S), S->P, S->st, A, nsteps, mode, step ? *step : 0,
+                     step != nullptr);
   S->launches++;
 }
 #endif  // CLMD_CYCLE_MIXED

@@ -88,10 +88,11 @@ void scatter_in_launch(clmd_system* S, int hx, int hy, int hz, int hvx, int hvy,
                        int hax, int hay, int haz);
 void gather_out_launch(clmd_system* S);
 
-// clmd_cycle.cu: the persistent step kernel (mode 0: nsteps integrator
-// steps; mode 1: one neighbor() rebuild)
 int cycle_blocks_for(clmd_system* S);
-void cycle_launch(clmd_system* S, int nsteps, int mode);
+// clmd_cycle.cu: the persistent step kernel (mode 0: nsteps integrator
+// steps; mode 1: one neighbor() rebuild).  step: the first step's number, or
+// null to go on from the device's counter
+void cycle_launch(clmd_system* S, int nsteps, int mode, const int* step = nullptr);
 
 // clmd_cluster.cu
 void stoddard_launch(clmd_system* S, int force);
