@@ -388,7 +388,9 @@ extern "C" int clmd_debug_barrier(clmd_system* S, int32_t extra_arrivals, int64_
   if (!S || extra_arrivals < 0 || spin_limit < 0) return set_last(CLMD_ERR_ARG);
   CK(cudaStreamSynchronize(S->stream));
   free_graphs(S);  // captured with the other barrier's kernel
-  S->debug_barrier = extra_arrivals > 0 || spin_limit > 0;
+  // small systems then run on the grid kernel; its barriers cannot pass, so it
+  // never reads the rows, which k_small may have grouped otherwise
+  S->debug_barrier = extra_arrivals > 0;
   k_debug_barrier<<<1, 1, 0, S->stream>>>(S->st, (unsigned)extra_arrivals, (long long)spin_limit);
   S->launches++;
   CK(cudaGetLastError());

@@ -256,9 +256,11 @@ struct Pair {
 #define CLMD_FORCE_GROUP 4
 #endif
 constexpr int kGroup = CLMD_FORCE_GROUP;
+// (the term an owner adds: negated where the reference subtracts it, zero
+// beyond the cut-off; adding a zero leaves a sum as it is)
 struct WarpStage {
   double tx[32 * kGroup], ty[32 * kGroup], tz[32 * kGroup];
-  int flag[32 * kGroup];  // 0 nothing, 1 add, 2 subtract
+  int more[32 * kGroup];  // (the search's buffer is a little larger)
 };
 
 template <bool MIXED>
@@ -385,27 +387,19 @@ __device__ __forceinline__ void warp_forces(const Params& P, DevState* st, const
       continue;
     }
     const int g = (c >> 5) % kGroup;
-    W.tx[32 * g + lane] = tx;
-    W.ty[32 * g + lane] = ty;
-    W.tz[32 * g + lane] = tz;
-    W.flag[32 * g + lane] = flag;
+    W.tx[32 * g + lane] = flag == 2 ? -tx : tx;
+    W.ty[32 * g + lane] = flag == 2 ? -ty : ty;
+    W.tz[32 * g + lane] = flag == 2 ? -tz : tz;
     if (g != kGroup - 1 && c + 32 < tot) continue;  // the group is not full yet
     __syncwarp();
     const int cg = c - 32 * g;  // the group's first entry
     const int b0 = e > cg ? e : cg;
     const int b1 = (e + len) < (c + 32) ? (e + len) : (c + 32);
-    for (int a = b0; a < b1; a++) {
-      int q = a - cg;
-      int f = W.flag[q];
-      if (f == 1) {
-        fx = fx + W.tx[q];
-        fy = fy + W.ty[q];
-        fz = fz + W.tz[q];
-      } else if (f == 2) {
-        fx = fx - W.tx[q];
-        fy = fy - W.ty[q];
-        fz = fz - W.tz[q];
-      }
+#pragma unroll 2
+    for (int q = b0 - cg; q < b1 - cg; q++) {
+      fx = fx + W.tx[q];
+      fy = fy + W.ty[q];
+      fz = fz + W.tz[q];
     }
     __syncwarp();
   }

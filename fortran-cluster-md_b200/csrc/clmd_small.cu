@@ -241,7 +241,7 @@ enum { SS_MAX = 0, SS_SUMV2, SS_EPOT, SS_VIR, SS_EKIN, SS_WV, SS_VV };
 
 template <bool NH, bool THERMO, bool MIXED>
 __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, CycleArgs A, int nsteps,
-                                                   int mode, int first, int set) {
+                                                   int mode, int first, int set, int per) {
   // set: the first step's number (main.f's loop counter) comes with the call
   if (set && blockIdx.x == 0 && threadIdx.x == 0) st->cur_step = first;
   if (gated(st)) return;  // uniform: CTA 0 writes it back after the last barrier
@@ -275,7 +275,8 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
     S.err[0] = S.err[1] = 0;
   }
   int step = set ? first : st->cur_step;
-  const int p = G.rank * NT + tid;
+  // `per` atoms per warp, in its first lanes
+  const int p = G.lane < per ? G.mine * per + G.lane : N;
   Atom a;
   a.act = p < N;
   a.q = make_double4(0.0, 0.0, 0.0, 1.0);
@@ -536,7 +537,7 @@ done:
 
 // compiled twice, like clmd_cycle.cu: FP64 kernels with the host side, and
 // the mixed-precision kernels alone
-typedef void (*SmallKernel)(Params, DevState*, CycleArgs, int, int, int, int);
+typedef void (*SmallKernel)(Params, DevState*, CycleArgs, int, int, int, int, int);
 
 #ifdef CLMD_CYCLE_MIXED
 SmallKernel small_kernel_mixed(bool nh, bool th) {
@@ -566,18 +567,25 @@ static void small_config(const clmd_system* S, cudaLaunchConfig_t& cfg, cudaLaun
   cfg.numAttrs = 1;
 }
 
-// Whether the system runs on one cluster, and its shape: 128 threads a CTA
-// while that covers the atoms with 16 CTAs or fewer, then 16 CTAs of more
-// threads; one atom per thread, so N <= 16 * kSmallThreads.
+// Whether the system runs on one cluster, and its shape.  The shortest step
+// has the fewest pair terms per warp: 8 or 16 atoms in a warp's first lanes
+// while 16 CTAs of 16 warps hold the system at that, else 32.  (Mixed
+// precision sums a row's terms by chunks of the warp's entries: always 32, the
+// grid kernel's grouping.)  4 warps a CTA until that takes 16 CTAs, then more.
 void small_setup(clmd_system* S) {
   S->small_ctas = 0;
   const int N = S->P.N;
   if (N > kSC * kSmallThreads) return;
-  int nt = 128, c = (N + nt - 1) / nt;
+  int per = 32;
+  if (S->P.precision != CLMD_PREC_MIXED)
+    while (per > 8 && (N + per / 2 - 1) / (per / 2) <= kSC * kSW) per /= 2;
+  const int warps = (N + per - 1) / per;
+  int c = (warps + 3) / 4, nt = 128;
   if (c > kSC) {
     c = kSC;
-    nt = ((N + c - 1) / c + 31) / 32 * 32;
+    nt = (warps + c - 1) / c * 32;
   }
+  S->small_per = per;
   SmallKernel k = small_kernel(S);
   S->small_ctas = c;
   S->small_threads = nt;
@@ -600,7 +608,7 @@ void small_launch(clmd_system* S, const CycleArgs& A, int nsteps, int mode, cons
   cudaLaunchAttribute at[1];
   small_config(S, cfg, at);
   cudaLaunchKernelEx(&cfg, small_kernel(S), S->P, S->st, A, nsteps, mode, step ? *step : 0,
-                     step != nullptr);
+                     step != nullptr, S->small_per);
   S->launches++;
 }
 #endif  // CLMD_CYCLE_MIXED

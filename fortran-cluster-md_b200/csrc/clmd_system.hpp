@@ -62,7 +62,7 @@ struct clmd_system {
   int nblk = 1;          // ceil(N / kBlock)
   int cyc_blocks = 1;    // co-resident blocks of the persistent kernel
   int small_ctas = 0;    // CTAs of the small-system kernel's cluster (0: the grid kernel)
-  int small_threads = 0;
+  int small_threads = 0, small_per = 32;  // its threads per CTA, atoms per warp
   bool debug_barrier = false;  // clmd_debug_barrier in force
   long long launches = 0;
   // captured main-loop graph: analysis + ftcsi steps
