@@ -1075,7 +1075,8 @@ def fp64_ensemble_rate(specs, args, windows=3):
 # ---------------------------------------------------------------------------
 SERVED = dict(rate=200.0, nmin=100, nmax=50000, rho=(0.01, 0.05), temp=(0.65, 0.85),
               budget=(1e4, 1e6), csover=101, ftcsi=100, seed=11)
-POOL_BYTES_PER_ATOM = 9 * 8 + 3 * 8 + 192 * 4 + 6 * 4  # x..vzn, a, ELL list, int scratch
+POOL_BYTES_PER_ATOM = 9 * 8 + 3 * 8 + 192 * 4 + 7 * 4 + 8 + 32  # x..vzn, a, ELL list, int
+# scratch, the search's candidates, a window's packed positions
 
 
 def served_trace(arrival_s, seed):

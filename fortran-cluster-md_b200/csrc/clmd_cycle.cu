@@ -6,7 +6,7 @@
 // are separated by a grid barrier instead of kernel boundaries:
 //
 //   velocity Verlet, per step:  [force_n + kick_n + drift_n+1] -> barrier
-//                               -> skin decision -> (rebuild: 7 barriers)
+//                               -> skin decision -> (rebuild: 5 barriers)
 //   Nose-Hoover, per step:      [velocities_n + drift_n+1] -> barrier ->
 //                               (rebuild) -> force_n+1 -> barrier
 //

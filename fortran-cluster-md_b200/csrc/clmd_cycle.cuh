@@ -430,7 +430,9 @@ constexpr int kRowCap = (int)(sizeof(WarpStage) / 32 / 8);
 // FP32 rounding of the list radius: the same list, a quarter of the FP64
 // instructions, and 16 bytes a candidate instead of 36.  Two candidates are
 // loaded at a time and the next cell row's range ahead of this one's tests:
-// a thread's chain of loads, not their number, bounds the search.
+// a thread's chain of loads, not their number, bounds the search.  With the
+// rank sort of long rows neighbor() took 553 -> 380 us (N = 1,000,003) and
+// 440 -> 150 us (30,011 atoms, 30 liquid droplets).
 __device__ __forceinline__ int row_search(const Params& P, const Geo& g, int p, int ref,
                                           const double4& pa, const double4* pos,
                                           const float4* cf, const int* cs, int2* buf, int* out) {

@@ -621,7 +621,9 @@ __device__ void cta_scan16(unsigned* word, int nw) {
 // r^2), which FP64 positions decide (mi_sel and r^2 rounded term by term; r^2
 // does not depend on the pair's orientation): the pair set is the FP64
 // test's.  That test alone, three FP64 positions a candidate gathered by
-// slot, ran a chain of ~150 cycles per candidate in every lane.  Two
+// slot, ran a chain of ~150 cycles per candidate in every lane (a rebuild of
+// the average batched replica 133k cycles, now 77k; the window 57.5 -> 50.5
+// ms).  Two
 // candidates are loaded at a time, and the next cell row's range ahead of
 // this one's tests.
 template <bool SM>
@@ -1695,8 +1697,7 @@ struct clmd_ensemble {
   int* d_iwin = nullptr;   // windows per item (balanced launches)
   int* h_iwin = nullptr;   // pinned
   float* h_wtime = nullptr;  // pinned copy of A.wtime
-  // one replica's arrays on their way in or out (9 n doubles of the largest so
-  // far): contiguous, in atom order
+  // one replica's arrays on their way in or out, contiguous, in atom order
   double *d_xfer = nullptr, *h_xfer = nullptr;
   size_t xfer_cap = 0;
   double* d_stage = nullptr;  // bulk copies in atom order (pool doubles, on first use)
@@ -2044,16 +2045,16 @@ extern "C" int clmd_ens_pair_terms(clmd_ensemble* E, int64_t* total) {
 static int ensure_xfer(clmd_ensemble* E, int n) {
   size_t need = 9 * (size_t)n;
   if (need <= E->xfer_cap) return CLMD_OK;
-  // (doubled: admissions in ascending sizes would allocate each time)
-  need = std::max(need, std::min(std::max(2 * E->xfer_cap, (size_t)9 * 4096),
-                                 9 * (size_t)E->A.pool));
+  // (once for all replicas of up to 65,536 atoms: allocating takes longer than
+  // an admission)
+  need = std::max(need, 9 * (size_t)std::min<long long>(E->A.pool, 65536));
   ECK(cudaStreamSynchronize(E->stream));
   cudaFree(E->d_xfer);
   cudaFreeHost(E->h_xfer);
   E->d_xfer = E->h_xfer = nullptr;
   E->xfer_cap = 0;
   ECK(cudaMalloc(&E->d_xfer, 8 * need));
-  ECK(cudaMallocHost(&E->h_xfer, 8 * need));
+  ECK(cudaMallocHost(&E->h_xfer, 8 * need / 9 * 6));  // (only x..vz go in)
   E->xfer_cap = need;
   return CLMD_OK;
 }
@@ -2255,12 +2256,13 @@ static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const i
   }
   L.smem = (L.smem + 7) & ~(size_t)7;
   L.k = kernel_for(shape, sm, mixed);
-  // the attribute only grows: classes that share a kernel may launch it
-  // with different amounts in one sequence (occupancy follows each launch)
+  // the limit is the kernel's for the whole process, so every ensemble sets the
+  // same one (occupancy follows each launch's own amount)
   size_t& lim = E->attr_smem[(void*)L.k];
-  if (L.smem > lim) {
-    ECK(cudaFuncSetAttribute(L.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
-    lim = L.smem;
+  if (lim == 0) {
+    const size_t most = E->smem_cap - 8192;
+    ECK(cudaFuncSetAttribute(L.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    lim = most;
   }
   int per_sm = 0;
   ECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, L.k, nt, L.smem));

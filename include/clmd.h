@@ -486,7 +486,9 @@ int clmd_stoddard_noalloc(int32_t natom, const double* x, const double* y, const
  * beyond the grid (none come) and gives up after `spin_limit` polls (0: the
  * default, ~2 s); the launch then ends with CLMD_ERR_TIMEOUT, latched in the
  * status like any other error.  (0, 0) restores normal barriers.  Only for
- * tests: a timed-out system must be cleared (clmd_clear_status) or dropped. */
+ * tests: a timed-out system must be cleared (clmd_clear_status) or dropped.
+ * A system of up to 8,192 atoms, which runs on one thread-block cluster with
+ * hardware barriers, runs on the grid's while extra_arrivals > 0. */
 int clmd_debug_barrier(clmd_system* S, int32_t extra_arrivals, int64_t spin_limit);
 
 const char* clmd_status_string(int status);

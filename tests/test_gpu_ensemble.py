@@ -685,3 +685,18 @@ def test_list_entries_match_fp64(gpu, n, box, rskin):
     half = int((d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1] + d[:, 2] * d[:, 2] <= rskin * rskin).sum())
     assert e.results()[0].nrebuild == 1
     assert e.pair_terms() == 2 * half
+
+
+def test_ensembles_side_by_side(gpu):
+    """Ensembles of one process that share a kernel and need different amounts
+    of shared memory step in turn."""
+    es = []
+    for n, rho in ((4000, 0.05), (3000, 0.01), (2500, 0.05)):
+        e = clmd.Ensemble(clmd.ens_config(n, 1, ftcsi=5))
+        box, arrs = replica_inputs(n, rho, 0.75, n)
+        assert e.add(n, box, 0.75, *arrs) is not None
+        es.append(e)
+    for _ in range(2):
+        for e in es:
+            e.step(1)
+    assert [e.results()[0].step for e in es] == [10, 10, 10]
