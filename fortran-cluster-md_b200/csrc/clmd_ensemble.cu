@@ -1698,7 +1698,7 @@ struct clmd_ensemble {
   int* h_iwin = nullptr;   // pinned
   float* h_wtime = nullptr;  // pinned copy of A.wtime
   // one replica's arrays on their way in or out, contiguous, in atom order
-  double *d_xfer = nullptr, *h_xfer = nullptr;
+  double* d_xfer = nullptr;
   size_t xfer_cap = 0;
   double* d_stage = nullptr;  // bulk copies in atom order (pool doubles, on first use)
   long long* d_hoff = nullptr;  // clmd_ens_step_io: each slot's offset in the host arrays
@@ -1970,7 +1970,6 @@ extern "C" int clmd_ens_destroy(clmd_ensemble* E) {
   if (E->h_iwin) cudaFreeHost(E->h_iwin);
   if (E->h_wtime) cudaFreeHost(E->h_wtime);
   if (E->h_summary) cudaFreeHost(E->h_summary);
-  if (E->h_xfer) cudaFreeHost(E->h_xfer);
   if (E->stream) cudaStreamDestroy(E->stream);
   for (int c = 0; c < clmd_ensemble::kClasses; c++) {
     if (E->cstream[c]) cudaStreamDestroy(E->cstream[c]);
@@ -2045,16 +2044,14 @@ extern "C" int clmd_ens_pair_terms(clmd_ensemble* E, int64_t* total) {
 static int ensure_xfer(clmd_ensemble* E, int n) {
   size_t need = 9 * (size_t)n;
   if (need <= E->xfer_cap) return CLMD_OK;
-  // (once for all replicas of up to 65,536 atoms: allocating takes longer than
-  // an admission)
-  need = std::max(need, 9 * (size_t)std::min<long long>(E->A.pool, 65536));
+  // (for replicas of up to 16,384 atoms at once; then doubled)
+  need = std::max(need, std::min(std::max(2 * E->xfer_cap, (size_t)9 * 16384),
+                                 9 * (size_t)E->A.pool));
   ECK(cudaStreamSynchronize(E->stream));
   cudaFree(E->d_xfer);
-  cudaFreeHost(E->h_xfer);
-  E->d_xfer = E->h_xfer = nullptr;
+  E->d_xfer = nullptr;
   E->xfer_cap = 0;
   ECK(cudaMalloc(&E->d_xfer, 8 * need));
-  ECK(cudaMallocHost(&E->h_xfer, 8 * need / 9 * 6));  // (only x..vz go in)
   E->xfer_cap = need;
   return CLMD_OK;
 }
@@ -2123,8 +2120,9 @@ extern "C" int clmd_ens_add(clmd_ensemble* E, const clmd_replica_spec* sp, const
     }
   }
   const double* src[6] = {x, y, z, vx, vy, vz};
-  for (int k = 0; k < 6; k++) memcpy(E->h_xfer + (size_t)k * N, src[k], 8 * (size_t)N);
-  ECK(cudaMemcpyAsync(E->d_xfer, E->h_xfer, 48 * (size_t)N, cudaMemcpyHostToDevice, st));
+  for (int k = 0; k < 6; k++)
+    ECK(cudaMemcpyAsync(E->d_xfer + (size_t)k * N, src[k], 8 * (size_t)N, cudaMemcpyHostToDevice,
+                        st));
   Rep& R = E->h_reps[s];
   memset(&R, 0, sizeof(Rep));
   R.box = sp->box;
