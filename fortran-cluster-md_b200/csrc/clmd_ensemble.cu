@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/clmd.h"
+#include "clmd_ens_launch.hpp"
 #include "clmd_mixed.cuh"
 
 namespace clmd_ens {
@@ -87,7 +88,6 @@ struct Args {
   int smem;  // dynamic shared memory of this launch (bytes)
   int lg;  // mixed force pass: 1 << lg lanes per atom (0: one thread per atom)
   int reorder_every;  // the atoms' order renewed at every k-th rebuild
-  int ncmax;  // cells per dimension this launch's shared memory holds
   int4* summary;  // per slot: done, status, step, maxcs
   float* wtime;   // per slot: device ms per MD step in its last launch (one CTA)
   // replicas run by a thread-block cluster: each cluster's cell counts and
@@ -1780,8 +1780,6 @@ static bool shape_ok(int shape) {
   }
 }
 
-typedef void (*EnsKernel)(Args);
-
 // the cluster kernel of cs CTAs per replica (1024 threads each)
 static EnsKernel cluster_kernel(int cs, bool mixed) {
   switch (cs) {
@@ -2201,16 +2199,6 @@ static EnsKernel kernel_for(int shape, bool sm, bool mixed) {
   }
 }
 
-// the launch shape of one size class: kernel, dynamic shared memory, grid
-struct ClassLaunch {
-  EnsKernel k = nullptr;
-  size_t smem = 0;
-  int grid = 0, nt = 0, ncmax = 1, item0 = 0, nitems = 0;
-  int cs = 1;       // CTAs per replica (thread-block cluster size)
-  int lg = 0;       // lanes per atom in the mixed force pass: 1 << lg
-  int region0 = 0;  // first cell-count region (cluster classes)
-};
-
 static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const int* slots,
                          int shape, ClassLaunch& L) {
   L = ClassLaunch();
@@ -2227,8 +2215,9 @@ static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const i
     L.cs = E->cls_cs[c];
     L.nt = 1024;
     L.k = cluster_kernel(L.cs, mixed);
-    for (int k = 0; k < nitems; k++) L.ncmax = std::max(L.ncmax, E->h_reps[slots[k]].ncmax);
-    L.smem = cluster_smem(L.ncmax);
+    int ncmax = 1;
+    for (int k = 0; k < nitems; k++) ncmax = std::max(ncmax, E->h_reps[slots[k]].ncmax);
+    L.smem = cluster_smem(ncmax);
     L.region0 = E->cl_region0[c];
     const int nclu = std::min(E->cl_max_clusters[c], nitems);
     if (nclu < 1) return CLMD_ERR_ARG;
@@ -2250,7 +2239,6 @@ static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const i
       need = with + 8192 <= E->smem_cap ? with : base;
     }
     L.smem = std::max(L.smem, need);
-    L.ncmax = std::max(L.ncmax, R.ncmax);
   }
   L.smem = (L.smem + 7) & ~(size_t)7;
   L.k = kernel_for(shape, sm, mixed);
@@ -2281,7 +2269,6 @@ static int enqueue_class(clmd_ensemble* E, int c, const ClassLaunch& L, int nwin
   A.ctr = E->d_ctr + c;
   A.nitems = L.nitems;
   A.nwin = nwin;
-  A.ncmax = L.ncmax;
   A.lg = L.lg;
   A.smem = (int)L.smem;
   const unsigned fl = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -2396,26 +2383,17 @@ static int launch_all(clmd_ensemble* E, int nwin, const int* threads, float min_
   }
   if (total == 0) return CLMD_OK;
   ClassLaunch L[clmd_ensemble::kClasses];
-  std::vector<long long> key;
-  key.reserve(total + 64);
-  key.push_back(total);
-  key.push_back(nwin);
-  key.push_back(balanced);
-  for (int k = 0; k < total; k++) key.push_back(E->h_items[k]);
   {
     int off = 0;
     for (int c = 0; c < clmd_ensemble::kClasses; c++) {
       for (int s : cls[c]) E->last_atoms[c] += E->h_reps[s].natom;
       int st = prepare_class(E, c, off, (int)cls[c].size(), cls[c].data(), threads[c], L[c]);
       if (st) return st;
-      key.push_back(L[c].nt);
-      key.push_back(L[c].lg);
-      key.push_back(L[c].grid);
-      key.push_back((long long)L[c].smem);
-      key.push_back((long long)(size_t)L[c].k);
       off += (int)cls[c].size();
     }
   }
+  const std::vector<long long> key =
+      launch_key(nwin, balanced, E->h_items, total, L, clmd_ensemble::kClasses);
   // the sequence: item list (+ balanced step counts) in, the classes on their
   // streams, per-slot timings and summaries out
   auto enqueue = [&](bool capturing) -> int {
