@@ -213,24 +213,6 @@ __device__ __forceinline__ bool cta_nh_root_commit(double S, double psi1, double
   return sh[101] != 0.0;
 }
 
-// block max of a and sum of b in one round (as cta_sum2)
-template <int NT>
-__device__ __forceinline__ void cta_maxsum(double& a, double& b, double* sh) {
-  constexpr int W = NT / 32;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  a = wmax(a);
-  b = wsum(b);
-  if (lane == 0) {
-    sh[w] = a;
-    sh[W + w] = b;
-  }
-  __syncthreads();
-  double ta = lane < W ? sh[lane] : 0.0, tb = lane < W ? sh[W + lane] : 0.0;
-  a = wmax(ta);
-  b = wsum(tb);
-  __syncthreads();
-}
-
 // minimum image of a pair difference d in (-L - skin, L + skin): the image
 // the reference's formulas pick for every pair nearer than L/2 (they differ
 // only within rounding of |d| = L/2, beyond every cut-off since the list
@@ -269,6 +251,7 @@ __device__ __forceinline__ double mi_bf(double d, double L, double iL, double bf
 struct Cta {
   double xred[3 * 16];  // cluster reductions: the CTAs' partials (rank 0's copy is read)
   double xloc[4];       // cluster reductions: the totals, for this CTA's threads
+  double* sub;          // cluster: the warps' sums of a pass's first half, by slot
   double* sx;  // positions in shared memory (nullptr: global)
   double* sy;
   double* sz;
@@ -317,22 +300,52 @@ __device__ __forceinline__ void gsync() {
     cg::this_cluster().sync();
 }
 
-// the cluster level of a reduction of nv values (v[k]: this CTA's totals,
-// the same in every thread): returns the cluster totals in v.  op 0 sums,
-// op 1 takes maxima.  Two cluster barriers: the partials are published, then
-// read by every CTA before any CTA may write the next reduction's.
-template <int CS>
-__device__ __forceinline__ void cl_reduce(double* v, int nv, const int* op, Cta& C) {
+// A replica's sums do not depend on the cluster that runs it, so that the
+// launch may choose that by its load (launch_all): their shape is that of the
+// replica's wider cluster.  On the one of half as many CTAs (H = 2) the loops
+// that sum go over the atoms in two halves: thread t of CTA r stands for
+// thread t of CTA r, then for thread t of CTA r + CS, of the wider one.  The
+// first half's warp sums wait in C.sub (half_out) for the grp_* call.  The
+// two halves cost 1-2% of a window (FP64: 2-3%).
+__device__ __forceinline__ void half_out(double& v, int slot, Cta& C) {
+  v = wsum(v);
+  if ((threadIdx.x & 31) == 0) C.sub[32 * slot + (threadIdx.x >> 5)] = v;
+  v = 0.0;
+}
+
+// a reduction over a cluster's threads (1024 a CTA) of nv <= 3 values,
+// returned in v to every thread; op 0 sums, op 1 takes maxima; H = 2: the
+// sums' first halves are in C.sub's slots from `slot` on.  Two cluster
+// barriers: the CTAs' partials are published, then read by every CTA before
+// any CTA may write the next reduction's.
+template <int CS, int H>
+__device__ __forceinline__ void cl_reduce(double* v, int nv, const int* op, Cta& C, int slot) {
   auto cl = cg::this_cluster();
   const unsigned r = cl.block_rank();
-  double* b0 = cl.map_shared_rank(C.xred, 0);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < nv; k++) b0[k * 16 + r] = v[k];
-  cl.sync();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int k = 0; k < nv; k++) {
+    const double t = op[k] ? wmax(v[k]) : wsum(v[k]);
+    if (lane == 0) C.red[32 * k + w] = t;
+  }
+  __syncthreads();
+  if (w == 0) {
+    double* b0 = cl.map_shared_rank(C.xred, 0);
     for (int k = 0; k < nv; k++) {
-      double t = lane < CS ? b0[k * 16 + lane] : (op[k] ? -1.0e300 : 0.0);
+      double t = C.red[32 * k + lane], t0 = 0.0;
+      if (H == 2) t0 = op[k] ? t : C.sub[32 * (slot + k) + lane];
+      t = op[k] ? wmax(t) : wsum(t);
+      if (H == 2) t0 = op[k] ? t : wsum(t0);
+      if (lane == 0) {
+        if (H == 2) b0[k * 16 + r] = t0;
+        b0[k * 16 + (H - 1) * CS + r] = t;
+      }
+    }
+  }
+  cl.sync();
+  if (w == 0) {
+    const double* b0 = cl.map_shared_rank(C.xred, 0);
+    for (int k = 0; k < nv; k++) {
+      double t = lane < H * CS ? b0[k * 16 + lane] : (op[k] ? -1.0e300 : 0.0);
       t = op[k] ? wmax(t) : wsum(t);
       if (lane == 0) C.xloc[k] = t;
     }
@@ -341,64 +354,46 @@ __device__ __forceinline__ void cl_reduce(double* v, int nv, const int* op, Cta&
   for (int k = 0; k < nv; k++) v[k] = C.xloc[k];
 }
 
-template <int NT, int CS>
-__device__ __forceinline__ double grp_sum(double v, Cta& C) {
-  double t = cta_sum<NT>(v, C.red);
-  if constexpr (CS > 1) {
+template <int NT, int CS, int H = 1>
+__device__ __forceinline__ double grp_sum(double v, Cta& C, int slot = 0) {
+  if constexpr (CS == 1) {
+    return cta_sum<NT>(v, C.red);
+  } else {
     const int op[1] = {0};
-    cl_reduce<CS>(&t, 1, op, C);
+    cl_reduce<CS, H>(&v, 1, op, C, slot);
+    return v;
   }
-  return t;
 }
 template <int NT, int CS>
 __device__ __forceinline__ double grp_max(double v, Cta& C) {
-  double t = cta_max<NT>(v, C.red);
-  if constexpr (CS > 1) {
+  if constexpr (CS == 1) {
+    return cta_max<NT>(v, C.red);
+  } else {
     const int op[1] = {1};
-    cl_reduce<CS>(&t, 1, op, C);
-  }
-  return t;
-}
-template <int NT, int CS>
-__device__ __forceinline__ void grp_maxsum(double& a, double& b, Cta& C) {
-  cta_maxsum<NT>(a, b, C.red);
-  if constexpr (CS > 1) {
-    double v[2] = {a, b};
-    const int op[2] = {1, 0};
-    cl_reduce<CS>(v, 2, op, C);
-    a = v[0];
-    b = v[1];
+    cl_reduce<CS, 1>(&v, 1, op, C, 0);
+    return v;
   }
 }
+// (two integer sums, exact in any order, and an "any" flag)
 template <int NT, int CS>
 __device__ __forceinline__ void grp_sum2(double& a, double& b, int& f, Cta& C) {
-  cta_sum2<NT>(a, b, f, C.red);
-  if constexpr (CS > 1) {
+  if constexpr (CS == 1) {
+    cta_sum2<NT>(a, b, f, C.red);
+  } else {
     double v[3] = {a, b, f ? 1.0 : 0.0};
     const int op[3] = {0, 0, 1};
-    cl_reduce<CS>(v, 3, op, C);
+    cl_reduce<CS, 1>(v, 3, op, C, 0);
     a = v[0];
     b = v[1];
     f = v[2] != 0.0;
   }
 }
-template <int NT, int CS>
-__device__ __forceinline__ int grp_or(int f, Cta& C) {
-  if constexpr (CS == 1) {
-    return __syncthreads_or(f);
-  } else {
-    double v[1] = {(double)__syncthreads_or(f)};
-    const int op[1] = {1};
-    cl_reduce<CS>(v, 1, op, C);
-    return v[0] != 0.0;
-  }
-}
 // the closed-form Nose-Hoover root of a cluster's total of S: warp 0 of
 // every CTA takes the same root from the same total
-template <int NT, int CS>
+template <int NT, int CS, int H>
 __device__ __forceinline__ bool cl_nh_root(double S, double psi1, double nkt3, double dth,
                                            double Q, Cta& C, double& Stot, double& p) {
-  const double t = grp_sum<NT, CS>(S, C);
+  const double t = grp_sum<NT, CS, H>(S, C);
   if (threadIdx.x < 32) {
     double pr;
     const bool ok = clmd_nh_root(t, psi1, nkt3, dth, Q, pr);
@@ -946,7 +941,7 @@ struct RowWalk {
 // velocity-Verlet second half kick; FP64 energy/virial sums when asked
 // NHF: also the Nose-Hoover solve's first pass on the fresh accelerations
 // (vo = v: vxn = v, s0 += v.v, dp += b vo dt/Q with b = -dth (a - psi1 vo))
-template <int NT, bool SM, bool MIXED, int CS, bool NHF = false>
+template <int NT, bool SM, bool MIXED, int CS, int H, bool NHF = false>
 __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kick,
                        bool energies, double* s0 = nullptr) {
   const int N = R.natom, off = R.off, tid = threadIdx.x;
@@ -1029,106 +1024,117 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
         if (energies) ek += 0.5 * (vxi * vxi + vyi * vyi + vzi * vzi);
       }
     }
-  } else
-  for (int i0 = 0; i0 < N; i0 += GT) {
-    const int i = i0 + gt;
-    if (i >= N) continue;
-    double xi, yi, zi;
-    P.get(i, xi, yi, zi);
-    const int len = A.rlen[off + i];
-    double ax, ay, az;
-    if (MIXED) {
-      float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-      RowWalk<SM> w(P, A.list + lbase + i, len, N);
+  } else {
+    for (int h = 0; h < H; h++) {
+      if (h > 0) {
+        if (NHF) half_out(*s0, 0, C);
+        if (energies) {
+          half_out(esum, 1, C);
+          half_out(vir, 2, C);
+          half_out(ek, 3, C);
+        }
+      }
+      for (int i0 = h * GT; i0 < N; i0 += H * GT) {
+        const int i = i0 + gt;
+        if (i >= N) continue;
+        double xi, yi, zi;
+        P.get(i, xi, yi, zi);
+        const int len = A.rlen[off + i];
+        double ax, ay, az;
+        if (MIXED) {
+          float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+          RowWalk<SM> w(P, A.list + lbase + i, len, N);
 #pragma unroll 2
-      for (int k = 0; k < len; k++) {
-        const int j = w.j;
-        double dx, dy, dz;
-        w.get(P, dx, dy, dz);
-        w.next(P, k);
-        dx = mi_sel(xi - dx, L, hL);
-        dy = mi_sel(yi - dy, L, hL);
-        dz = mi_sel(zi - dz, L, hL);
-        double r2d = dx * dx + dy * dy + dz * dz;
-        if (r2d <= rc2) {
-          float r2 = (float)r2d;
-          float ri2 = clmd_rcp_f32(r2);
-          float r6 = ri2 * ri2 * ri2;
-          float fij = 48.0f * ri2 * r6 * (r6 - 0.5f);
-          kahan(fx, cx, fij * (float)dx);
-          kahan(fy, cy, fij * (float)dy);
-          kahan(fz, cz, fij * (float)dz);
-          if (energies && i < j) {
-            esum += (double)(4.0f * r6 * (r6 - 1.0f));
-            vir += (double)(fij * r2);
+          for (int k = 0; k < len; k++) {
+            const int j = w.j;
+            double dx, dy, dz;
+            w.get(P, dx, dy, dz);
+            w.next(P, k);
+            dx = mi_sel(xi - dx, L, hL);
+            dy = mi_sel(yi - dy, L, hL);
+            dz = mi_sel(zi - dz, L, hL);
+            double r2d = dx * dx + dy * dy + dz * dz;
+            if (r2d <= rc2) {
+              float r2 = (float)r2d;
+              float ri2 = clmd_rcp_f32(r2);
+              float r6 = ri2 * ri2 * ri2;
+              float fij = 48.0f * ri2 * r6 * (r6 - 0.5f);
+              kahan(fx, cx, fij * (float)dx);
+              kahan(fy, cy, fij * (float)dy);
+              kahan(fz, cz, fij * (float)dz);
+              if (energies && i < j) {
+                esum += (double)(4.0f * r6 * (r6 - 1.0f));
+                vir += (double)(fij * r2);
+              }
+            }
           }
+          float* a = (float*)A.a;
+          a[off + i] = fx;
+          a[A.pool + off + i] = fy;
+          a[2 * A.pool + off + i] = fz;
+          ax = (double)fx;
+          ay = (double)fy;
+          az = (double)fz;
+        } else {
+          double fx = 0.0, fy = 0.0, fz = 0.0;
+          RowWalk<SM> w(P, A.list + lbase + i, len, N);
+          for (int k = 0; k < len; k++) {
+            const int j = w.j;
+            double dx, dy, dz;
+            w.get(P, dx, dy, dz);
+            w.next(P, k);
+            dx = mi_sel(xi - dx, L, hL);
+            dy = mi_sel(yi - dy, L, hL);
+            dz = mi_sel(zi - dz, L, hL);
+            double r2d = dx * dx + dy * dy + dz * dz;
+            if (r2d <= rc2) {
+              double ri2 = 1.0 / r2d;
+              double r6 = ri2 * ri2 * ri2;
+              double fij = 48.0 * ri2 * r6 * (r6 - 0.5);
+              fx += fij * dx;
+              fy += fij * dy;
+              fz += fij * dz;
+              if (energies && i < j) {
+                esum += 4.0 * r6 * (r6 - 1.0);
+                vir += fij * r2d;
+              }
+            }
+          }
+          double* a = (double*)A.a;
+          a[off + i] = fx;
+          a[A.pool + off + i] = fy;
+          a[2 * A.pool + off + i] = fz;
+          ax = fx;
+          ay = fy;
+          az = fz;
+        }
+        if (NHF) {
+          // closed-form solve (clmd_nh_root): W = V + dth a into vn, s0 += W.W
+          const double dth = 0.5 * dt;
+          const double wx = A.vx[off + i] + dth * ax;
+          const double wy = A.vy[off + i] + dth * ay;
+          const double wz = A.vz[off + i] + dth * az;
+          A.vxn[off + i] = wx;
+          A.vyn[off + i] = wy;
+          A.vzn[off + i] = wz;
+          *s0 += wx * wx + wy * wy + wz * wz;
+        }
+        if (kick) {
+          double vxi = A.vx[off + i] + 0.5 * ax * dt;
+          double vyi = A.vy[off + i] + 0.5 * ay * dt;
+          double vzi = A.vz[off + i] + 0.5 * az * dt;
+          A.vx[off + i] = vxi;
+          A.vy[off + i] = vyi;
+          A.vz[off + i] = vzi;
+          if (energies) ek += 0.5 * (vxi * vxi + vyi * vyi + vzi * vzi);
         }
       }
-      float* a = (float*)A.a;
-      a[off + i] = fx;
-      a[A.pool + off + i] = fy;
-      a[2 * A.pool + off + i] = fz;
-      ax = (double)fx;
-      ay = (double)fy;
-      az = (double)fz;
-    } else {
-      double fx = 0.0, fy = 0.0, fz = 0.0;
-      RowWalk<SM> w(P, A.list + lbase + i, len, N);
-      for (int k = 0; k < len; k++) {
-        const int j = w.j;
-        double dx, dy, dz;
-        w.get(P, dx, dy, dz);
-        w.next(P, k);
-        dx = mi_sel(xi - dx, L, hL);
-        dy = mi_sel(yi - dy, L, hL);
-        dz = mi_sel(zi - dz, L, hL);
-        double r2d = dx * dx + dy * dy + dz * dz;
-        if (r2d <= rc2) {
-          double ri2 = 1.0 / r2d;
-          double r6 = ri2 * ri2 * ri2;
-          double fij = 48.0 * ri2 * r6 * (r6 - 0.5);
-          fx += fij * dx;
-          fy += fij * dy;
-          fz += fij * dz;
-          if (energies && i < j) {
-            esum += 4.0 * r6 * (r6 - 1.0);
-            vir += fij * r2d;
-          }
-        }
-      }
-      double* a = (double*)A.a;
-      a[off + i] = fx;
-      a[A.pool + off + i] = fy;
-      a[2 * A.pool + off + i] = fz;
-      ax = fx;
-      ay = fy;
-      az = fz;
-    }
-    if (NHF) {
-      // closed-form solve (clmd_nh_root): W = V + dth a into vn, s0 += W.W
-      const double dth = 0.5 * dt;
-      const double wx = A.vx[off + i] + dth * ax;
-      const double wy = A.vy[off + i] + dth * ay;
-      const double wz = A.vz[off + i] + dth * az;
-      A.vxn[off + i] = wx;
-      A.vyn[off + i] = wy;
-      A.vzn[off + i] = wz;
-      *s0 += wx * wx + wy * wy + wz * wz;
-    }
-    if (kick) {
-      double vxi = A.vx[off + i] + 0.5 * ax * dt;
-      double vyi = A.vy[off + i] + 0.5 * ay * dt;
-      double vzi = A.vz[off + i] + 0.5 * az * dt;
-      A.vx[off + i] = vxi;
-      A.vy[off + i] = vyi;
-      A.vz[off + i] = vzi;
-      if (energies) ek += 0.5 * (vxi * vxi + vyi * vyi + vzi * vzi);
     }
   }
   if (energies) {
-    double e = grp_sum<NT, CS>(esum, C);
-    double w = grp_sum<NT, CS>(vir, C);
-    double k = kick ? grp_sum<NT, CS>(ek, C) : 0.0;
+    double e = grp_sum<NT, CS, H>(esum, C, 1);
+    double w = grp_sum<NT, CS, H>(vir, C, 2);
+    double k = kick ? grp_sum<NT, CS, H>(ek, C, 3) : 0.0;
     if (tid == 0) {
       R.epot = e;
       R.virial = w;
@@ -1157,30 +1163,40 @@ __device__ __forceinline__ void get_a(const Args& A, int k, double& ax, double& 
 }
 
 // stopdead-m.f:28-69 (one species, m = 1): COM removal and rescale to T
-template <int NT, int CS>
+template <int NT, int CS, int H>
 __device__ void stopdead(Rep& R, Cta& C, const Args& A) {
   const int N = R.natom, off = R.off, tid = threadIdx.x;
   const int gt = gtid<NT, CS>();
   constexpr int GT = NT * CS;
   for (int loop = 0; loop < 10; loop++) {
     double px = 0, py = 0, pz = 0;
-    for (int i = gt; i < N; i += GT) {
-      px += A.vx[off + i];
-      py += A.vy[off + i];
-      pz += A.vz[off + i];
+    for (int h = 0; h < H; h++) {
+      if (h > 0) {
+        half_out(px, 0, C);
+        half_out(py, 1, C);
+        half_out(pz, 2, C);
+      }
+      for (int i = gt + h * GT; i < N; i += H * GT) {
+        px += A.vx[off + i];
+        py += A.vy[off + i];
+        pz += A.vz[off + i];
+      }
     }
-    double vxs = grp_sum<NT, CS>(px, C) / (double)N;
-    double vys = grp_sum<NT, CS>(py, C) / (double)N;
-    double vzs = grp_sum<NT, CS>(pz, C) / (double)N;
+    double vxs = grp_sum<NT, CS, H>(px, C, 0) / (double)N;
+    double vys = grp_sum<NT, CS, H>(py, C, 1) / (double)N;
+    double vzs = grp_sum<NT, CS, H>(pz, C, 2) / (double)N;
     double ek = 0.0;
-    for (int i = gt; i < N; i += GT) {
-      double a = A.vx[off + i] - vxs, b = A.vy[off + i] - vys, c = A.vz[off + i] - vzs;
-      A.vx[off + i] = a;
-      A.vy[off + i] = b;
-      A.vz[off + i] = c;
-      ek += 0.5 * (a * a + b * b + c * c);
+    for (int h = 0; h < H; h++) {
+      if (h > 0) half_out(ek, 0, C);
+      for (int i = gt + h * GT; i < N; i += H * GT) {
+        double a = A.vx[off + i] - vxs, b = A.vy[off + i] - vys, c = A.vz[off + i] - vzs;
+        A.vx[off + i] = a;
+        A.vy[off + i] = b;
+        A.vz[off + i] = c;
+        ek += 0.5 * (a * a + b * b + c * c);
+      }
     }
-    ek = grp_sum<NT, CS>(ek, C);
+    ek = grp_sum<NT, CS, H>(ek, C);
     double kf = sqrt(R.ekinT / ek);  // scalev-nh-m.f with step = -1
     for (int i = gt; i < N; i += GT) {
       A.vx[off + i] *= kf;
@@ -1332,7 +1348,7 @@ __device__ void host_io(const Rep& R, const Cta& C, const Args& A, bool in) {
   gsync<CS>();
 }
 
-template <int NT, bool SM, bool MIXED, int CS>
+template <int NT, bool SM, bool MIXED, int CS, int H>
 __device__ void run_window(Rep& R, Cta& C, const Args& A) {
   const int tid = threadIdx.x;
   const int gt = gtid<NT, CS>();
@@ -1362,11 +1378,11 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
   gsync<CS>();
   if (!R.started) {
     // stopdead(-1), neighbor(0), a = 0 + AccAtom, main.f:156-166
-    stopdead<NT, CS>(R, C, A);
+    stopdead<NT, CS, H>(R, C, A);
     if (tid == 0) C.flag = prologue(R, C, A, 0);
     gsync<CS>();
     if (!C.flag || !rebuild<NT, SM, CS>(R, C, A, P)) goto out;
-    forces<NT, SM, MIXED, CS>(R, C, A, P, false, true);
+    forces<NT, SM, MIXED, CS, H>(R, C, A, P, false, true);
     if (tid == 0) {
       R.sumv2 = 2.0 * R.ekin;
       R.psi = (R.ethst == 'N') ? (R.sumv2 - R.nkt3_d) / R.Q : 0.0;
@@ -1413,43 +1429,49 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
       const double* svz = vin_n ? A.vzn : A.vz;
       const double sc = vin_n ? vsc : 1.0;
       vin_n = false;
-      for (int i = gt; i < N; i += GT) {
-        double vxi = svx[off + i], vyi = svy[off + i], vzi = svz[off + i];
-        vxi = vxi * sc;
-        vyi = vyi * sc;
-        vzi = vzi * sc;
-        double axi, ayi, azi;
-        get_a<MIXED>(A, off + i, axi, ayi, azi);
-        double dx, dy, dz;
-        if (!nh) {
-          double hx = 0.5 * axi * dt, hy = 0.5 * ayi * dt, hz = 0.5 * azi * dt;
-          dx = (vxi + hx) * dt;
-          dy = (vyi + hy) * dt;
-          dz = (vzi + hz) * dt;
-          vxi += hx;
-          vyi += hy;
-          vzi += hz;
-        } else {
-          dx = dt * vxi + dt2 * (axi - psi * vxi);
-          dy = dt * vyi + dt2 * (ayi - psi * vyi);
-          dz = dt * vzi + dt2 * (azi - psi * vzi);
-          sv += vxi * vxi + vyi * vyi + vzi * vzi;
-          vxi = vxi + dth * (axi - psi * vxi);
-          vyi = vyi + dth * (ayi - psi * vyi);
-          vzi = vzi + dth * (azi - psi * vzi);
+      for (int h = 0; h < H; h++) {
+        if (h > 0) half_out(sv, 0, C);
+        for (int i = gt + h * GT; i < N; i += H * GT) {
+          double vxi = svx[off + i], vyi = svy[off + i], vzi = svz[off + i];
+          vxi = vxi * sc;
+          vyi = vyi * sc;
+          vzi = vzi * sc;
+          double axi, ayi, azi;
+          get_a<MIXED>(A, off + i, axi, ayi, azi);
+          double dx, dy, dz;
+          // (products of the half kick rounded before the addition, in every
+          // kernel alike)
+          if (!nh) {
+            const double hx = __dmul_rn(0.5 * axi, dt), hy = __dmul_rn(0.5 * ayi, dt),
+                         hz = __dmul_rn(0.5 * azi, dt);
+            vxi = __dadd_rn(vxi, hx);
+            vyi = __dadd_rn(vyi, hy);
+            vzi = __dadd_rn(vzi, hz);
+            dx = vxi * dt;
+            dy = vyi * dt;
+            dz = vzi * dt;
+          } else {
+            dx = dt * vxi + dt2 * (axi - psi * vxi);
+            dy = dt * vyi + dt2 * (ayi - psi * vyi);
+            dz = dt * vzi + dt2 * (azi - psi * vzi);
+            sv += vxi * vxi + vyi * vyi + vzi * vzi;
+            vxi = __dadd_rn(vxi, __dmul_rn(dth, axi - psi * vxi));
+            vyi = __dadd_rn(vyi, __dmul_rn(dth, ayi - psi * vyi));
+            vzi = __dadd_rn(vzi, __dmul_rn(dth, azi - psi * vzi));
+          }
+          double px, py, pz;
+          P.get(i, px, py, pz);
+          P.set(i, px + dx, py + dy, pz + dz);
+          A.vx[off + i] = vxi;
+          A.vy[off + i] = vyi;
+          A.vz[off + i] = vzi;
+          d2 = fmax(d2, dx * dx + dy * dy + dz * dz);
         }
-        double px, py, pz;
-        P.get(i, px, py, pz);
-        P.set(i, px + dx, py + dy, pz + dz);
-        A.vx[off + i] = vxi;
-        A.vy[off + i] = vyi;
-        A.vz[off + i] = vzi;
-        d2 = fmax(d2, dx * dx + dy * dy + dz * dz);
       }
       // the step's scalar logic on thread 0 (the reference's NH half step of
       // PSI and s, int-verlet-mav.f:64-74 skin bookkeeping, the rebuild
       // decision); one CTA: warp 0 takes the block totals between the two
-      // barriers (the same tree as cta_maxsum), so one barrier fewer
+      // barriers, so one barrier fewer
       double dmmr = 0.0, sumv2 = 0.0;
       if constexpr (CS == 1) {
         constexpr int W = NT / 32;
@@ -1466,9 +1488,12 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
           sumv2 = wsum(lane < W ? C.red[W + lane] : 0.0);
         }
       } else {
-        grp_maxsum<NT, CS>(d2, sv, C);
-        dmmr = d2;
-        sumv2 = sv;
+        // (slot 0 of C.sub is the second value's)
+        double t[2] = {d2, sv};
+        const int op[2] = {1, 0};
+        cl_reduce<CS, H>(t, 2, op, C, -1);
+        dmmr = t[0];
+        sumv2 = t[1];
       }
       if (tid == 0) {
         if (nh) {
@@ -1485,18 +1510,18 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
       if (C.flag == 0) goto out;
       if (C.flag == 2 && !rebuild<NT, SM, CS>(R, C, A, P)) goto out;
       if (!nh) {
-        forces<NT, SM, MIXED, CS>(R, C, A, P, true, last);
+        forces<NT, SM, MIXED, CS, H>(R, C, A, P, true, last);
       } else {
         // int-verlet-nh-mav.f:91-180: the implicit solve in closed form
         // (clmd_nh_root); the force pass leaves W = V + dth a in vn
         const double Q = R.Q, psi1 = R.psi;
         double S = 0.0, p;
-        forces<NT, SM, MIXED, CS, true>(R, C, A, P, false, last, &S);
+        forces<NT, SM, MIXED, CS, H, true>(R, C, A, P, false, last, &S);
         if constexpr (CS == 1) {
           if (!cta_nh_root_commit<NT>(S, psi1, R.nkt3_i, dth, Q, C.red, R, step, p)) goto out;
           committed = true;
         } else {
-          if (!cl_nh_root<NT, CS>(S, psi1, R.nkt3_i, dth, Q, C, S, p)) {
+          if (!cl_nh_root<NT, CS, H>(S, psi1, R.nkt3_i, dth, Q, C, S, p)) {
             if (tid == 0 && R.status == 0) R.status = CLMD_ERR_NH_NOCONVERGE;
             gsync<CS>();
             goto out;
@@ -1598,7 +1623,7 @@ __global__ void __launch_bounds__(NT, MINB) k_ens(Args A) {
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     }
     __syncthreads();
-    if (!R.done && !R.status) run_window<NT, SM, MIXED, 1>(R, C, A);
+    if (!R.done && !R.status) run_window<NT, SM, MIXED, 1, 1>(R, C, A);
     if (threadIdx.x == 0 && R.step > step0) {
       unsigned long long t1;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
@@ -1621,11 +1646,12 @@ __global__ void __launch_bounds__(NT, MINB) k_ens(Args A) {
 // replica record and cell starts and applies the same scalar logic to the
 // same totals; rank 0 alone writes the shared results back.  Each cluster
 // takes replicas from the device counter like the single-CTA kernel.
-template <int NT, bool MIXED, int CS>
+template <int NT, bool MIXED, int CS, int H>
 __global__ void __launch_bounds__(NT, 1) k_ens_cl(Args A) {
   extern __shared__ double dsm[];
   __shared__ Rep R;
   __shared__ Cta C;
+  __shared__ double sub[4 * 32];
   __shared__ int item;
   auto cl = cg::this_cluster();
   const unsigned rank = cl.block_rank();
@@ -1647,6 +1673,7 @@ __global__ void __launch_bounds__(NT, 1) k_ens_cl(Args A) {
       C.cstart = (int*)dsm;
       C.cand = A.cand + R.off;
       C.sx = C.sy = C.sz = nullptr;
+      C.sub = sub;
     }
     unsigned long long t0 = 0;
     const int step0 = R.step;
@@ -1655,7 +1682,7 @@ __global__ void __launch_bounds__(NT, 1) k_ens_cl(Args A) {
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
     }
     cl.sync();
-    if (!R.done && !R.status) run_window<NT, false, MIXED, CS>(R, C, A);
+    if (!R.done && !R.status) run_window<NT, false, MIXED, CS, H>(R, C, A);
     if (rank == 0) {
       if (threadIdx.x == 0 && R.step > step0) {
         unsigned long long t1;
@@ -1707,7 +1734,7 @@ struct clmd_ensemble {
   // size classes: each has its own block size, shared-memory budget, stream.
   // 0-3: one CTA per replica, split by atom count (cls_max); 4-7: replicas
   // whose positions do not fit in shared memory, one thread-block cluster
-  // of 2, 4, 8 or 16 CTAs per replica (kClusterAtoms atoms per CTA or more)
+  // of 2, 4, 8 or 16 CTAs per replica (cluster_class, wider_class)
   static constexpr int kClasses = 8;
   static constexpr int kCtaClasses = 4;
   int cls_max[kCtaClasses] = {2048, 4096, 6144, 1 << 30};  // measured best of a few splits
@@ -1780,13 +1807,18 @@ static bool shape_ok(int shape) {
   }
 }
 
-// the cluster kernel of cs CTAs per replica (1024 threads each)
-static EnsKernel cluster_kernel(int cs, bool mixed) {
+// the cluster kernel of cs CTAs per replica (1024 threads each); two: sums
+// laid out as on 2 cs CTAs
+template <int CS, int H>
+static EnsKernel pick_cl(bool mixed) {
+  return mixed ? k_ens_cl<1024, true, CS, H> : k_ens_cl<1024, false, CS, H>;
+}
+static EnsKernel cluster_kernel(int cs, bool two, bool mixed) {
   switch (cs) {
-    case 2: return mixed ? k_ens_cl<1024, true, 2> : k_ens_cl<1024, false, 2>;
-    case 4: return mixed ? k_ens_cl<1024, true, 4> : k_ens_cl<1024, false, 4>;
-    case 8: return mixed ? k_ens_cl<1024, true, 8> : k_ens_cl<1024, false, 8>;
-    default: return mixed ? k_ens_cl<1024, true, 16> : k_ens_cl<1024, false, 16>;
+    case 2: return two ? pick_cl<2, 2>(mixed) : pick_cl<2, 1>(mixed);
+    case 4: return two ? pick_cl<4, 2>(mixed) : pick_cl<4, 1>(mixed);
+    case 8: return two ? pick_cl<8, 2>(mixed) : pick_cl<8, 1>(mixed);
+    default: return pick_cl<16, 1>(mixed);
   }
 }
 static size_t cluster_smem(int ncmax) {
@@ -1802,7 +1834,7 @@ static int setup_clusters(clmd_ensemble* E) {
   int region = 0;
   for (int c = clmd_ensemble::kCtaClasses; c < clmd_ensemble::kClasses; c++) {
     const int cs = E->cls_cs[c];
-    EnsKernel k = cluster_kernel(cs, mixed);
+    EnsKernel k = cluster_kernel(cs, false, mixed), k2 = cluster_kernel(cs, true, mixed);
     E->cl_max_clusters[c] = 0;
     if (cs > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
                       cudaSuccess) {
@@ -1810,11 +1842,12 @@ static int setup_clusters(clmd_ensemble* E) {
       continue;
     }
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess) {
+            cudaSuccess ||
+        cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess) {
       cudaGetLastError();
       continue;
     }
-    E->attr_smem[(void*)k] = smem;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(cs);
     lc.blockDim = dim3(1024);
@@ -2187,6 +2220,10 @@ static EnsKernel pick(bool sm, bool mixed) {
 // a block shape: threads per CTA, with CLMD_ENS_LEAN for the 64-register
 // variant (128, 256 and 512 threads)
 static int shape_threads(int shape) { return shape & 0xffff; }
+static int shape_ctas_per_sm(int shape) {  // by its registers
+  const int nt = shape_threads(shape);
+  return ((shape & CLMD_ENS_LEAN) || nt == 1024 ? 1024 : 512) / nt;
+}
 static int shape_lanes_log2(int shape) { return (shape >> CLMD_ENS_LANES_SHIFT) & 3; }
 
 static EnsKernel kernel_for(int shape, bool sm, bool mixed) {
@@ -2199,8 +2236,35 @@ static EnsKernel kernel_for(int shape, bool sm, bool mixed) {
   }
 }
 
+// the class of a replica on one CTA
+static int cta_class(const clmd_ensemble* E, int n) {
+  int c = 0;
+  while (c < clmd_ensemble::kCtaClasses - 1 && n > E->cls_max[c]) c++;
+  return c;
+}
+// the cluster class of a replica whose positions do not fit in shared
+// memory: about 6,144 atoms or more per CTA, the cluster size a power of two
+// in [2, 16], the largest usable one not above it (-1: none usable)
+constexpr int kClusterAtoms = 6144;
+static int cluster_class(const clmd_ensemble* E, int n) {
+  int want = 2;
+  while (want < 16 && want * kClusterAtoms < n) want *= 2;
+  for (int c = clmd_ensemble::kClasses - 1; c >= clmd_ensemble::kCtaClasses; c--)
+    if (E->cls_cs[c] <= want && E->cl_max_clusters[c] > 0) return c;
+  return -1;
+}
+// the class of twice as many CTAs, where there is one: the replicas of class
+// c may run there instead, and their sums are laid out for it on either
+static int wider_class(const clmd_ensemble* E, int c) {
+  const int w = c + 1;
+  return w < clmd_ensemble::kClasses && E->cls_cs[w] == 2 * E->cls_cs[c] &&
+                 E->cl_max_clusters[w] > 0
+             ? w
+             : c;
+}
+
 static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const int* slots,
-                         int shape, ClassLaunch& L) {
+                         int shape, bool wide, ClassLaunch& L) {
   L = ClassLaunch();
   L.item0 = item0;
   L.nitems = nitems;
@@ -2214,7 +2278,7 @@ static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const i
     // starts (kNcMax^3 at most) in each CTA's shared memory
     L.cs = E->cls_cs[c];
     L.nt = 1024;
-    L.k = cluster_kernel(L.cs, mixed);
+    L.k = cluster_kernel(L.cs, !wide && wider_class(E, c) != c, mixed);
     int ncmax = 1;
     for (int k = 0; k < nitems; k++) ncmax = std::max(ncmax, E->h_reps[slots[k]].ncmax);
     L.smem = cluster_smem(ncmax);
@@ -2304,39 +2368,44 @@ static int enqueue_class(clmd_ensemble* E, int c, const ClassLaunch& L, int nwin
 // that every CTA stays busy about min_ms whatever its replica's size (a
 // replica not yet timed runs a few steps)
 // only >= 0: that size class alone (the autotuner's trials)
-// the cluster class of a replica whose positions do not fit in shared
-// memory: about `per` atoms or more per CTA, the cluster size a power of two
-// in [2, 16], the largest usable one not above it (-1: none usable).  Large
-// pools: 6144 (300 replicas of 9,000-50,000 atoms 6.92e9 atom-steps/s, 6.66e9
-// with 3072, 5.50e9 with 1536).  A pool of at most 2304 atoms per SM cannot
-// fill the GPU at that: 3072 (9 such replicas 7.55 -> 4.74 ms per 100 steps,
-// 12: 6.82 -> 4.82, 14: 7.70 -> 7.04; beyond, 16: 8.36 -> 8.12, but 19:
-// 7.82 -> 8.75).  The pool's size, not its present load, decides: a replica's
-// sums keep their shape whatever shares the launch
-constexpr int kClusterAtoms = 6144, kClusterAtomsSmallPool = 3072, kSmallPoolPerSm = 2304;
-static int cluster_class(const clmd_ensemble* E, int n) {
-  const int per = E->A.pool <= (long long)kSmallPoolPerSm * E->nsm ? kClusterAtomsSmallPool
-                                                                     : kClusterAtoms;
-  int want = 2;
-  while (want < 16 && want * per < n) want *= 2;
-  for (int c = clmd_ensemble::kClasses - 1; c >= clmd_ensemble::kCtaClasses; c--)
-    if (E->cls_cs[c] <= want && E->cl_max_clusters[c] > 0) return c;
-  return -1;
-}
-
 static int launch_all(clmd_ensemble* E, int nwin, const int* threads, float min_ms = 0.0f,
                       int only = -1) {
   std::vector<int> cls[clmd_ensemble::kClasses];
   int nmax[clmd_ensemble::kClasses] = {};
-  for (int s = 0; s < E->cfg.max_replicas; s++)
-    if (E->used[s] && !E->h_summary[s].x && !E->h_summary[s].y) {
-      const int n = E->h_reps[s].natom;
-      int c = -1;
-      if (E->use_clusters && E->h_reps[s].reorder == 1) c = cluster_class(E, n);
-      if (c < 0) {
-        c = 0;
-        while (c < clmd_ensemble::kCtaClasses - 1 && n > E->cls_max[c]) c++;
+  auto running = [&](int s) { return E->used[s] && !E->h_summary[s].x && !E->h_summary[s].y; };
+  auto cluster_of = [&](int s) {
+    return E->use_clusters && E->h_reps[s].reorder == 1 ? cluster_class(E, E->h_reps[s].natom)
+                                                        : -1;
+  };
+  // Replicas on clusters take the wider ones (~3,072 atoms per CTA) if all
+  // running replicas then fit on the GPU at once: a cluster takes the place of
+  // two of half its size, of which the GPU holds cl_max_clusters, and the CTAs
+  // the SMs.  ms per 100 steps, ~6,144 and ~3,072 atoms per CTA: 9 replicas of
+  // 9,000-50,000 atoms 6.9 and 4.2, 12 6.9 and 4.3, 30 of 9,500 5.6 and 3.8;
+  // and where they do not fit: 16 of 14,000 4.8 and 6.0, 9 of 25,000 4.6 and
+  // 6.3, 24 of 9,000-50,000 7.3 and 10.6, 300 87 and 98.
+  bool wide = true;
+  {
+    long long n[clmd_ensemble::kClasses] = {}, held = 0;
+    double sms = 0.0;
+    for (int s = 0; s < E->cfg.max_replicas; s++)
+      if (running(s)) {
+        int c = cluster_of(s);
+        c = c < 0 ? cta_class(E, E->h_reps[s].natom) : wider_class(E, c);
+        n[c]++;
+        sms += (double)E->cls_cs[c] / shape_ctas_per_sm(threads[c]);
       }
+    for (int c = clmd_ensemble::kClasses - 1; c >= clmd_ensemble::kCtaClasses; c--) {
+      held = 2 * held + n[c];
+      if (held > E->cl_max_clusters[c]) wide = false;
+    }
+    if (sms > E->nsm) wide = false;
+  }
+  for (int s = 0; s < E->cfg.max_replicas; s++)
+    if (running(s)) {
+      const int n = E->h_reps[s].natom;
+      int c = cluster_of(s);
+      c = c < 0 ? cta_class(E, n) : wide ? wider_class(E, c) : c;
       if (only >= 0 && c != only) continue;
       cls[c].push_back(s);
       nmax[c] = std::max(nmax[c], n);
@@ -2387,7 +2456,8 @@ static int launch_all(clmd_ensemble* E, int nwin, const int* threads, float min_
     int off = 0;
     for (int c = 0; c < clmd_ensemble::kClasses; c++) {
       for (int s : cls[c]) E->last_atoms[c] += E->h_reps[s].natom;
-      int st = prepare_class(E, c, off, (int)cls[c].size(), cls[c].data(), threads[c], L[c]);
+      int st = prepare_class(E, c, off, (int)cls[c].size(), cls[c].data(), threads[c], wide,
+                             L[c]);
       if (st) return st;
       off += (int)cls[c].size();
     }

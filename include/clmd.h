@@ -276,9 +276,10 @@ int clmd_ens_add(clmd_ensemble* e, const clmd_replica_spec* spec, const double* 
  * persistent launch per size class, the classes concurrently); replicas stop
  * when done.  A replica runs on one CTA, or -- when its positions do not fit
  * in one SM's shared memory (about 9,000 atoms and more) -- on a
- * thread-block cluster of 2, 4, 8 or 16 CTAs (about 6,144 atoms per CTA or
- * more; 3,072 in a pool of at most 2,304 atoms per SM) that splits its atoms
- * and meets at cluster barriers
+ * thread-block cluster of 2, 4, 8 or 16 CTAs that splits its atoms and meets
+ * at cluster barriers: about 3,072 atoms per CTA while all running replicas
+ * fit on the GPU at once, else about 6,144 (its results are the same bits on
+ * either, whatever the pool)
  * (CLMD_ENS_CLUSTERS=0 in the environment at creation: one CTA each).  The
  * launch sequence is captured once into a CUDA graph and replayed while the
  * set of running replicas and the launch shapes stay the same

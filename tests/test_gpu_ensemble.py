@@ -700,3 +700,36 @@ def test_ensembles_side_by_side(gpu):
         for e in es:
             e.step(1)
     assert [e.results()[0].step for e in es] == [10, 10, 10]
+
+
+@pytest.mark.parametrize("precision", [clmd.PREC_MIXED, clmd.PREC_FP64])
+@pytest.mark.parametrize("n", [9400, 14000, 30000, 52000])
+def test_cluster_replica_in_any_pool(gpu, precision, n):
+    """A cluster replica's bits depend on itself alone: in a pool of its own
+    size, in a large pool, beside enough others that the launch gives it a
+    smaller cluster, and when that changes between its windows."""
+    box, arrs = replica_inputs(n, 0.03, 0.7, 900 + n)
+    others = [(12500, replica_inputs(12500, 0.03, 0.75, 9))] * 30
+
+    def run(pool, before, between):
+        e = clmd.Ensemble(clmd.ens_config(pool, 40, ftcsi=20, precision=precision))
+        for m, (b2, a2) in others[:before]:
+            assert e.add(m, b2, 0.75, *a2, csover=10**6) is not None
+        s = e.add(n, box, 0.7, *arrs, csover=10**6)
+        e.step(1)
+        for m, (b2, a2) in others[:between]:
+            assert e.add(m, b2, 0.75, *a2, csover=10**6) is not None
+        e.step(2)
+        st, cl = e.state(s)
+        r = e.results()[s]
+        e.close()
+        assert r.status == 0 and r.step == 60
+        return st, cl, r
+
+    a, ca, ra = run(n, 0, 0)
+    for pool, before, between in ((n + 400000, 0, 0), (n + 400000, 30, 0), (n + 400000, 0, 30)):
+        b, cb, rb = run(pool, before, between)
+        for k in ("x", "y", "z", "vx", "vy", "vz", "ax", "ay", "az"):
+            assert np.array_equal(getattr(a, k), getattr(b, k)), (k, pool, before, between)
+        assert np.array_equal(ca, cb)
+        assert (ra.psi, ra.s, ra.ekin, ra.epot) == (rb.psi, rb.s, rb.ekin, rb.epot)
