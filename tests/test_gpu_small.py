@@ -92,3 +92,49 @@ def test_small_mixed_forces(gpu, n):
     oa = np.stack([b.ax, b.ay, b.az])
     assert np.linalg.norm(ga - oa) <= 1e-5 * np.linalg.norm(oa)
     assert g.scalars().status == 0
+
+
+def block_tree(e):
+    """The sum of e over blocks of 256 as a block reduces it: xor butterflies
+    over 32 lanes, over a block's 8 warps, then over the blocks."""
+    def butterfly(v):
+        for o in (16, 8, 4, 2, 1):
+            v = v + v[..., np.arange(32) ^ o]
+        return v[..., 0]
+    nb = -(-len(e) // 256)
+    v = np.zeros(256 * nb)
+    v[:len(e)] = e
+    warps = np.zeros((nb, 32))
+    warps[:, :8] = butterfly(v.reshape(nb, 8, 32))
+    blocks = np.zeros(32)
+    blocks[:nb] = butterfly(warps)
+    return butterfly(blocks)
+
+
+@pytest.mark.parametrize("n", [3, 33, 256, 257, 2011, 5000, 8191, 8192])
+@pytest.mark.parametrize("two", [False, True])
+def test_velocity_scaling_bits(gpu, n, two):
+    """Velocity scaling of small systems (one launch): the factor of each
+    species, and with it every velocity, to the last bit of the tree of sums
+    that larger systems use (all atoms in input order, no list yet)."""
+    n2 = n // 3 if two else 0
+    cfg = clmd.lj_config(n, 0.02, 0.8, species=dict(n=n2, mass=1.7) if two else None)
+    cfg.apth = b"XX" + b"-" * (clmd.MXSORTS - 2)
+    rng = np.random.default_rng(n)
+    st = random_state(cfg, n) if n > 3 else clmd.State(*rng.uniform(0, cfg.boxx, (3, n)),
+                                                       *rng.normal(size=(3, n)),
+                                                       *np.zeros((3, n)))
+    api = np.r_[np.full(n - n2, 1), np.full(n2, 2)].astype(np.int32) if two else None
+    g = clmd.System(cfg)
+    g.set_state(st, api=api, scalars=clmd.scalars_init(cfg))
+    v = np.stack([st.vx, st.vy, st.vz])
+    sp = np.r_[np.zeros(n - n2, int), np.ones(n2, int)]
+    mass = np.array([1.0, 1.7])
+    e = 0.5 * mass[sp] * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2])
+    g.thermostat(1)
+    out = g.get_state()
+    for s in range(2 if two else 1):
+        m = sp == s
+        kf = np.sqrt(1.5 * clmd.CIKB * cfg.att * m.sum() / block_tree(np.where(m, e, 0.0)))
+        for got, was in zip((out.vx, out.vy, out.vz), v):
+            assert np.array_equal(got[m], was[m] * kf), s
