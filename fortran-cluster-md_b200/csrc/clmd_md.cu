@@ -221,70 +221,59 @@ __global__ void k_thermo_scale(Params P, DevState* st, const int* perm, double* 
 }
 
 // the same in one launch, one block, for systems of a few thousand atoms: two
-// launches cost more there than the block's passes over the velocities
-// (thermostat() at N = 2,011: 30 -> 20 us).  The sums are the two launches',
-// tree for tree (a warp's 32 atoms, 8 warps of a block of 256, the blocks),
-// so the factors are the same bits.
+// launches cost more there than the block's passes over the velocities.  The
+// sums are the two launches', tree for tree (a warp's 32 atoms, the 8 warps of
+// a block of 256, the blocks), so the factors are the same bits.
 constexpr int kThermoOne = 8192;
 __global__ void __launch_bounds__(1024) k_thermo_one(Params P, DevState* st, const int* perm,
                                                      double* vx, double* vy, double* vz,
                                                      int step) {
   if (gated(st)) return;
-  constexpr int K = kThermoOne / 1024;
-  static_assert(kThermoOne <= 32 * kBlock && kBlock == 256, "one warp per block of the tree");
-  __shared__ double warps[kThermoOne / 32], blocks[32], eks[CLMD_MXSORTS], kfs[CLMD_MXSORTS];
+  static_assert(kThermoOne <= 32 * kBlock && kBlock == 256, "one lane per block of the tree");
+  __shared__ double warps[32 * 9], kfs[CLMD_MXSORTS];  // (a block's 8 warps, 9 apart)
   __shared__ int scs[CLMD_MXSORTS];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  double e[K];
-  int sp[K];
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    const int i = 1024 * k + tid;
-    sp[k] = -1;
-    e[k] = 0.0;
-    if (i < P.N) {
-      sp[k] = species_block(P, perm[i]);
-      if (sp[k] >= 0)
-        e[k] = 0.5 * P.apmas[sp[k]] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
-    }
-  }
+  const int tid = threadIdx.x, lane = tid & 31;
+  double ekin = 0.0;
   for (int s = 0; s < P.atsorts; s++) {
+    for (int i0 = 0; i0 < P.N; i0 += 2048) {
+      double e[2];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      if (1024 * k >= P.N) break;
-      const double t = warp_sum(sp[k] == s ? e[k] : 0.0);
-      if (lane == 0) warps[32 * k + w] = t;
+      for (int k = 0; k < 2; k++) {  // (both rounds' loads in flight)
+        const int j = min(i0 + 1024 * k + tid, P.N - 1);
+        const double x = vx[j], y = vy[j], z = vz[j];
+        e[k] = 0.5 * P.apmas[s] * (x * x + y * y + z * z);
+      }
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int i = i0 + 1024 * k + tid;
+        const bool in = i < P.N && (P.atsorts == 1 || species_block(P, perm[i]) == s);
+        e[k] = warp_sum(in ? e[k] : 0.0);
+        if (lane == 0) warps[9 * (i >> 8) + ((i >> 5) & 7)] = e[k];
+      }
     }
     __syncthreads();
-    const int c = 8 * w + lane;
-    const double t = warp_sum(lane < 8 && 32 * c < P.N ? warps[c] : 0.0);
-    if (lane == 0) blocks[w] = t;
+    if (tid < 32) {
+      const double* t = warps + 9 * lane;
+      double ek = 0.0;
+      if (kBlock * lane < P.N)
+        ek = ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
+      ek = warp_sum(ek);
+      if (lane == 0) {
+        ekin = ekin + ek;
+        kfs[s] = sqrt(P.ekinT[s] / ek);
+        scs[s] = (P.apth[s] == 'X' || step == -1);
+        if (scs[s]) ekin = ekin - ek + P.ekinT[s];
+      }
+    }
     __syncthreads();
-    if (w == 0) {
-      const double ek = warp_sum(kBlock * lane < P.N ? blocks[lane] : 0.0);
-      if (lane == 0) eks[s] = ek;
-    }
   }
-  if (tid == 0) {
-    double ekin = 0.0;
-    for (int s = 0; s < P.atsorts; s++) {
-      const double ek = eks[s];
-      ekin = ekin + ek;
-      kfs[s] = sqrt(P.ekinT[s] / ek);
-      scs[s] = (P.apth[s] == 'X' || step == -1);
-      if (scs[s]) ekin = ekin - ek + P.ekinT[s];
-    }
-    st->s.ekin = ekin;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; k++) {
-    const int i = 1024 * k + tid;
-    if (sp[k] < 0 || !scs[sp[k]]) continue;
-    const double kf = kfs[sp[k]];
-    vx[i] = vx[i] * kf;
-    vy[i] = vy[i] * kf;
-    vz[i] = vz[i] * kf;
+  if (tid == 0) st->s.ekin = ekin;
+  for (int i = tid; i < P.N; i += 1024) {
+    const int sp = P.atsorts == 1 ? 0 : species_block(P, perm[i]);
+    if (sp < 0 || !scs[sp]) continue;
+    vx[i] = vx[i] * kfs[sp];
+    vy[i] = vy[i] * kfs[sp];
+    vz[i] = vz[i] * kfs[sp];
   }
 }
 
