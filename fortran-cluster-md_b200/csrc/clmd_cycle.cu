@@ -317,6 +317,49 @@ static __device__ bool rebuild(const Params& P, DevState* st, Blk& B, const Cycl
 enum { SLOT_MAX = 0, SLOT_SUMV2 = 1, SLOT_EPOT = 2, SLOT_VIR = 3, SLOT_EKIN = 4,
        SLOT_WV = 5, SLOT_VV = 4, SLOT_EK0 = 6 /* ek per species: 6..15 */ };
 
+// Nose-Hoover by the reference's own sweeps where the closed form does not
+// stand for them (clmd_nh_closed): the two further sums, then the number of
+// sweeps.  red0, red1: the partial buffers, the next one first.
+struct Swept {
+  int n;     // sweeps; kNhSweeps + 1: no convergence; 0: a barrier timed out
+  double p;  // the new PSI
+};
+static __device__ __noinline__ Swept nh_sweep(DevState* st, int N, const double* vx,
+                                              const double* vy, const double* vz,
+                                              const double* ax, const double* ay,
+                                              const double* az, double dt, double m, double nkt3,
+                                              double Q, double sww, double psi, double* red0,
+                                              double* red1, double* sh, double* bc) {
+  const int G = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const double dth = dt / 2;
+  double wv = 0.0, vv = 0.0, swv = 0.0, svv = 0.0;
+  int need = 1;
+  for (int pass = 0; pass < 2; pass++) {
+    for (int p = t0; p < N; p += G) {
+      const double V[3] = {vx[p], vy[p], vz[p]};
+      const double W[3] = {V[0] + dth * ax[p], V[1] + dth * ay[p], V[2] + dth * az[p]};
+      if (pass == 0) {
+        wv = wv + W[0] * V[0] + W[1] * V[1] + W[2] * V[2];
+        vv = vv + V[0] * V[0] + V[1] * V[1] + V[2] * V[2];
+      } else {
+        need = max(need, clmd_nh_sweeps(W, V, sww, swv, svv, psi, m, nkt3, dt, Q));
+      }
+    }
+    if (pass == 0) {
+      put_sum(red0, SLOT_WV, wv, sh);
+      put_sum(red0, SLOT_VV, vv, sh);
+      if (!gbar(st)) return {0, 0.0};
+      swv = get_sum(red0, SLOT_WV, sh, bc);
+      svv = get_sum(red0, SLOT_VV, sh, bc);
+    } else {
+      put_max(red1, SLOT_MAX, (double)need, sh);
+      if (!gbar(st)) return {0, 0.0};
+      need = (int)get_max(red1, SLOT_MAX, sh, bc);
+    }
+  }
+  return {need, clmd_nh_swept(need, sww, swv, svv, psi, m, nkt3, dt, Q)};
+}
+
 template <bool NH, bool THERMO, bool MIXED>
 __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevState* st,
                                                                 CycleArgs A, int nsteps,
@@ -610,10 +653,24 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
         rb ^= 1;
         // every block solves the same scalar equation from the same sums
         double pn;
-        if (!clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn)) {
+        bool ok = clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn);
+        int iters = 1;
+        if (!MIXED && !clmd_nh_closed(ok, psi, dth)) {
+          double* const r0 = red();
+          rb ^= 1;
+          const Swept w = nh_sweep(st, N, A.vx, A.vy, A.vz, A.ax, A.ay, A.az, dt, m, P.nkt3_i, Q,
+                                   sumv2, psi, r0, red(), sh, B.bcast);
+          rb ^= 1;
+          if (w.n == 0) goto timeout;
+          iters = w.n;
+          pn = w.p;
+          ok = iters <= kNhSweeps;
+        }
+        if (!ok) {
           if (threadIdx.x == 0 && B.q.status == 0) {
             B.q.status = CLMD_ERR_NH_NOCONVERGE;
             B.q.fail_step = step;
+            if (!MIXED) B.q.nh_iters = min(iters, kNhSweeps);
           }
           __syncthreads();
           goto done;
@@ -662,7 +719,7 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
           A.vz[p] = vzi;
         }
         if (threadIdx.x == 0) {
-          B.q.nh_iters = 1;
+          B.q.nh_iters = iters;
           B.q.sumv2 = sumv2 * c * c;
           B.q.psi = pn;
           B.q.ekin = 0.5 * m * B.q.sumv2;
@@ -681,7 +738,7 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
           put_max(red(), SLOT_MAX, (double)sweeps, sh);
           if (!gbar(st)) goto timeout;
           const double n = get_max(red(), SLOT_MAX, sh, B.bcast);
-          if (threadIdx.x == 0) B.q.nh_iters = (int)n;
+          if (threadIdx.x == 0) B.q.nh_iters = min((int)n, kNhSweeps);
           rb ^= 1;
         }
       }

@@ -178,7 +178,7 @@ __device__ __forceinline__ void cta_sum2(double& a, double& b, int& f, double* s
 // step's end is folded in (one CTA per replica): lane 0 of warp 0 also records the replica's new PSI, sum v^2, ekin, step and pair
 // terms (or the solve's failure) before the barrier that publishes the root,
 // so the step needs no barrier of its own to publish them
-template <int NT>
+template <int NT, bool MIXED>
 __device__ __forceinline__ bool cta_nh_root_commit(double S, double psi1, double nkt3,
                                                    double dth, double Q, double* sh, Rep& R,
                                                    int step, double& p) {
@@ -190,7 +190,8 @@ __device__ __forceinline__ bool cta_nh_root_commit(double S, double psi1, double
   if (w == 0) {
     const double t = wsum(lane < W ? sh[lane] : 0.0);
     double pr;
-    const bool ok = clmd_nh_root(t, psi1, nkt3, dth, Q, pr);
+    bool ok = clmd_nh_root(t, psi1, nkt3, dth, Q, pr);
+    if (!MIXED) ok = clmd_nh_closed(ok, psi1, dth);
     if (lane == 0) {
       // slots 100, 101: past every slot a reduction of the next step writes
       // (up to 3 * 32), since no barrier separates these reads from them
@@ -203,7 +204,7 @@ __device__ __forceinline__ bool cta_nh_root_commit(double S, double psi1, double
         R.ekin = 0.5 * R.sumv2;
         R.step = step + 1;
         R.pterms += R.nfull;
-      } else if (R.status == 0) {
+      } else if (MIXED && R.status == 0) {
         R.status = CLMD_ERR_NH_NOCONVERGE;
       }
     }
@@ -1147,6 +1148,56 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
   if constexpr (!(NHF && CS == 1)) gsync<CS>();
 }
 
+// A step's Nose-Hoover velocities and end by the reference's own sweeps (FP64,
+// where the closed form does not stand for them: clmd_nh_closed): W is in w,
+// V in v, which gets the velocities.  False: no convergence.
+template <int NT, int CS, int H>
+__device__ __noinline__ bool nh_sweep(Rep& R, Cta& C, double dt, const double* wx,
+                                      const double* wy, const double* wz, double* vx, double* vy,
+                                      double* vz) {
+  const int N = R.natom, gt = gtid<NT, CS>();
+  constexpr int GT = NT * CS;
+  const double psi1 = R.psi, nkt3 = R.nkt3_i, Q = R.Q;
+  double s[3] = {0.0, 0.0, 0.0};
+  for (int h = 0; h < H; h++) {
+    if (h > 0)
+      for (int k = 0; k < 3; k++) half_out(s[k], k, C);
+    for (int i = gt + h * GT; i < N; i += H * GT) {
+      s[0] += wx[i] * wx[i] + wy[i] * wy[i] + wz[i] * wz[i];
+      s[1] += wx[i] * vx[i] + wy[i] * vy[i] + wz[i] * vz[i];
+      s[2] += vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i];
+    }
+  }
+  for (int k = 0; k < 3; k++) s[k] = grp_sum<NT, CS, H>(s[k], C, k);
+  int need = 1;
+  for (int i = gt; i < N; i += GT) {
+    const double W[3] = {wx[i], wy[i], wz[i]}, V[3] = {vx[i], vy[i], vz[i]};
+    need = max(need, clmd_nh_sweeps(W, V, s[0], s[1], s[2], psi1, 1.0, nkt3, dt, Q));
+  }
+  need = (int)grp_max<NT, CS>((double)need, C);
+  const bool ok = need <= kNhSweeps;
+  if (ok) {
+    const double p = clmd_nh_swept(need, s[0], s[1], s[2], psi1, 1.0, nkt3, dt, Q);
+    const double c = 1.0 / (1.0 + dt / 2 * p);
+    for (int i = gt; i < N; i += GT) {
+      vx[i] = wx[i] * c;
+      vy[i] = wy[i] * c;
+      vz[i] = wz[i] * c;
+    }
+    if (threadIdx.x == 0) {
+      R.sumv2 = s[0] * c * c;
+      R.psi = p;
+      R.ekin = 0.5 * R.sumv2;
+      R.step = R.step + 1;
+      R.pterms += R.nfull;
+    }
+  } else if (threadIdx.x == 0 && R.status == 0) {
+    R.status = CLMD_ERR_NH_NOCONVERGE;
+  }
+  gsync<CS>();
+  return ok;
+}
+
 template <bool MIXED>
 __device__ __forceinline__ void get_a(const Args& A, int k, double& ax, double& ay, double& az) {
   if (MIXED) {
@@ -1348,8 +1399,10 @@ __device__ void host_io(const Rep& R, const Cta& C, const Args& A, bool in) {
   gsync<CS>();
 }
 
+// True: the step's velocities are still to come from nh_sweep (then C.nsteps
+// steps are left)
 template <int NT, bool SM, bool MIXED, int CS, int H>
-__device__ void run_window(Rep& R, Cta& C, const Args& A) {
+__device__ bool run_steps(Rep& R, Cta& C, const Args& A) {
   const int tid = threadIdx.x;
   const int gt = gtid<NT, CS>();
   constexpr int GT = NT * CS;
@@ -1359,7 +1412,7 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
   Pos<SM> P{A, C, off};
   bool vin_n = false;  // uniform: the current velocities are in vxn, not vx
   double vsc = 1.0;    // then the velocities are vn * vsc (clmd_nh_root)
-  if (A.hx) host_io<NT, CS>(R, C, A, true);
+  bool sweep = false;
   for (int i = gt; i < N; i += GT) P.set(i, A.x[off + i], A.y[off + i], A.z[off + i]);
   gsync<CS>();
   // the grid of the current list
@@ -1517,21 +1570,29 @@ __device__ void run_window(Rep& R, Cta& C, const Args& A) {
         const double Q = R.Q, psi1 = R.psi;
         double S = 0.0, p;
         forces<NT, SM, MIXED, CS, H, true>(R, C, A, P, false, last, &S);
+        bool ok;
         if constexpr (CS == 1) {
-          if (!cta_nh_root_commit<NT>(S, psi1, R.nkt3_i, dth, Q, C.red, R, step, p)) goto out;
+          ok = cta_nh_root_commit<NT, MIXED>(S, psi1, R.nkt3_i, dth, Q, C.red, R, step, p);
           committed = true;
         } else {
-          if (!cl_nh_root<NT, CS, H>(S, psi1, R.nkt3_i, dth, Q, C, S, p)) {
-            if (tid == 0 && R.status == 0) R.status = CLMD_ERR_NH_NOCONVERGE;
-            gsync<CS>();
-            goto out;
-          }
+          ok = cl_nh_root<NT, CS, H>(S, psi1, R.nkt3_i, dth, Q, C, S, p);
+          if (!MIXED) ok = clmd_nh_closed(ok, psi1, dth);
           if (tid == 0) {
-            const double c = 1.0 / (1.0 + dth * p);
-            R.sumv2 = S * c * c;
-            R.psi = p;
-            R.ekin = 0.5 * R.sumv2;
+            if (ok) {
+              const double c = 1.0 / (1.0 + dth * p);
+              R.sumv2 = S * c * c;
+              R.psi = p;
+              R.ekin = 0.5 * R.sumv2;
+            } else if (MIXED && R.status == 0) {
+              R.status = CLMD_ERR_NH_NOCONVERGE;
+            }
           }
+        }
+        if (!ok) {
+          sweep = !MIXED;
+          if (sweep && tid == 0) C.nsteps = todo - 1;
+          gsync<CS>();
+          goto out;
         }
         vsc = 1.0 / (1.0 + dth * p);
         vin_n = true;
@@ -1575,6 +1636,17 @@ out:
   }
   for (int i = gt; i < N; i += GT) P.get(i, A.x[off + i], A.y[off + i], A.z[off + i]);
   gsync<CS>();
+  return sweep;
+}
+
+template <int NT, bool SM, bool MIXED, int CS, int H>
+__device__ __forceinline__ void run_window(Rep& R, Cta& C, const Args& A) {
+  const long long off = R.off;
+  if (A.hx) host_io<NT, CS>(R, C, A, true);
+  while (run_steps<NT, SM, MIXED, CS, H>(R, C, A) && !MIXED)
+    if (!nh_sweep<NT, CS, H>(R, C, A.dt, A.vxn + off, A.vyn + off, A.vzn + off, A.vx + off,
+                             A.vy + off, A.vz + off))
+      break;
   if (A.hx) host_io<NT, CS>(R, C, A, false);
 }
 

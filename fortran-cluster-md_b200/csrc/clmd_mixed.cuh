@@ -27,7 +27,8 @@ __device__ __forceinline__ float clmd_rcp_f32(float x) {
 // step limit is 1e-13 of the terms' scale (|p| + |psi1| + (S + 3NkT) dth/Q;
 // rounding noise in f is a few 1e-16 of it, so a tighter limit can stall).
 // False (no convergence) if the root is not finite or the iteration does not
-// settle, as the reference's STOP.
+// settle: mixed precision then stops, as the reference's STOP; FP64 takes the
+// sweeps (clmd_nh_closed).
 __device__ __forceinline__ bool clmd_nh_root(double S, double psi1, double nkt3, double dth,
                                              double Q, double& p) {
   const double k0 = dth / Q;
@@ -44,34 +45,63 @@ __device__ __forceinline__ bool clmd_nh_root(double S, double psi1, double nkt3,
   return false;
 }
 
-// How many of the reference's sweeps (int-verlet-nh-mav.f:105-147) one atom
-// needs until the relative change of each of its velocity components stays
-// within 1e-10.  The sweeps' iterates are vn_k = al W + be V with factors
-// common to all atoms, so the scalars of every sweep follow from three sums
-// (sum W.W, W.V, V.V) without a pass over the atoms.
-__device__ __forceinline__ int clmd_nh_sweeps(const double* W, const double* V, double sww,
-                                              double swv, double svv, double psi1, double m,
-                                              double nkt3, double dt, double Q) {
-  const double dth = dt / 2, dt2 = dt * dt / 2;
-  double al = 0.0, be = 1.0, p = psi1;
-  int need = 1;
-  for (int k = 1; k <= 16; k++) {
+// The reference's sweeps (int-verlet-nh-mav.f:105-147) on scalars alone: their
+// iterates are vn_k = al W + be V with factors common to all atoms, so every
+// sweep follows from three sums (sum W.W, W.V, V.V).
+struct ClmdSweep {
+  double al = 0.0, be = 1.0, p;
+  __device__ __forceinline__ explicit ClmdSweep(double psi1) : p(psi1) {}
+  __device__ __forceinline__ void next(double sww, double swv, double svv, double psi1, double m,
+                                       double nkt3, double dt, double Q) {
+    const double dth = dt / 2, dt2 = dt * dt / 2;
     const double sumv2 = al * al * sww + 2.0 * al * be * swv + be * be * svv;
     const double up = 1.0 + dth * p;
     const double draw = (up * sumv2 - (al * sww + be * swv)) * m * dt / Q;
     double delps = draw + up * ((-m * sumv2 + nkt3) * dth / Q - (psi1 - p));
     delps = delps / (-dt2 * m * sumv2 / Q - up);
     const double a1 = (1.0 - dth * delps * al) / up, b1 = -dth * delps * be / up;
-    bool moved = false;
-    for (int d = 0; d < 3; d++) {
-      const double nx = a1 * W[d] + b1 * V[d], vo = al * W[d] + be * V[d];
-      moved |= fabs(nx - vo) > 1e-10 * fabs(nx);
-    }
-    if (moved) need = k + 1;
     al = a1;
     be = b1;
     p += delps;
+  }
+};
+
+constexpr int kNhSweeps = 1000;  // the reference's limit; more: it stops
+
+// How many sweeps one atom needs until the relative change of each of its
+// velocity components stays within 1e-10; kNhSweeps + 1 if it never does.
+__device__ __forceinline__ int clmd_nh_sweeps(const double* W, const double* V, double sww,
+                                              double swv, double svv, double psi1, double m,
+                                              double nkt3, double dt, double Q) {
+  ClmdSweep s(psi1);
+  int need = 1;
+  for (int k = 1; k <= kNhSweeps; k++) {
+    const double al = s.al, be = s.be;
+    s.next(sww, swv, svv, psi1, m, nkt3, dt, Q);
+    bool moved = false;
+    for (int d = 0; d < 3; d++) {
+      const double nx = s.al * W[d] + s.be * V[d], vo = al * W[d] + be * V[d];
+      moved |= fabs(nx - vo) > 1e-10 * fabs(nx);
+    }
+    if (moved) need = k + 1;
     if (!moved && k > 1) break;
   }
   return need;
+}
+
+// PSI after n sweeps
+static __device__ __noinline__ double clmd_nh_swept(int n, double sww, double swv, double svv,
+                                                    double psi1, double m, double nkt3,
+                                                    double dt, double Q) {
+  ClmdSweep s(psi1);
+  for (int k = 0; k < n; k++) s.next(sww, swv, svv, psi1, m, nkt3, dt, Q);
+  return s.p;
+}
+
+// Whether the closed form stands for the sweeps (FP64): a root was found from
+// a PSI with 1 + dth PSI > 0.  Otherwise (a thermostat mass so small, or a PSI
+// so negative, that a step turns velocities round; a NaN) the kernels take
+// the sweeps themselves.
+__device__ __forceinline__ bool clmd_nh_closed(bool root, double psi1, double dth) {
+  return root && 1.0 + dth * psi1 > 0.0;
 }

@@ -243,6 +243,32 @@ static __device__ bool s_rebuild(const Params& P, DevState* st, SmallShared& S, 
 
 enum { SS_MAX = 0, SS_SUMV2, SS_EPOT, SS_VIR, SS_EKIN, SS_WV, SS_VV };
 
+// Nose-Hoover by the reference's own sweeps where the closed form does not
+// stand for them (clmd_nh_closed).  Two phases: G's parity stays as it is.
+struct Swept {
+  int n;     // sweeps; kNhSweeps + 1: no convergence
+  double p;  // the new PSI
+};
+static __device__ __noinline__ Swept s_sweep(Grp G, bool act, double wx, double wy, double wz,
+                                             double vx, double vy, double vz, double sww,
+                                             double psi, double m, double nkt3, double dt,
+                                             double Q) {
+  G.put_sum(SS_WV, wx * vx + wy * vy + wz * vz);
+  G.put_sum(SS_VV, vx * vx + vy * vy + vz * vz);
+  G.barrier();
+  const double swv = G.get_sum(SS_WV), svv = G.get_sum(SS_VV);
+  G.rb ^= 1;
+  int n = 1;
+  if (act) {
+    const double W[3] = {wx, wy, wz}, V[3] = {vx, vy, vz};
+    n = clmd_nh_sweeps(W, V, sww, swv, svv, psi, m, nkt3, dt, Q);
+  }
+  G.put_max(SS_MAX, (double)n);
+  G.barrier();
+  n = (int)G.get_max(SS_MAX);
+  return {n, clmd_nh_swept(n, sww, swv, svv, psi, m, nkt3, dt, Q)};
+}
+
 template <bool NH, bool THERMO, bool MIXED>
 __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, CycleArgs A, int nsteps,
                                                    int mode, int first, int set, int per) {
@@ -474,23 +500,31 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
       const double svv = !MIXED && last ? G.get_sum(SS_VV) : 0.0;
       G.rb ^= 1;
       double pn;  // every thread takes the same root of the same sum
-      if (!clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn)) {
-        if (tid == 0 && B.q.status == 0) {
-          B.q.status = CLMD_ERR_NH_NOCONVERGE;
-          B.q.fail_step = step;
-        }
-        goto done;
-      }
       int sweeps = 1;
-      if (!MIXED && last) {
+      bool ok = clmd_nh_root(m * sumv2, psi, P.nkt3_i, dth, Q, pn);
+      if (!MIXED && !clmd_nh_closed(ok, psi, dth)) {
+        const Swept w = s_sweep(G, a.act, wx, wy, wz, a.vx, a.vy, a.vz, sumv2, psi, m, P.nkt3_i,
+                                dt, Q);
+        pn = w.p;
+        sweeps = min(w.n, kNhSweeps);
+        ok = w.n <= kNhSweeps;
+      } else if (!MIXED && last) {
         if (a.act) {
           const double W3[3] = {wx, wy, wz}, V3[3] = {a.vx, a.vy, a.vz};
           sweeps = clmd_nh_sweeps(W3, V3, sumv2, swv, svv, psi, m, P.nkt3_i, dt, Q);
         }
         G.put_max(SS_MAX, (double)sweeps);
         G.barrier();
-        sweeps = (int)G.get_max(SS_MAX);
+        sweeps = min((int)G.get_max(SS_MAX), kNhSweeps);
         G.rb ^= 1;
+      }
+      if (!ok) {
+        if (tid == 0 && B.q.status == 0) {
+          B.q.status = CLMD_ERR_NH_NOCONVERGE;
+          B.q.fail_step = step;
+          if (!MIXED) B.q.nh_iters = sweeps;
+        }
+        goto done;
       }
       const double c = 1.0 / (1.0 + dth * pn);
       a.vx = wx * c;

@@ -117,7 +117,10 @@ typedef struct clmd_scalars {
   int32_t cbiggest, cbiggestf, clookfor, clookforf;
   int32_t status;                /* first error, CLMD_OK if none */
   int32_t fail_step;             /* step at which status was set */
-  int32_t nh_iters;              /* sweeps of the last Nose-Hoover velocity solve */
+  /* sweeps (1..1000) in which int-verlet-nh-mav.f:105-147 settles the last
+   * step's Nose-Hoover velocities, counted for that step from the sums of the
+   * closed-form solve; 1000 if they do not settle.  Mixed precision: 1 */
+  int32_t nh_iters;
   int32_t nrebuild;              /* neighbour-list rebuilds so far */
   int32_t last_rebuild_step;
   int32_t aborted;               /* chk_nucleation negated the step */
