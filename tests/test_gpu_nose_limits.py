@@ -74,6 +74,33 @@ def test_nose_nan(gpu, n):
     assert np.isnan(g.get_state().vx).all()
 
 
+@pytest.mark.parametrize("n", [33, 8193])
+@pytest.mark.parametrize("apart", [0.5, 0.1, 0.02])
+@pytest.mark.parametrize("precision,tol", [(clmd.PREC_FP64, 1e-8), (clmd.PREC_MIXED, 1e-5)])
+def test_nose_overlap(gpu, n, apart, precision, tol):
+    """Two atoms that nearly coincide, their first forces met inside the step:
+    the velocity solve's sum is up to 1e50 times the thermal one.  (Mixed: PSI
+    goes with the 2/3 power of the force, whose FP32 terms hold to 1e-6.)"""
+    cfg = clmd.lj_config(n, 0.04, 0.8, ethst="N", integrator=clmd.INT_NOSE)
+    st = random_state(cfg, 3 + n)
+    st.x[1], st.y[1], st.z[1] = st.x[0] + apart, st.y[0], st.z[0]
+    st.vx[1], st.vy[1], st.vz[1] = st.vx[0], st.vy[0], st.vz[0]
+    o = orc.Oracle(cfg, neighbor_mode=1 if n > 64 else 0)
+    o.set_state(st, scalars=orc.scalars_init(cfg))
+    o.neighbor(0)
+    cfg.precision = precision
+    g = clmd.System(cfg)
+    g.set_state(st, scalars=clmd.scalars_init(cfg))
+    g.neighbor(0)
+    o.integrator(1)
+    g.integrator(1)
+    sg, so = g.scalars(), o.scalars()
+    assert so.status == 0 and sg.status == 0
+    assert abs(sg.psi - so.psi) <= tol * abs(so.psi)
+    a, b = g.get_state(), o.get_state()
+    np.testing.assert_allclose(a.vx, b.vx, rtol=0, atol=10 * tol * np.abs(b.vx).max())
+
+
 @pytest.mark.parametrize("n", [400, 10000])  # one CTA, a cluster
 @pytest.mark.parametrize("limit", ["mass1e-5", "mass1.8e-5", "mass2.2e-5", "nan"])
 def test_nose_limits_ensemble(gpu, n, limit):
