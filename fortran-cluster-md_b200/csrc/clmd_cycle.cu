@@ -156,9 +156,9 @@ static __device__ bool rebuild(const Params& P, DevState* st, Blk& B, const Cycl
   if (t0 == 0) st->list_used = 0ull;
   for (int p = t0; p < N; p += G) {
     const double4 v = wrap_box(P, pos[p]);
-    int cx = min((int)(v.x * g.cfx), g.ncx - 1);
-    int cy = min((int)(v.y * g.cfy), g.ncy - 1);
-    int cz = min((int)(v.z * g.cfz), g.ncz - 1);
+    const int cx = clmd_cell(v.x, g.cfx, g.ncx);
+    const int cy = clmd_cell(v.y, g.cfy, g.ncy);
+    const int cz = clmd_cell(v.z, g.cfz, g.ncz);
     int c = (cz * g.ncy + cy) * g.ncx + cx;
     A.atom_cell[p] = c;
     A.row_lo[p] = atomicAdd(&A.cell_count[c], 1);

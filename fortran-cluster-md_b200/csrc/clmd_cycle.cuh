@@ -437,9 +437,9 @@ __device__ __forceinline__ int row_search(const Params& P, const Geo& g, int p, 
                                           const double4& pa, const double4* pos,
                                           const float4* cf, const int* cs, int2* buf, int* out) {
   const int ncx = g.ncx, ncy = g.ncy, ncz = g.ncz, noy = g.noy, noz = g.noz;
-  const int cx = min((int)(pa.x * g.cfx), ncx - 1);
-  const int cy = min((int)(pa.y * g.cfy), ncy - 1);
-  const int cz = min((int)(pa.z * g.cfz), ncz - 1);
+  const int cx = clmd_cell(pa.x, g.cfx, ncx);
+  const int cy = clmd_cell(pa.y, g.cfy, ncy);
+  const int cz = clmd_cell(pa.z, g.cfz, ncz);
   const float lx = (float)P.boxx, ly = (float)P.boxy, lz = (float)P.boxz;
   const float px = (float)pa.x, py = (float)pa.y, pz = (float)pa.z;
   const float flo = g.flo, fhi = g.fhi;

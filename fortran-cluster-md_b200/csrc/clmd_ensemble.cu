@@ -629,13 +629,8 @@ __device__ __forceinline__ int search_row(const Cta& C, const Args& A, const Pos
   const unsigned ulo = C.ulo, uhi = C.uhi;
   const uint2* cand = C.cand;
   const uint2 me = cand[q0];
-  int cx, cy, cz;
-  {
-    const double cf = C.cf;
-    cx = min((int)(P.x(i) * cf), ncx - 1);
-    cy = min((int)(P.y(i) * cf), ncx - 1);
-    cz = min((int)(P.z(i) * cf), ncx - 1);
-  }
+  const int cx = clmd_cell(P.x(i), C.cf, ncx), cy = clmd_cell(P.y(i), C.cf, ncx),
+            cz = clmd_cell(P.z(i), C.cf, ncx);
   // the cells of a row: [xa, xb), and the one the row wraps to (edge)
   const int xa = nox < 3 ? 0 : max(cx - 1, 0), xb = nox < 3 ? ncx : min(cx + 2, ncx);
   const bool edge = nox == 3 && (cx == 0 || cx == ncx - 1);
@@ -724,8 +719,8 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
       y = wrap_box(y, L);
       z = wrap_box(z, L);
       P.set(i, x, y, z);
-      const int cx = min((int)(x * C.cf), C.ncx - 1), cy = min((int)(y * C.cf), C.ncx - 1),
-                cz = min((int)(z * C.cf), C.ncx - 1);
+      const int cx = clmd_cell(x, C.cf, C.ncx), cy = clmd_cell(y, C.cf, C.ncx),
+                cz = clmd_cell(z, C.cf, C.ncx);
       const int c = (cz * C.ncx + cy) * C.ncx + cx, sh = 16 * (c & 1);
       const unsigned before = (atomicAdd(word + (c >> 1), 1u << sh) >> sh) & 0xffffu;
       A.cellid[off + i] = (int)(before << 15) | c;
@@ -762,9 +757,9 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
       y = wrap_box(y, L);
       z = wrap_box(z, L);
       P.set(i, x, y, z);
-      int cx = min((int)(x * C.cf), C.ncx - 1), cy = min((int)(y * C.cf), C.ncx - 1),
-          cz = min((int)(z * C.cf), C.ncx - 1);
-      int c = (cz * C.ncx + cy) * C.ncx + cx;
+      const int cx = clmd_cell(x, C.cf, C.ncx), cy = clmd_cell(y, C.cf, C.ncx),
+                cz = clmd_cell(z, C.cf, C.ncx);
+      const int c = (cz * C.ncx + cy) * C.ncx + cx;
       A.cellid[off + i] = c;
       atomicAdd(&cnt[c + 1], 1);
     }

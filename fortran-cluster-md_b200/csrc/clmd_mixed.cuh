@@ -15,6 +15,14 @@ __device__ __forceinline__ float clmd_rcp_f32(float x) {
   return r;
 }
 
+// The cell (0 .. n - 1) of a coordinate wrapped into the box, c cells per unit
+// length.  A NaN, which wrapping leaves one, would convert to the smallest
+// integer: its cell is the first.  (Not max(.., 0) on the integers: built so,
+// the ensemble's search lists pairs of the first two cells twice.)
+__device__ __forceinline__ int clmd_cell(double x, double c, int n) {
+  return min((int)fmax(x * c, 0.0), n - 1);
+}
+
 // The implicit Nose-Hoover velocity step of int-verlet-nh-mav.f:105-147 in
 // closed form.  The reference's Newton sweeps stop at the
 // fixed point v (1 + dth p) = V + dth a =: W, p = psi1 + (m sum v^2 - 3NkT)

@@ -119,9 +119,9 @@ static __device__ bool s_rebuild(const Params& P, DevState* st, SmallShared& S, 
   int cell = 0, arrival = 0;
   if (a.act) {
     a.q = wrap_box(P, a.q);
-    const int cx = min((int)(a.q.x * g.cfx), g.ncx - 1);
-    const int cy = min((int)(a.q.y * g.cfy), g.ncy - 1);
-    const int cz = min((int)(a.q.z * g.cfz), g.ncz - 1);
+    const int cx = clmd_cell(a.q.x, g.cfx, g.ncx);
+    const int cy = clmd_cell(a.q.y, g.cfy, g.ncy);
+    const int cz = clmd_cell(a.q.z, g.cfz, g.ncz);
     cell = (cz * g.ncy + cy) * g.ncx + cx;
     arrival = atomicAdd(&A.cell_count[cell], 1);
   }
