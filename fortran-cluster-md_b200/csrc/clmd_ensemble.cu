@@ -611,7 +611,9 @@ __device__ void cta_scan16(unsigned* word, int nw) {
 // (neighbour k at list[lbase + k N + i], at most the stride of them); returns
 // the neighbours found.
 // A candidate is 8 bytes in cell order: its coordinates in 2^-16 of the box
-// and its slot's low 16 bits.  The 16-bit differences wrap like the periodic
+// and its slot (below 2^15 where positions are in shared memory; elsewhere not
+// kept), with the top bit set for an atom at a NaN, which is nobody's
+// neighbour.  The 16-bit differences wrap like the periodic
 // box, so the nearest image needs no test, and three integer products decide
 // all candidates but those within the truncation of the list radius (~0.3% of
 // r^2), which FP64 positions decide (mi_sel and r^2 rounded term by term; r^2
@@ -658,7 +660,7 @@ __device__ __forceinline__ int search_row(const Cta& C, const Args& A, const Pos
     const int dx = (short)(me.x - c.x), dy = (short)((me.x >> 16) - (c.x >> 16)),
               dz = (short)(me.y - c.y);
     const unsigned u = (unsigned)(dx * dx) + (unsigned)(dy * dy) + (unsigned)(dz * dz);
-    if (u > uhi || q == q0) return;
+    if (u > uhi || q == q0 || (int)c.y < 0) return;
     const int j = SM ? (int)(c.y >> 16) : (C.ident ? q : A.sorted[P.off + q]);
     if (u >= ulo) {
       const double hL = 0.5 * L;
@@ -844,7 +846,11 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
     auto u16 = [&](double x) { return (unsigned)(int)(x * k) & 0xffffu; };
     for (int q = gt; q < N; q += GT) {
       const int i = C.ident ? q : A.sorted[off + q];
-      C.cand[q] = make_uint2(u16(P.x(i)) | u16(P.y(i)) << 16, u16(P.z(i)) | (unsigned)i << 16);
+      double x, y, z;
+      P.get(i, x, y, z);
+      unsigned tag = SM ? (unsigned)i : 0u;
+      if (isnan(x + y + z)) tag |= 0x8000u;
+      C.cand[q] = make_uint2(u16(x) | u16(y) << 16, u16(z) | tag << 16);
     }
     gsync<CS>();
   }
@@ -853,8 +859,7 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
   // candidates read by several lanes at once)
   for (int q0 = gt; q0 < N; q0 += GT) {
     const int i = C.ident ? q0 : A.sorted[off + q0];
-    const double fin = P.x(i) + P.y(i) + P.z(i);  // (an atom at a NaN has no neighbours)
-    const int n = fin == fin ? search_row<SM>(C, A, P, q0, i, N, L, lbase) : 0;
+    const int n = (int)C.cand[q0].y < 0 ? 0 : search_row<SM>(C, A, P, q0, i, N, L, lbase);
     if (n > A.lstride) over = 1;
     A.rlen[off + i] = min(n, A.lstride);
     nsum += min(n, A.lstride);

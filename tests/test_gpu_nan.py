@@ -51,8 +51,11 @@ def test_system_rebuild(gpu, n, rho, precision):
 
 @pytest.mark.parametrize("n,rho", [(60, 0.35), (300, 0.05), (8200, 0.05), (12000, 0.03)])
 def test_replica_rebuild(gpu, n, rho):
-    """Candidates in and outside shared memory, and a cluster."""
+    """Candidates in and outside shared memory, and a cluster; some atoms near
+    the origin, where the cell of the NaNs is."""
     box, x, ok = positions(n, rho, n)
+    for a in x:
+        a[20:28] = np.random.default_rng(1).uniform(0, 0.4, 8)
     v = np.random.default_rng(n).normal(size=(3, n)) * 1e-9
     e = clmd.Ensemble(clmd.ens_config(n, 1, ftcsi=1, rskin=RSKIN, integrator=clmd.INT_VERLET,
                                       precision=clmd.PREC_FP64, dt=1e-30, list_stride=512))
@@ -60,5 +63,6 @@ def test_replica_rebuild(gpu, n, rho):
     e.step(1)
     r = e.results()[0]
     assert r.status == 0 and r.nrebuild == 1
+    assert e.pair_terms() == ordered_pairs(x, ok, box, RSKIN)
     st, _ = e.state(0)
     assert np.isfinite(np.stack([st.ax, st.ay, st.az])[:, ok]).all()
