@@ -32,23 +32,26 @@ __device__ __forceinline__ int clmd_cell(double x, double c, int n) {
 // velocity is W / (1 + dth p): one reduction instead of a reduction per
 // sweep (FP64, 500 replicas 9.07 -> 6.32 ms a window; N = 5,921 on one cluster
 // 6.05 -> 4.10 ms per 200 steps).  Newton's method from psi1, two or three
-// steps in practice (from below, where overlapping atoms make S huge, each
-// multiplies 1 + dth p by 1.5: some 200 for S = 1e100), until f is 1e-13 of its
-// terms at p: |psi1| + (S / (1 + dth p)^2 + 3NkT) dth/Q, and p's own part |p| f'
-// (rounding noise in f is a few 1e-16 of them, so a tighter limit can stall).
+// steps in practice; the step limit is 1e-13 of the terms' scale (|p| + |psi1| +
+// (S + 3NkT) dth/Q; rounding noise in f is a few 1e-16 of it, so a tighter limit
+// can stall).  Where overlapping atoms make S huge, that scale is far above p,
+// and steps from below multiply 1 + dth p by 1.5 each (some 200 for S = 1e100):
+// the last one must also be 1e-8 of 1 + dth p.
 // False (no convergence) if the root is not finite or the iteration does not
 // settle: mixed precision then stops, as the reference's STOP; FP64 takes the
 // sweeps (clmd_nh_closed).
 __device__ __forceinline__ bool clmd_nh_root(double S, double psi1, double nkt3, double dth,
                                              double Q, double& p) {
   const double k0 = dth / Q;
+  const double scale = fabs(psi1) + k0 * (S + fabs(nkt3));
   p = psi1;
   for (int it = 0; it < 1000; it++) {
     const double c = 1.0 / (1.0 + dth * p);
     const double f = p - psi1 - (S * c * c - nkt3) * k0;
     const double fp = 1.0 + 2.0 * S * dth * k0 * c * c * c;
-    p = p - f / fp;
-    if (!(fabs(f) > 1e-13 * (fabs(psi1) + k0 * (S * (c * c) + fabs(nkt3)) + fabs(p * fp))))
+    const double d = f / fp;
+    p = p - d;
+    if (!(fabs(d) > 1e-13 * (scale + fabs(p))) && !(dth * fabs(d) > 1e-8 * fabs(1.0 + dth * p)))
       return isfinite(p) && 1.0 + dth * p > 0.0;
   }
   return false;
