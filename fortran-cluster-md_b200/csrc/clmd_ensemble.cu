@@ -252,7 +252,6 @@ __device__ __forceinline__ double mi_bf(double d, double L, double iL, double bf
 struct Cta {
   double xred[3 * 16];  // cluster reductions: the CTAs' partials (rank 0's copy is read)
   double xloc[4];       // cluster reductions: the totals, for this CTA's threads
-  double* sub;          // cluster: the warps' sums of a pass's first half, by slot
   double* sx;  // positions in shared memory (nullptr: global)
   double* sy;
   double* sz;
@@ -263,7 +262,7 @@ struct Cta {
   uint2* cand;        // the search's candidates in cell order (search_row)
   unsigned ulo, uhi;  // its test: below ulo a neighbour, above uhi none
   double red[3 * 32 + 8];
-  int ncx, ncell, nox, offx[3];
+  int ncx, ncell, nox;
   double cf, rs2;
   int flag;
   int ident;  // sorted[] is the identity (the slots are in cell order)
@@ -306,17 +305,21 @@ __device__ __forceinline__ void gsync() {
 // replica's wider cluster.  On the one of half as many CTAs (H = 2) the loops
 // that sum go over the atoms in two halves: thread t of CTA r stands for
 // thread t of CTA r, then for thread t of CTA r + CS, of the wider one.  The
-// first half's warp sums wait in C.sub (half_out) for the grp_* call.  The
-// two halves cost 1-2% of a window (FP64: 2-3%).
-__device__ __forceinline__ void half_out(double& v, int slot, Cta& C) {
+// first half's warp sums wait in halves(), by slot (half_out), for the grp_*
+// call.  The two halves cost up to 1% of a window (FP64: 2%).
+__device__ __forceinline__ double* halves() {
+  __shared__ double sums[4 * 32];
+  return sums;
+}
+__device__ __forceinline__ void half_out(double& v, int slot) {
   v = wsum(v);
-  if ((threadIdx.x & 31) == 0) C.sub[32 * slot + (threadIdx.x >> 5)] = v;
+  if ((threadIdx.x & 31) == 0) halves()[32 * slot + (threadIdx.x >> 5)] = v;
   v = 0.0;
 }
 
 // a reduction over a cluster's threads (1024 a CTA) of nv <= 3 values,
 // returned in v to every thread; op 0 sums, op 1 takes maxima; H = 2: the
-// sums' first halves are in C.sub's slots from `slot` on.  Two cluster
+// sums' first halves are in halves()'s slots from `slot` on.  Two cluster
 // barriers: the CTAs' partials are published, then read by every CTA before
 // any CTA may write the next reduction's.
 template <int CS, int H>
@@ -333,7 +336,7 @@ __device__ __forceinline__ void cl_reduce(double* v, int nv, const int* op, Cta&
     double* b0 = cl.map_shared_rank(C.xred, 0);
     for (int k = 0; k < nv; k++) {
       double t = C.red[32 * k + lane], t0 = 0.0;
-      if (H == 2) t0 = op[k] ? t : C.sub[32 * (slot + k) + lane];
+      if (H == 2) t0 = op[k] ? t : halves()[32 * (slot + k) + lane];
       t = op[k] ? wmax(t) : wsum(t);
       if (H == 2) t0 = op[k] ? t : wsum(t0);
       if (lane == 0) {
@@ -461,13 +464,7 @@ __device__ bool prologue(Rep& R, Cta& C, const Args& A, int step) {
   C.ncx = n;
   C.ncell = n * n * n;
   C.cf = (double)n / R.box;
-  if (n >= 3) {
-    C.nox = 3; C.offx[0] = -1; C.offx[1] = 0; C.offx[2] = 1;
-  } else if (n == 2) {
-    C.nox = 2; C.offx[0] = 0; C.offx[1] = 1;
-  } else {
-    C.nox = 1; C.offx[0] = 0;
-  }
+  C.nox = min(n, 3);
   R.dmmax = fmax(R.dmms, R.dmmax);
   R.dmms = 0.0;
   R.dmmst = 0;
@@ -1028,11 +1025,11 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
   } else {
     for (int h = 0; h < H; h++) {
       if (h > 0) {
-        if (NHF) half_out(*s0, 0, C);
+        if (NHF) half_out(*s0, 0);
         if (energies) {
-          half_out(esum, 1, C);
-          half_out(vir, 2, C);
-          half_out(ek, 3, C);
+          half_out(esum, 1);
+          half_out(vir, 2);
+          half_out(ek, 3);
         }
       }
       for (int i0 = h * GT; i0 < N; i0 += H * GT) {
@@ -1161,7 +1158,7 @@ __device__ __noinline__ bool nh_sweep(Rep& R, Cta& C, double dt, const double* w
   double s[3] = {0.0, 0.0, 0.0};
   for (int h = 0; h < H; h++) {
     if (h > 0)
-      for (int k = 0; k < 3; k++) half_out(s[k], k, C);
+      for (int k = 0; k < 3; k++) half_out(s[k], k);
     for (int i = gt + h * GT; i < N; i += H * GT) {
       s[0] += wx[i] * wx[i] + wy[i] * wy[i] + wz[i] * wz[i];
       s[1] += wx[i] * vx[i] + wy[i] * vy[i] + wz[i] * vz[i];
@@ -1223,9 +1220,9 @@ __device__ void stopdead(Rep& R, Cta& C, const Args& A) {
     double px = 0, py = 0, pz = 0;
     for (int h = 0; h < H; h++) {
       if (h > 0) {
-        half_out(px, 0, C);
-        half_out(py, 1, C);
-        half_out(pz, 2, C);
+        half_out(px, 0);
+        half_out(py, 1);
+        half_out(pz, 2);
       }
       for (int i = gt + h * GT; i < N; i += H * GT) {
         px += A.vx[off + i];
@@ -1238,7 +1235,7 @@ __device__ void stopdead(Rep& R, Cta& C, const Args& A) {
     double vzs = grp_sum<NT, CS, H>(pz, C, 2) / (double)N;
     double ek = 0.0;
     for (int h = 0; h < H; h++) {
-      if (h > 0) half_out(ek, 0, C);
+      if (h > 0) half_out(ek, 0);
       for (int i = gt + h * GT; i < N; i += H * GT) {
         double a = A.vx[off + i] - vxs, b = A.vy[off + i] - vys, c = A.vz[off + i] - vzs;
         A.vx[off + i] = a;
@@ -1423,10 +1420,7 @@ __device__ bool run_steps(Rep& R, Cta& C, const Args& A) {
     C.ncell = n * n * n;
     C.cf = (double)n / R.box;
     C.rs2 = R.atrskin * R.atrskin;
-    C.nox = n >= 3 ? 3 : n;
-    C.offx[0] = n >= 3 ? -1 : 0;
-    C.offx[1] = n >= 3 ? 0 : 1;
-    C.offx[2] = 1;
+    C.nox = min(n, 3);
   }
   gsync<CS>();
   if (!R.started) {
@@ -1483,7 +1477,7 @@ __device__ bool run_steps(Rep& R, Cta& C, const Args& A) {
       const double sc = vin_n ? vsc : 1.0;
       vin_n = false;
       for (int h = 0; h < H; h++) {
-        if (h > 0) half_out(sv, 0, C);
+        if (h > 0) half_out(sv, 0);
         for (int i = gt + h * GT; i < N; i += H * GT) {
           double vxi = svx[off + i], vyi = svy[off + i], vzi = svz[off + i];
           vxi = vxi * sc;
@@ -1541,7 +1535,7 @@ __device__ bool run_steps(Rep& R, Cta& C, const Args& A) {
           sumv2 = wsum(lane < W ? C.red[W + lane] : 0.0);
         }
       } else {
-        // (slot 0 of C.sub is the second value's)
+        // (slot 0 of halves() is the second value's)
         double t[2] = {d2, sv};
         const int op[2] = {1, 0};
         cl_reduce<CS, H>(t, 2, op, C, -1);
@@ -1723,7 +1717,6 @@ __global__ void __launch_bounds__(NT, 1) k_ens_cl(Args A) {
   extern __shared__ double dsm[];
   __shared__ Rep R;
   __shared__ Cta C;
-  __shared__ double sub[4 * 32];
   __shared__ int item;
   auto cl = cg::this_cluster();
   const unsigned rank = cl.block_rank();
@@ -1745,7 +1738,6 @@ __global__ void __launch_bounds__(NT, 1) k_ens_cl(Args A) {
       C.cstart = (int*)dsm;
       C.cand = A.cand + R.off;
       C.sx = C.sy = C.sz = nullptr;
-      C.sub = sub;
     }
     unsigned long long t0 = 0;
     const int step0 = R.step;
@@ -2329,10 +2321,9 @@ static int cluster_class(const clmd_ensemble* E, int n) {
 // c may run there instead, and their sums are laid out for it on either
 static int wider_class(const clmd_ensemble* E, int c) {
   const int w = c + 1;
-  return w < clmd_ensemble::kClasses && E->cls_cs[w] == 2 * E->cls_cs[c] &&
-                 E->cl_max_clusters[w] > 0
-             ? w
-             : c;
+  const bool has = c >= clmd_ensemble::kCtaClasses && w < clmd_ensemble::kClasses &&
+                   E->cls_cs[w] == 2 * E->cls_cs[c] && E->cl_max_clusters[w] > 0;
+  return has ? w : c;
 }
 
 static int prepare_class(clmd_ensemble* E, int c, int item0, int nitems, const int* slots,
@@ -2442,13 +2433,15 @@ static int enqueue_class(clmd_ensemble* E, int c, const ClassLaunch& L, int nwin
 // only >= 0: that size class alone (the autotuner's trials)
 static int launch_all(clmd_ensemble* E, int nwin, const int* threads, float min_ms = 0.0f,
                       int only = -1) {
-  std::vector<int> cls[clmd_ensemble::kClasses];
-  int nmax[clmd_ensemble::kClasses] = {};
-  auto running = [&](int s) { return E->used[s] && !E->h_summary[s].x && !E->h_summary[s].y; };
-  auto cluster_of = [&](int s) {
-    return E->use_clusters && E->h_reps[s].reorder == 1 ? cluster_class(E, E->h_reps[s].natom)
-                                                        : -1;
-  };
+  // the running replicas and their classes
+  std::vector<std::pair<int, int>> run;
+  for (int s = 0; s < E->cfg.max_replicas; s++)
+    if (E->used[s] && !E->h_summary[s].x && !E->h_summary[s].y) {
+      const Rep& R = E->h_reps[s];
+      int c = -1;
+      if (E->use_clusters && R.reorder == 1) c = cluster_class(E, R.natom);
+      run.push_back({s, c < 0 ? cta_class(E, R.natom) : c});
+    }
   // Replicas on clusters take the wider ones (~3,072 atoms per CTA) if all
   // running replicas then fit on the GPU at once: a cluster takes the place of
   // two of half its size, of which the GPU holds cl_max_clusters, and the CTAs
@@ -2460,28 +2453,20 @@ static int launch_all(clmd_ensemble* E, int nwin, const int* threads, float min_
   {
     long long n[clmd_ensemble::kClasses] = {}, held = 0;
     double sms = 0.0;
-    for (int s = 0; s < E->cfg.max_replicas; s++)
-      if (running(s)) {
-        int c = cluster_of(s);
-        c = c < 0 ? cta_class(E, E->h_reps[s].natom) : wider_class(E, c);
-        n[c]++;
-        sms += (double)E->cls_cs[c] / shape_ctas_per_sm(threads[c]);
-      }
-    for (int c = clmd_ensemble::kClasses - 1; c >= clmd_ensemble::kCtaClasses; c--) {
+    for (const auto& r : run) n[wider_class(E, r.second)]++;
+    for (int c = clmd_ensemble::kClasses - 1; c >= 0; c--) {
+      sms += (double)(n[c] * E->cls_cs[c]) / shape_ctas_per_sm(threads[c]);
+      if (c < clmd_ensemble::kCtaClasses) continue;
       held = 2 * held + n[c];
       if (held > E->cl_max_clusters[c]) wide = false;
     }
     if (sms > E->nsm) wide = false;
   }
-  for (int s = 0; s < E->cfg.max_replicas; s++)
-    if (running(s)) {
-      const int n = E->h_reps[s].natom;
-      int c = cluster_of(s);
-      c = c < 0 ? cta_class(E, n) : wide ? wider_class(E, c) : c;
-      if (only >= 0 && c != only) continue;
-      cls[c].push_back(s);
-      nmax[c] = std::max(nmax[c], n);
-    }
+  std::vector<int> cls[clmd_ensemble::kClasses];
+  for (const auto& r : run) {
+    const int c = wide ? wider_class(E, r.second) : r.second;
+    if (only < 0 || c == only) cls[c].push_back(r.first);
+  }
   int total = 0;
   for (int c = 0; c < clmd_ensemble::kClasses; c++) {
     std::sort(cls[c].begin(), cls[c].end(), [&](int a, int b) {
