@@ -471,6 +471,8 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
         }
         G.barrier();
         if (const int err = S.err[G.rb]) {
+          // the positions of this step, not the fused drift's
+          if (fuse && a.act) a.q = (cur ? A.pos1 : A.pos0)[p];
           if (tid == 0 && B.q.status == 0) {
             B.q.status = err;
             B.q.fail_step = step;

@@ -4,6 +4,8 @@ largest size and the first beyond it, rows longer than the search's buffer.
 FP64 velocity Verlet is bit-identical to the oracle; Nose-Hoover and the
 energy sums agree within the rounding of the sums, mixed precision within
 the FP32 rounding of the pair terms over a few steps."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -138,3 +140,26 @@ def test_velocity_scaling_bits(gpu, n, two):
         kf = np.sqrt(1.5 * clmd.CIKB * cfg.att * m.sum() / block_tree(np.where(m, e, 0.0)))
         for got, was in zip((out.vx, out.vy, out.vz), v):
             assert np.array_equal(got[m], was[m] * kf), s
+
+
+@pytest.mark.parametrize("n", [64, 2049, 9000])  # one cluster, the grid
+def test_bad_species_leaves_positions(gpu, n):
+    """A pair of species without coefficients stops a run in its first force
+    pass: the positions are those of that step, whether the launch would have
+    gone on with the next step's drift or not."""
+    cfg = clmd.lj_config(n, 0.05, 0.8)
+    cfg.atsorts = 3
+    for s, (k, m) in enumerate(((n // 2, 1.0), (n // 4, 1.0), (n - n // 2 - n // 4, 1.0))):
+        cfg.apnum[s], cfg.apmas[s], cfg.apsig[s], cfg.apeps[s] = k, m, 1.0, 1.0
+    st = random_state(cfg, n)
+    out = []
+    for steps in (1, 3):
+        g = clmd.System(cfg)
+        g.set_state(st, scalars=clmd.scalars_init(cfg))
+        g.neighbor(0)
+        assert g.lib.clmd_steps(g.h, 1, steps) == clmd.ERR_BAD_SPECIES
+        x = [np.zeros(n) for _ in range(3)]
+        g.lib.clmd_get_state(g.h, *[clmd.ptr(a, C.c_double) for a in x], *([None] * 7))
+        out.append(x)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
