@@ -1788,9 +1788,6 @@ struct clmd_ensemble {
   int* d_iwin = nullptr;   // windows per item (balanced launches)
   int* h_iwin = nullptr;   // pinned
   float* h_wtime = nullptr;  // pinned copy of A.wtime
-  // one replica's arrays on their way in or out, contiguous, in atom order
-  double* d_xfer = nullptr;
-  size_t xfer_cap = 0;
   double* d_stage = nullptr;  // bulk copies in atom order (pool doubles, on first use)
   long long* d_hoff = nullptr;  // clmd_ens_step_io: each slot's offset in the host arrays
   int4* h_summary = nullptr;  // pinned copy of A.summary
@@ -2057,7 +2054,7 @@ extern "C" int clmd_ens_destroy(clmd_ensemble* E) {
   void* ps[] = {A.x, A.y, A.z, A.vx, A.vy, A.vz, A.vxn, A.vyn, A.vzn, A.a, A.list, A.rlen,
                 A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.cand, A.p4, A.reps, A.fpt, A.summary,
                 E->d_items, E->d_ctr, E->d_iwin, A.wtime, E->d_stage, A.cscr,
-                E->d_hoff, E->d_xfer};
+                E->d_hoff};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (E->h_reps) cudaFreeHost(E->h_reps);
@@ -2136,57 +2133,34 @@ extern "C" int clmd_ens_pair_terms(clmd_ensemble* E, int64_t* total) {
   return CLMD_OK;
 }
 
-static int ensure_xfer(clmd_ensemble* E, int n) {
-  size_t need = 9 * (size_t)n;
-  if (need <= E->xfer_cap) return CLMD_OK;
-  // (for replicas of up to 16,384 atoms at once; then doubled)
-  need = std::max(need, std::min(std::max(2 * E->xfer_cap, (size_t)9 * 16384),
-                                 9 * (size_t)E->A.pool));
-  ECK(cudaStreamSynchronize(E->stream));
-  cudaFree(E->d_xfer);
-  E->d_xfer = nullptr;
-  E->xfer_cap = 0;
-  ECK(cudaMalloc(&E->d_xfer, 8 * need));
-  E->xfer_cap = need;
-  return CLMD_OK;
-}
-
-// an admitted replica's atoms into its pool range: x..vz, each slot holding
-// its own atom, no list rows yet (the first order does not depend on the
-// pool's history), no first passages
-__global__ void k_admit(Args A, const double* in, int n, int off, int slot) {
+// what an admitted replica's pool range holds beside x..vz: each slot its own
+// atom, no list rows yet (the first order does not depend on the pool's
+// history), no first passages
+__global__ void k_admit(Args A, int n, int off, int slot) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < kFptCap) A.fpt[(size_t)slot * kFptCap + i] = -1;
   if (i == 0) A.summary[slot] = make_int4(0, 0, 0, 0);
   if (i >= n) return;
-  A.x[off + i] = in[i];
-  A.y[off + i] = in[n + i];
-  A.z[off + i] = in[2 * (size_t)n + i];
-  A.vx[off + i] = in[3 * (size_t)n + i];
-  A.vy[off + i] = in[4 * (size_t)n + i];
-  A.vz[off + i] = in[5 * (size_t)n + i];
   A.orig[off + i] = off + i;
   A.rlen[off + i] = 0;
 }
 
-// a replica's x..vz, ax..az in atom order (orig[]), nine arrays of n
+// a replica's x..vz, ax..az in atom order (orig[]): those that have a place
+struct Export {
+  double* p[9];
+};
 template <bool MIXED>
-__global__ void k_export(Args A, double* out, int n, int off) {
+__global__ void k_export(Args A, Export out, int n, int off) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const size_t s = (size_t)off + i;
-  double* o = out + (A.orig[s] - off);
-  o[0] = A.x[s];
-  o[n] = A.y[s];
-  o[2 * (size_t)n] = A.z[s];
-  o[3 * (size_t)n] = A.vx[s];
-  o[4 * (size_t)n] = A.vy[s];
-  o[5 * (size_t)n] = A.vz[s];
-  double ax, ay, az;
-  get_a<MIXED>(A, (int)s, ax, ay, az);
-  o[6 * (size_t)n] = ax;
-  o[7 * (size_t)n] = ay;
-  o[8 * (size_t)n] = az;
+  const int o = A.orig[s] - off;
+  const double* xv[6] = {A.x, A.y, A.z, A.vx, A.vy, A.vz};
+  double a[3];
+  get_a<MIXED>(A, (int)s, a[0], a[1], a[2]);
+#pragma unroll
+  for (int k = 0; k < 9; k++)
+    if (out.p[k]) out.p[k][o] = k < 6 ? xv[k][s] : a[k - 6];
 }
 
 extern "C" int clmd_ens_add(clmd_ensemble* E, const clmd_replica_spec* sp, const double* x,
@@ -2207,17 +2181,10 @@ extern "C" int clmd_ens_add(clmd_ensemble* E, const clmd_replica_spec* sp, const
   if (off < 0) return CLMD_ERR_NOMEM;
   Args& A = E->A;
   cudaStream_t st = E->stream;
-  {
-    const int rc = ensure_xfer(E, N);
-    if (rc) {
-      pool_free(E, off, N);
-      return rc;
-    }
-  }
   const double* src[6] = {x, y, z, vx, vy, vz};
+  double* dst[6] = {A.x, A.y, A.z, A.vx, A.vy, A.vz};
   for (int k = 0; k < 6; k++)
-    ECK(cudaMemcpyAsync(E->d_xfer + (size_t)k * N, src[k], 8 * (size_t)N, cudaMemcpyHostToDevice,
-                        st));
+    ECK(cudaMemcpyAsync(dst[k] + off, src[k], 8 * (size_t)N, cudaMemcpyHostToDevice, st));
   Rep& R = E->h_reps[s];
   memset(&R, 0, sizeof(Rep));
   R.box = sp->box;
@@ -2247,7 +2214,7 @@ extern "C" int clmd_ens_add(clmd_ensemble* E, const clmd_replica_spec* sp, const
   // CLMD_ENS_ORDER=cell: cell order for every replica
   R.reorder = (fits && !E->cell_order) ? 2 : 1;
   E->h_summary[s] = make_int4(0, 0, 0, 0);
-  k_admit<<<(std::max(N, kFptCap) + 255) / 256, 256, 0, st>>>(A, E->d_xfer, N, (int)off, s);
+  k_admit<<<(std::max(N, kFptCap) + 255) / 256, 256, 0, st>>>(A, N, (int)off, s);
   ECK(cudaGetLastError());
   E->launches++;
   ECK(cudaMemcpyAsync(A.reps + s, &R, sizeof(Rep), cudaMemcpyHostToDevice, st));
@@ -2738,19 +2705,29 @@ extern "C" int clmd_ens_get_state(clmd_ensemble* E, int32_t slot, double* x, dou
   const int N = E->h_reps[slot].natom;
   cudaStream_t st = E->stream;
   double* dst[9] = {x, y, z, vx, vy, vz, ax, ay, az};
-  bool any = false;
-  for (double* d : dst) any = any || d;
-  if (any) {
-    const int rc = ensure_xfer(E, N);
-    if (rc) return rc;
-    auto k = E->cfg.precision == CLMD_PREC_MIXED ? k_export<true> : k_export<false>;
-    k<<<(N + 255) / 256, 256, 0, st>>>(A, E->d_xfer, N, (int)off);
+  // in atom order through the replica's part of arrays that are free between
+  // windows: the window's velocities and positions, the candidates, and what
+  // FP32 accelerations leave of theirs (FP64: the ninth array after the others)
+  const bool mixed = E->cfg.precision == CLMD_PREC_MIXED;
+  double* room[9] = {A.vxn + off, A.vyn + off, A.vzn + off, (double*)(A.cand + off)};
+  for (int q = 4; q < 8; q++) room[q] = (double*)(A.p4 + off) + (size_t)(q - 4) * N;
+  room[8] = mixed ? (double*)A.a + (3 * A.pool + 1) / 2 + off : room[0];
+  auto k = mixed ? k_export<true> : k_export<false>;
+  for (int q0 = 0, q1 = mixed ? 9 : 8; q0 < 9; q0 = q1, q1 = 9) {
+    Export out = {};
+    bool any = false;
+    for (int q = q0; q < q1; q++)
+      if (dst[q]) {
+        out.p[q] = room[q];
+        any = true;
+      }
+    if (!any) continue;
+    k<<<(N + 255) / 256, 256, 0, st>>>(A, out, N, (int)off);
     ECK(cudaGetLastError());
     E->launches++;
-    for (int q = 0; q < 9; q++)
+    for (int q = q0; q < q1; q++)
       if (dst[q])
-        ECK(cudaMemcpyAsync(dst[q], E->d_xfer + (size_t)q * N, 8 * (size_t)N,
-                            cudaMemcpyDeviceToHost, st));
+        ECK(cudaMemcpyAsync(dst[q], out.p[q], 8 * (size_t)N, cudaMemcpyDeviceToHost, st));
   }
   if (cl) ECK(cudaMemcpyAsync(cl, A.cl + off, 4 * (size_t)N, cudaMemcpyDeviceToHost, st));
   ECK(cudaStreamSynchronize(st));

@@ -733,3 +733,22 @@ def test_cluster_replica_in_any_pool(gpu, precision, n):
             assert np.array_equal(getattr(a, k), getattr(b, k)), (k, pool, before, between)
         assert np.array_equal(ca, cb)
         assert (ra.psi, ra.s, ra.ekin, ra.epot) == (rb.psi, rb.s, rb.ekin, rb.epot)
+
+
+def test_admission_and_readout_take_no_memory(gpu):
+    """A replica's way in and out needs no device memory beyond the pool's: one
+    that fits the pool is admitted, and read out, however full the GPU is."""
+    import torch
+
+    n = 300000
+    e = clmd.Ensemble(clmd.ens_config(n + 1000, 2, ftcsi=1))
+    box, arrs = replica_inputs(500, 0.02, 0.7, 1)
+    e.state(e.add(500, box, 0.7, *arrs))  # (kernels loaded)
+    rng = np.random.default_rng(2)
+    xv = [rng.uniform(0, 300.0, n) for _ in range(3)] + [rng.normal(size=n) for _ in range(3)]
+    free = torch.cuda.mem_get_info()[0]
+    s = e.add(n, 300.0, 0.7, *xv)
+    st, _ = e.state(s)
+    assert torch.cuda.mem_get_info()[0] == free
+    for a, k in zip(xv, ("x", "y", "z", "vx", "vy", "vz")):
+        assert np.array_equal(getattr(st, k), a)
