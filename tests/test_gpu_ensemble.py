@@ -752,3 +752,62 @@ def test_admission_and_readout_take_no_memory(gpu):
     assert torch.cuda.mem_get_info()[0] == free
     for a, k in zip(xv, ("x", "y", "z", "vx", "vy", "vz")):
         assert np.array_equal(getattr(st, k), a)
+
+
+@pytest.mark.parametrize("n,rho", [(120, 0.3), (1000, 0.05), (5000, 0.03), (8200, 0.05),
+                                   (9300, 0.02), (12000, 0.04), (70000, 0.03)])
+def test_list_neighbours_by_their_forces(gpu, n, rho):
+    """Which neighbours the search finds, not only how many: each atom's
+    acceleration against the FP64 sum over the pairs of a k-d tree, on
+    positions where no pair overlaps (slots of 14 and more bits, candidates in
+    and outside shared memory, clusters).  Sums of some ten terms in another
+    order: 1e-12 of the largest."""
+    from scipy.spatial import cKDTree
+
+    box, arrs = replica_inputs(n, rho, 0.7, n)
+    e = clmd.Ensemble(clmd.ens_config(n, 1, ftcsi=1, integrator=clmd.INT_VERLET,
+                                      precision=clmd.PREC_FP64, dt=1e-30))
+    s = e.add(n, box, 0.7, *arrs, ethst="-", csover=10**6)
+    e.step(1)
+    st, _ = e.state(s)
+    x = np.mod(np.stack([st.x, st.y, st.z], 1), box)
+    i, j = cKDTree(x, boxsize=box).query_pairs(2.5, output_type="ndarray").T
+    d = x[i] - x[j]
+    d -= box * np.round(d / box)
+    r2 = (d * d).sum(1)
+    r6 = 1.0 / r2 ** 3
+    f = (48.0 * r6 * (r6 - 0.5) / r2)[:, None] * d
+    a = np.zeros((n, 3))
+    np.add.at(a, i, f)
+    np.subtract.at(a, j, f)
+    got = np.stack([st.ax, st.ay, st.az], 1)
+    np.testing.assert_allclose(got, a, rtol=0, atol=1e-12 * np.abs(a).max())
+
+
+def test_ensembles_side_by_side_as_alone(gpu):
+    """Ensembles that need different amounts of shared memory, stepped in turn:
+    the same bits as each alone."""
+    specs = [(4000, 0.05), (3000, 0.01), (2500, 0.05), (8500, 0.03), (400, 0.02)]
+
+    def make(n, rho):
+        e = clmd.Ensemble(clmd.ens_config(n, 1, ftcsi=5))
+        box, arrs = replica_inputs(n, rho, 0.75, n)
+        assert e.add(n, box, 0.75, *arrs, csover=10**6) is not None
+        return e
+
+    alone = []
+    for spec in specs:
+        e = make(*spec)
+        for _ in range(3):
+            e.step(1)
+        alone.append(e.state(0))
+        e.close()
+    es = [make(*spec) for spec in specs]
+    for _ in range(3):
+        for e in es:
+            e.step(1)
+    for e, (a, ca) in zip(es, alone):
+        b, cb = e.state(0)
+        for k in ("x", "y", "z", "vx", "vy", "vz", "ax", "ay", "az"):
+            assert np.array_equal(getattr(a, k), getattr(b, k)), k
+        assert np.array_equal(ca, cb)
