@@ -199,8 +199,8 @@ __device__ void clu_done(DevState* st) {
 // which the reference never resets)
 constexpr int kSmallBins = 64;
 
-__global__ void k_clu_hist(Params P, DevState* st, int force, const int* cs, const double* cek, int* csi,
-                           double* ceks, int* cfpt) {
+__global__ void k_clu_hist(Params P, DevState* st, int force, const int* cs, const double* cek,
+                           int* csi, double* ceks, int* cfpt) {
   if (clu_gate(st, force)) return;
   __shared__ int hc[kSmallBins];
   __shared__ double he[kSmallBins];
@@ -320,7 +320,8 @@ __global__ void k_liq_tiles(Params P, DevState* st, int force, const int* liq, i
   if (threadIdx.x == 0) st->nliq = carry;
 }
 
-__global__ void k_liq_rank(Params P, DevState* st, int force, const int* liq, const int* aux, int* rank) {
+__global__ void k_liq_rank(Params P, DevState* st, int force, const int* liq, const int* aux,
+                           int* rank) {
   if (clu_gate(st, force)) return;
   __shared__ int sh[33];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -330,8 +331,9 @@ __global__ void k_liq_rank(Params P, DevState* st, int force, const int* liq, co
   if (i < P.N) rank[i] = aux[blockIdx.x] + ex;
 }
 
-__global__ void k_liq_union(DevState* st, int force, const int2* bonds, const unsigned long long* nbonds,
-                            int bond_cap, const int* liq, const int* perm, int* parent2) {
+__global__ void k_liq_union(DevState* st, int force, const int2* bonds,
+                            const unsigned long long* nbonds, int bond_cap, const int* liq,
+                            const int* perm, int* parent2) {
   if (clu_gate(st, force)) return;
   unsigned long long nb = *nbonds;
   if (nb > (unsigned long long)bond_cap) nb = bond_cap;

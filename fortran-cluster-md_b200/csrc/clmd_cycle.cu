@@ -383,9 +383,6 @@ __global__ void __launch_bounds__(kPB, CLMD_CYCLE_MINB) k_cycle(Params P, DevSta
     B.g.cfx = st->cfx; B.g.cfy = st->cfy; B.g.cfz = st->cfz;
     B.g.ncx = st->ncx; B.g.ncy = st->ncy; B.g.ncz = st->ncz; B.g.ncell = st->ncell;
     B.g.nox = st->nox; B.g.noy = st->noy; B.g.noz = st->noz;
-    for (int d = 0; d < 3; d++) {
-      B.g.offx[d] = st->offx[d]; B.g.offy[d] = st->offy[d]; B.g.offz[d] = st->offz[d];
-    }
     B.stop = 0;
     B.rebuild = 0;
   }
@@ -769,9 +766,6 @@ done:
     st->cfx = B.g.cfx; st->cfy = B.g.cfy; st->cfz = B.g.cfz;
     st->ncx = B.g.ncx; st->ncy = B.g.ncy; st->ncz = B.g.ncz; st->ncell = B.g.ncell;
     st->nox = B.g.nox; st->noy = B.g.noy; st->noz = B.g.noz;
-    for (int d = 0; d < 3; d++) {
-      st->offx[d] = B.g.offx[d]; st->offy[d] = B.g.offy[d]; st->offz[d] = B.g.offz[d];
-    }
   }
 }
 
@@ -846,8 +840,8 @@ void cycle_launch(clmd_system* S, int nsteps, int mode, const int* step) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, cycle_kernel(S), S->P, S->st, cycle_args(S), nsteps, mode, step ? *step : 0,
-                     step != nullptr);
+  cudaLaunchKernelEx(&cfg, cycle_kernel(S), S->P, S->st, cycle_args(S), nsteps, mode,
+                     step ? *step : 0, step != nullptr);
   S->launches++;
 }
 #endif  // CLMD_CYCLE_MIXED

@@ -14,8 +14,7 @@ constexpr int kSmallThreads = 512; // threads per CTA of the small-system kernel
 struct Geo {
   double rs2, cfx, cfy, cfz;
   int ncx, ncy, ncz, ncell;
-  int nox, noy, noz, pad;
-  int offx[3], offy[3], offz[3];
+  int nox, noy, noz, pad;  // cells searched per dimension: 1, 2 or 3
   // the FP32 list test: r^2 below flo is a neighbour, above fhi is none; in
   // between the FP64 test decides
   float flo, fhi;
@@ -60,17 +59,10 @@ static __device__ void prologue(const Params& P, Blk& B, int step) {
   double side = q.atrskin * (1.0 + 1e-9);
   int n3[3] = {(int)floor(P.boxx / side), (int)floor(P.boxy / side), (int)floor(P.boxz / side)};
   int mx[3] = {P.ncx_max, P.ncy_max, P.ncz_max};
-  int* offs[3] = {g.offx, g.offy, g.offz};
   int* nos[3] = {&g.nox, &g.noy, &g.noz};
   for (int d = 0; d < 3; d++) {
     n3[d] = max(1, min(n3[d], mx[d]));
-    if (n3[d] >= 3) {
-      offs[d][0] = -1; offs[d][1] = 0; offs[d][2] = 1; *nos[d] = 3;
-    } else if (n3[d] == 2) {
-      offs[d][0] = 0; offs[d][1] = 1; *nos[d] = 2;
-    } else {
-      offs[d][0] = 0; *nos[d] = 1;
-    }
+    *nos[d] = min(n3[d], 3);
   }
   g.ncx = n3[0];
   g.ncy = n3[1];

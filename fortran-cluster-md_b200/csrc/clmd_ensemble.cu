@@ -148,36 +148,34 @@ __device__ __forceinline__ double cta_max(double v, double* sh) {
   return r;
 }
 
-// two block-wide sums and an "any" flag in one round: every warp reduces the
+// a block-wide sum and an "any" flag in one round: every warp reduces the
 // per-warp partials itself, so one barrier publishes them and one guards the
 // buffer's reuse (fixed shape: deterministic)
 template <int NT>
-__device__ __forceinline__ void cta_sum2(double& a, double& b, int& f, double* sh) {
+__device__ __forceinline__ void cta_sum_any(double& a, int& f, double* sh) {
   constexpr int W = NT / 32;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   a = wsum(a);
-  b = wsum(b);
   f = __any_sync(0xffffffffu, f);
   if (lane == 0) {
     sh[w] = a;
-    sh[W + w] = b;
-    sh[2 * W + w] = f ? 1.0 : 0.0;
+    sh[W + w] = f ? 1.0 : 0.0;
   }
   __syncthreads();
-  double ta = lane < W ? sh[lane] : 0.0, tb = lane < W ? sh[W + lane] : 0.0;
-  const int tf = lane < W ? (sh[2 * W + lane] != 0.0) : 0;
+  const double ta = lane < W ? sh[lane] : 0.0;
+  const int tf = lane < W ? (sh[W + lane] != 0.0) : 0;
   a = wsum(ta);
-  b = wsum(tb);
   f = __any_sync(0xffffffffu, tf);
   __syncthreads();
 }
 
-// the block sum of S (the tree of cta_sum2) and the closed-form Nose-Hoover
+// the block sum of S (the tree of cta_sum) and the closed-form Nose-Hoover
 // root (clmd_nh_root) on warp 0 alone, published by the second barrier:
 // the other warps skip the scalar Newton steps and their divisions.  The
-// step's end is folded in (one CTA per replica): lane 0 of warp 0 also records the replica's new PSI, sum v^2, ekin, step and pair
-// terms (or the solve's failure) before the barrier that publishes the root,
-// so the step needs no barrier of its own to publish them
+// step's end is folded in (one CTA per replica): lane 0 of warp 0 also records
+// the replica's new PSI, sum v^2, ekin, step and pair terms (mixed: or the
+// solve's failure) before the barrier that publishes the root, so the step
+// needs no barrier of its own to publish them
 template <int NT, bool MIXED>
 __device__ __forceinline__ bool cta_nh_root_commit(double S, double psi1, double nkt3,
                                                    double dth, double Q, double* sh, Rep& R,
@@ -250,8 +248,8 @@ __device__ __forceinline__ double mi_bf(double d, double L, double iL, double bf
 }
 
 struct Cta {
-  double xred[3 * 16];  // cluster reductions: the CTAs' partials (rank 0's copy is read)
-  double xloc[4];       // cluster reductions: the totals, for this CTA's threads
+  double xred[2 * 16];  // cluster reductions: the CTAs' partials (rank 0's copy is read)
+  double xloc[2];       // cluster reductions: the totals, for this CTA's threads
   double* sx;  // positions in shared memory (nullptr: global)
   double* sy;
   double* sz;
@@ -317,7 +315,7 @@ __device__ __forceinline__ void half_out(double& v, int slot) {
   v = 0.0;
 }
 
-// a reduction over a cluster's threads (1024 a CTA) of nv <= 3 values,
+// a reduction over a cluster's threads (1024 a CTA) of nv <= 2 values,
 // returned in v to every thread; op 0 sums, op 1 takes maxima; H = 2: the
 // sums' first halves are in halves()'s slots from `slot` on.  Two cluster
 // barriers: the CTAs' partials are published, then read by every CTA before
@@ -378,18 +376,17 @@ __device__ __forceinline__ double grp_max(double v, Cta& C) {
     return v;
   }
 }
-// (two integer sums, exact in any order, and an "any" flag)
+// (an integer sum, exact in any order, and an "any" flag)
 template <int NT, int CS>
-__device__ __forceinline__ void grp_sum2(double& a, double& b, int& f, Cta& C) {
+__device__ __forceinline__ void grp_sum_any(double& a, int& f, Cta& C) {
   if constexpr (CS == 1) {
-    cta_sum2<NT>(a, b, f, C.red);
+    cta_sum_any<NT>(a, f, C.red);
   } else {
-    double v[3] = {a, b, f ? 1.0 : 0.0};
-    const int op[3] = {0, 0, 1};
-    cl_reduce<CS, 1>(v, 3, op, C, 0);
+    double v[2] = {a, f ? 1.0 : 0.0};
+    const int op[2] = {0, 1};
+    cl_reduce<CS, 1>(v, 2, op, C, 0);
     a = v[0];
-    b = v[1];
-    f = v[2] != 0.0;
+    f = v[1] != 0.0;
   }
 }
 // the closed-form Nose-Hoover root of a cluster's total of S: warp 0 of
@@ -864,8 +861,8 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
   {
     // the rows' total (pair terms of each force pass until the next
     // rebuild) and "any row overflowed" in one reduction
-    double tn = (double)nsum, unused = 0.0;
-    grp_sum2<NT, CS>(tn, unused, over, C);
+    double tn = (double)nsum;
+    grp_sum_any<NT, CS>(tn, over, C);
     if (tid == 0) R.nfull = (int)tn;
   }
   if (over) {
@@ -937,8 +934,8 @@ struct RowWalk {
 
 // pair forces (for-a-lj-n-pbc-m.f, sigma = eps = m = 1) -> a; optional
 // velocity-Verlet second half kick; FP64 energy/virial sums when asked
-// NHF: also the Nose-Hoover solve's first pass on the fresh accelerations
-// (vo = v: vxn = v, s0 += v.v, dp += b vo dt/Q with b = -dth (a - psi1 vo))
+// NHF: also the pass of the Nose-Hoover solve on the fresh accelerations,
+// W = V + dth a into vn and s0 += W.W (clmd_nh_root)
 template <int NT, bool SM, bool MIXED, int CS, int H, bool NHF = false>
 __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kick,
                        bool energies, double* s0 = nullptr) {
@@ -961,7 +958,7 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
       const bool own = i < N;
       const int ii = own ? i : w0;
       double xi, yi, zi;
-    P.get(ii, xi, yi, zi);
+      P.get(ii, xi, yi, zi);
       const int len = own ? A.rlen[off + i] : 0;
       float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
       const int* lp = A.list + lbase + (long long)sub * N + ii;
@@ -1139,7 +1136,7 @@ __device__ void forces(Rep& R, Cta& C, const Args& A, const Pos<SM>& P, bool kic
       if (kick) R.ekin = k;
     }
   }
-  // one CTA, mixed Nose-Hoover: the closed-form root that follows opens with
+  // one CTA, Nose-Hoover: the closed-form root that follows opens with
   // barriers of its own (cta_nh_root_commit), which order this pass's
   // per-atom writes before anyone reads them
   if constexpr (!(NHF && CS == 1)) gsync<CS>();
@@ -2052,8 +2049,8 @@ extern "C" int clmd_ens_destroy(clmd_ensemble* E) {
   cudaStreamSynchronize(E->stream);
   Args& A = E->A;
   void* ps[] = {A.x, A.y, A.z, A.vx, A.vy, A.vz, A.vxn, A.vyn, A.vzn, A.a, A.list, A.rlen,
-                A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.cand, A.p4, A.reps, A.fpt, A.summary,
-                E->d_items, E->d_ctr, E->d_iwin, A.wtime, E->d_stage, A.cscr,
+                A.sorted, A.cellid, A.parent, A.cs, A.cl, A.orig, A.cand, A.p4, A.reps, A.fpt,
+                A.summary, E->d_items, E->d_ctr, E->d_iwin, A.wtime, E->d_stage, A.cscr,
                 E->d_hoff};
   for (void* p : ps)
     if (p) cudaFree(p);

@@ -62,7 +62,6 @@ struct DevState {
   int err_new;                  // error raised inside a kernel, merged later
   int ncx, ncy, ncz, ncell;
   int nox, noy, noz;
-  int offx[3], offy[3], offz[3];
   double cfx, cfy, cfz;         // cells per unit length
   double rs2;
   // thermostat

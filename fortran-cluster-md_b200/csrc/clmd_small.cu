@@ -97,10 +97,6 @@ struct Atom {
   bool act;
 };
 
-// neighbor-pbc-mav.f:67-99: positions wrapped, atoms put in cell order (ties
-// by reference index, as k_cycle), rows searched and sorted.  acc: the
-// accelerations move with their atoms (a rebuild inside a step runs before
-// the force pass that overwrites them).  False: the cluster must stop.
 template <class T>
 __device__ __forceinline__ T s_pre(T v, int lane) {  // inclusive scan over the warp
 #pragma unroll
@@ -111,6 +107,10 @@ __device__ __forceinline__ T s_pre(T v, int lane) {  // inclusive scan over the 
   return v;
 }
 
+// neighbor-pbc-mav.f:67-99: positions wrapped, atoms put in cell order (ties
+// by reference index, as k_cycle), rows searched and sorted.  acc: the
+// accelerations move with their atoms (a rebuild inside a step runs before
+// the force pass that overwrites them).  False: the cluster must stop.
 static __device__ bool s_rebuild(const Params& P, DevState* st, SmallShared& S, Grp& G,
                                  const CycleArgs& A, double4* pos, Atom& a, int p, bool acc) {
   const Geo& g = S.B.g;
@@ -297,9 +297,6 @@ __global__ void __launch_bounds__(kSNT, 1) k_small(Params P, DevState* st, Cycle
     B.g.cfx = st->cfx; B.g.cfy = st->cfy; B.g.cfz = st->cfz;
     B.g.ncx = st->ncx; B.g.ncy = st->ncy; B.g.ncz = st->ncz; B.g.ncell = st->ncell;
     B.g.nox = st->nox; B.g.noy = st->noy; B.g.noz = st->noz;
-    for (int d = 0; d < 3; d++) {
-      B.g.offx[d] = st->offx[d]; B.g.offy[d] = st->offy[d]; B.g.offz[d] = st->offz[d];
-    }
     B.stop = 0;
     B.rebuild = 0;
     S.err[0] = S.err[1] = 0;
@@ -563,9 +560,6 @@ done:
     st->cfx = B.g.cfx; st->cfy = B.g.cfy; st->cfz = B.g.cfz;
     st->ncx = B.g.ncx; st->ncy = B.g.ncy; st->ncz = B.g.ncz; st->ncell = B.g.ncell;
     st->nox = B.g.nox; st->noy = B.g.noy; st->noz = B.g.noz;
-    for (int d = 0; d < 3; d++) {
-      st->offx[d] = B.g.offx[d]; st->offy[d] = B.g.offy[d]; st->offz[d] = B.g.offz[d];
-    }
   }
   __syncthreads();
   {
