@@ -263,6 +263,7 @@ struct Cta {
   int ncx, ncell, nox;
   double cf, rs2;
   int flag;
+  int nan;  // the replica has an atom at a NaN
   int ident;  // sorted[] is the identity (the slots are in cell order)
   int rep;  // slot of the replica being run
   int nsteps;  // MD steps this replica runs in this launch
@@ -605,24 +606,22 @@ __device__ void cta_scan16(unsigned* word, int nw) {
 // (neighbour k at list[lbase + k N + i], at most the stride of them); returns
 // the neighbours found.
 // A candidate is 8 bytes in cell order: its coordinates in 2^-16 of the box
-// and its slot (below 2^15 where positions are in shared memory; elsewhere not
-// kept), with the top bit set for an atom at a NaN, which is nobody's
-// neighbour.  The 16-bit differences wrap like the periodic
+// and its slot's low 16 bits.  The 16-bit differences wrap like the periodic
 // box, so the nearest image needs no test, and three integer products decide
 // all candidates but those within the truncation of the list radius (~0.3% of
 // r^2), which FP64 positions decide (mi_sel and r^2 rounded term by term; r^2
 // does not depend on the pair's orientation): the pair set is the FP64
-// test's.  That test alone, three FP64 positions a candidate gathered by
-// slot, ran a chain of ~150 cycles per candidate in every lane (a rebuild of
-// the average batched replica 133k cycles, now 77k; the window 57.5 -> 50.5
-// ms).  Two
-// candidates are loaded at a time, and the next cell row's range ahead of
-// this one's tests.
+// test's.  (With an atom at a NaN, whose coordinates mean nothing here, FP64
+// decides every candidate.)  That test alone, three FP64 positions a candidate
+// gathered by slot, ran a chain of ~150 cycles per candidate in every lane (a
+// rebuild of the average batched replica 133k cycles, now 77k; the window
+// 57.5 -> 50.5 ms).  Two candidates are loaded at a time, and the next cell
+// row's range ahead of this one's tests.
 template <bool SM>
 __device__ __forceinline__ int search_row(const Cta& C, const Args& A, const Pos<SM>& P, int q0,
                                           int i, int N, double L, long long lbase) {
   const int ncx = C.ncx, nox = C.nox;
-  const unsigned ulo = C.ulo, uhi = C.uhi;
+  const unsigned ulo = C.nan ? 0u : C.ulo, uhi = C.uhi;
   const uint2* cand = C.cand;
   const uint2 me = cand[q0];
   const int cx = clmd_cell(P.x(i), C.cf, ncx), cy = clmd_cell(P.y(i), C.cf, ncx),
@@ -654,7 +653,7 @@ __device__ __forceinline__ int search_row(const Cta& C, const Args& A, const Pos
     const int dx = (short)(me.x - c.x), dy = (short)((me.x >> 16) - (c.x >> 16)),
               dz = (short)(me.y - c.y);
     const unsigned u = (unsigned)(dx * dx) + (unsigned)(dy * dy) + (unsigned)(dz * dz);
-    if (u > uhi || q == q0 || (int)c.y < 0) return;
+    if (u > uhi || q == q0) return;
     const int j = SM ? (int)(c.y >> 16) : (C.ident ? q : A.sorted[P.off + q]);
     if (u >= ulo) {
       const double hL = 0.5 * L;
@@ -697,7 +696,7 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
   const int gt = gtid<NT, CS>();
   constexpr int GT = NT * CS;
   const double L = R.box;
-  if (tid == 0) C.ident = 0;  // until a reorder into cell order below
+  if (tid == 0) C.ident = C.nan = 0;  // until a reorder into cell order, an atom at a NaN
   if constexpr (SM) {
     // 16-bit counts, two to a word: the count before an atom's own is its
     // arrival number; both travel in cellid[] (cells < 2^15).  The slots go
@@ -842,9 +841,13 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
       const int i = C.ident ? q : A.sorted[off + q];
       double x, y, z;
       P.get(i, x, y, z);
-      unsigned tag = SM ? (unsigned)i : 0u;
-      if (isnan(x + y + z)) tag |= 0x8000u;
-      C.cand[q] = make_uint2(u16(x) | u16(y) << 16, u16(z) | tag << 16);
+      C.cand[q] = make_uint2(u16(x) | u16(y) << 16, u16(z) | (unsigned)i << 16);
+      if (isnan(x + y + z)) {
+        if constexpr (CS == 1)
+          C.nan = 1;
+        else
+          for (int r = 0; r < CS; r++) *cg::this_cluster().map_shared_rank(&C.nan, r) = 1;
+      }
     }
     gsync<CS>();
   }
@@ -853,7 +856,7 @@ __device__ bool rebuild(Rep& R, Cta& C, const Args& A, const Pos<SM>& P) {
   // candidates read by several lanes at once)
   for (int q0 = gt; q0 < N; q0 += GT) {
     const int i = C.ident ? q0 : A.sorted[off + q0];
-    const int n = (int)C.cand[q0].y < 0 ? 0 : search_row<SM>(C, A, P, q0, i, N, L, lbase);
+    const int n = search_row<SM>(C, A, P, q0, i, N, L, lbase);
     if (n > A.lstride) over = 1;
     A.rlen[off + i] = min(n, A.lstride);
     nsum += min(n, A.lstride);
